@@ -36,20 +36,48 @@ __device__ __forceinline__ void bf16_limbs2(float x0, float x1, uint32_t& p0, ui
     p2 = bf16x2_rn(s0, s1);
 }
 
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float4 add_rn(float4 a, float4 b) {
+    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+
+// Four floats `step` apart, read and added like a float4.
+struct Strided4 {
+    const float* at;
+    size_t step;
+};
+__device__ __forceinline__ Strided4 operator+(Strided4 p, size_t n) { return {p.at + n, p.step}; }
+__device__ __forceinline__ float4 __ldcg(Strided4 p) {
+    return make_float4(::__ldcg(p.at), ::__ldcg(p.at + p.step), ::__ldcg(p.at + 2 * p.step), ::__ldcg(p.at + 3 * p.step));
+}
+using ::__ldcg;
+
 // src[0] + src[stride] + ... + src[(n - 1) stride], added in that order with
-// round-to-nearest FP32 adds (the slice order of the split-K reductions); the
-// loads are issued BATCH at a time so that they overlap (a batch of 64 covers
-// every split in one round trip to L2).
-template <int BATCH = 16>
-__device__ __forceinline__ float ordered_sum(const float* __restrict__ src, size_t stride, int n) {
-    float acc = __ldcs(src);
-    for (int z = 1; z < n; z += BATCH) {
-        float v[BATCH];
+// round-to-nearest FP32 adds (the slice order of the split-K reductions), for
+// one output per thread (src a float pointer) or four (a float4 pointer, or
+// Strided4 with the stride in floats). The loads of BATCH slices are issued
+// together so that they overlap; slices past n are not read. Loads from L2:
+// the slices were written just before.
+template <int BATCH, typename Src>
+__device__ __forceinline__ auto ordered_sum(Src src, size_t stride, int n) {
+    auto acc = __ldcg(src);
+    using T = decltype(acc);
+    int z = 1;
+    for (; z + BATCH <= n; z += BATCH) {
+        T v[BATCH];
 #pragma unroll
-        for (int j = 0; j < BATCH; j++) v[j] = (z + j < n) ? __ldcs(src + (size_t)(z + j) * stride) : 0.0f;
+        for (int j = 0; j < BATCH; j++) v[j] = __ldcg(src + (size_t)(z + j) * stride);
+#pragma unroll
+        for (int j = 0; j < BATCH; j++) acc = add_rn(acc, v[j]);
+    }
+    if (z < n) {
+        T v[BATCH];
 #pragma unroll
         for (int j = 0; j < BATCH; j++)
-            if (z + j < n) acc = __fadd_rn(acc, v[j]);
+            if (z + j < n) v[j] = __ldcg(src + (size_t)(z + j) * stride);
+#pragma unroll
+        for (int j = 0; j < BATCH; j++)
+            if (z + j < n) acc = add_rn(acc, v[j]);
     }
     return acc;
 }

@@ -1332,34 +1332,54 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 }
 
 // Split-K reduction for plans that cut every tile into K slices. The GEMM
-// wrote one partial tile per (128-row half, slice); each thread here sums one
-// element over the slices in slice order -- the order of the in-kernel fixup,
-// so C is the same bit for bit -- and stores it. The slices of a tile are
-// read by many threads at once, 16 loads in flight per thread, instead of one
-// warp walking them in turn at the end of the GEMM. HBM-bound: nsplit
-// partials in, C out.
-template <int BN>
+// wrote one partial tile per (128-row half, slice); here each output is summed
+// over the slices in slice order -- the order of the in-kernel fixup, so C is
+// the same bit for bit. Bound by the reads of the partials (nsplit floats per
+// output, from L2 while they fit). Measured (ncu): 1500 x 1999 x 4 slices 10.8 us
+// (5.4 TB/s), 1024^2 x 4 5.8 us, 128 x 512 x 37 5.0 us; one output per thread
+// down a column, which stored C 4 bytes at a time, took 32.1, 12.7 and 5.7 us.
+//
+// Partial tiles are column-major (element (r, c) at c * 128 + r), C is
+// row-major. A block takes 32 rows x 8 E columns: warp w reads columns w, w +
+// 8, ... with one row per lane (128-byte lines), and the sums cross a padded
+// shared tile so that C is written in runs of 8 E columns (128 bytes for E = 4)
+// instead of 4-byte pieces N apart.
+template <int BN, int E, int BATCH>
 __global__ void __launch_bounds__(256)
 tc_splitk_reduce_kernel(const TcParams p) {
     constexpr size_t TILE = (size_t)128 * BN;
+    static_assert(E == 1 || E == 4, "columns per thread");
+    constexpr int CB = 8 * E, CGROUPS = BN / CB;              // columns per block, blocks per tile row group
+    __shared__ float sh[CB][33];
     const int halves = p.bm / 128;
-    const int64_t total = p.tiles * halves * (int64_t)TILE;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        // Partial tiles are column-major (c * 128 + r): consecutive threads
-        // read consecutive partial elements down a column.
-        const int lrow = (int)(i % 128);
-        const int q = (int)((i / 128) % BN);
-        const int64_t th = i / (int64_t)TILE;                   // tile * halves + half
-        const int64_t t = halves == 2 ? th >> 1 : th;
-        int tm, tn;
-        if (p.tiles <= (int64_t)UINT32_MAX) tile_coords_t<uint32_t>(p, (uint32_t)t, tm, tn);
-        else tile_coords_t<uint64_t>(p, (uint64_t)t, tm, tn);
-        const int64_t row = (int64_t)tm * p.bm + (th - t * halves) * 128 + lrow;
-        const int64_t col = (int64_t)tn * BN + q;
-        if (row >= p.M || col >= p.N) continue;
-        const float* src = p.partial + (size_t)th * p.max_splits * TILE + (size_t)q * 128 + (size_t)lrow;
-        p.C[(size_t)row * (size_t)p.N + (size_t)col] = ordered_sum(src, TILE, p.main_splits);
+    const int64_t b = blockIdx.x;
+    const int rg = (int)(b & 3), cg = (int)((b >> 2) % CGROUPS);
+    const int64_t th = (b >> 2) / CGROUPS;                    // tile * halves + half
+    const int64_t t = halves == 2 ? th >> 1 : th;
+    int tm, tn;
+    if (p.tiles <= (int64_t)UINT32_MAX) tile_coords_t<uint32_t>(p, (uint32_t)t, tm, tn);
+    else tile_coords_t<uint64_t>(p, (uint64_t)t, tm, tn);
+    const int64_t row0 = (int64_t)tm * p.bm + (th - t * halves) * 128 + rg * 32;
+    const int64_t col0 = (int64_t)tn * BN + cg * CB;
+    if (row0 >= p.M || col0 >= p.N) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* src = p.partial + (size_t)th * p.max_splits * TILE + (size_t)(cg * CB + warp) * 128 + rg * 32 + lane;
+    // Rows past M and columns past N are read too: every slice wrote its whole
+    // tile; they are not stored.
+    if constexpr (E == 4) {
+        const float4 v = ordered_sum<BATCH>(Strided4{src, (size_t)8 * 128}, TILE, p.main_splits);
+        sh[warp][lane] = v.x;
+        sh[warp + 8][lane] = v.y;
+        sh[warp + 16][lane] = v.z;
+        sh[warp + 24][lane] = v.w;
+    } else {
+        sh[warp][lane] = ordered_sum<BATCH>(src, TILE, p.main_splits);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const int i = threadIdx.x + 256 * e, r = i / CB, c = i % CB;
+        if (row0 + r < p.M && col0 + c < p.N) p.C[(size_t)(row0 + r) * (size_t)p.N + (size_t)(col0 + c)] = sh[c][r];
     }
 }
 
@@ -1368,14 +1388,24 @@ tc_splitk_reduce_kernel(const TcParams p) {
 // slice to arrive, inside the GEMM.
 constexpr int kReduceAfterSplits = 3;
 
+template <int BN, int E>
+cudaError_t launch_reduce_e(const TcParams& prm, cudaStream_t s) {
+    const unsigned blocks = (unsigned)(prm.tiles * (prm.bm / 128) * 4 * (BN / (8 * E)));
+    if (prm.main_splits <= 4) tc_splitk_reduce_kernel<BN, E, 3><<<blocks, 256, 0, s>>>(prm);
+    else if (prm.main_splits <= 8) tc_splitk_reduce_kernel<BN, E, 7><<<blocks, 256, 0, s>>>(prm);
+    else if (E > 1 || prm.main_splits <= 16) tc_splitk_reduce_kernel<BN, E, 15><<<blocks, 256, 0, s>>>(prm);
+    else tc_splitk_reduce_kernel<BN, E, 63><<<blocks, 256, 0, s>>>(prm);
+    return cudaGetLastError();
+}
+
+// 32-column blocks (whole 128-byte runs of C) when they number at least two an
+// SM; else 8-column blocks, four times as many, which a narrow C needs to
+// spread the reads of its many slices over the GPU (128 x 512 has 64 of the
+// former, 256 of the latter).
 template <int BN>
 cudaError_t launch_reduce(const TcParams& prm, cudaStream_t s) {
-    const int64_t total = prm.tiles * (prm.bm / 128) * 128 * BN;
-    int64_t blocks = (total + 255) / 256;
-    const int64_t cap = (int64_t)device_sm_count() * 8;
-    if (cap > 0 && blocks > cap) blocks = cap;
-    tc_splitk_reduce_kernel<BN><<<(unsigned)blocks, 256, 0, s>>>(prm);
-    return cudaGetLastError();
+    const int64_t wide = prm.tiles * (prm.bm / 128) * 4 * (BN / 32);
+    return wide >= 2 * (int64_t)device_sm_count() ? launch_reduce_e<BN, 4>(prm, s) : launch_reduce_e<BN, 1>(prm, s);
 }
 
 // Host-side schedule of one launch (see TcParams).
