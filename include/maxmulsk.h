@@ -422,6 +422,7 @@ const char* maxmulsk_version(void);
  *   "split"   operand planes of the split-precision path (pre-pass)
  *   "gemm"    the GEMM kernel (SIMT or tcgen05)
  *   "reduce"  the split-K reduction kernel of plans with 3 or more K slices
+ *             (FP32: 2 or more)
  *   "grouped" one grouped batch (its CUDA graph)
  *   "h2d" / "d2h"  the host entry points' copies (pipelined copies overlap)
  * Up to 65536 phases are held between two reports; later ones are dropped.

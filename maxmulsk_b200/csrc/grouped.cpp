@@ -57,7 +57,7 @@ struct maxmulsk_grouped_s {
     unsigned* d_next = nullptr;
     void* d_scratch = nullptr;             // [counters of all split problems][partials]
     size_t counter_bytes = 0;
-    int grid = 0;
+    int sms = 0;
     // split-precision part
     void* d_tc = nullptr;                  // [problems][units][tensor maps][counters][partials]
     mmsk::TcGroupArgs tc{};
@@ -91,12 +91,12 @@ namespace {
 
 inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Relative throughput of the SIMT tile shapes (measured at 4096^3: 48, 41 and
-// 32 TFLOP/s for 128x128, 128x64, 64x64).
+// Relative throughput of the SIMT tile shapes (measured at 4096^3: 58, 54 and
+// 51 TFLOP/s for 128x128, 128x64, 64x64).
 double tile_rate(int bm, int bn) {
     if (bm == 128 && bn == 128) return 1.0;
-    if (bm == 128 && bn == 64) return 0.85;
-    return 0.66;
+    if (bm == 128 && bn == 64) return 0.93;
+    return 0.87;
 }
 
 // Padded work of a problem on a tile shape, in multiply-adds.
@@ -187,8 +187,7 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
         q.a.kchunk = (int64_t)slice_len(p.K, sk[j]);
         q.a.splits = p.K ? slice_count(p.K, sk[j]) : 1;
         q.tiles_n = (int32_t)((p.N + bn - 1) / bn);
-        q.vec = (p.K % 4 == 0) && (p.N % 4 == 0) && ((uintptr_t)p.A % 16 == 0) && ((uintptr_t)p.B % 16 == 0) &&
-                ((uintptr_t)p.C % 16 == 0);
+        simt_set_widths(q.a);
         if (q.a.splits > 1) {
             q.a.counters = reinterpret_cast<unsigned*>(static_cast<char*>(g->d_scratch) + ctr_off[j]);
             q.a.partial = reinterpret_cast<float*>(static_cast<char*>(g->d_scratch) + g->counter_bytes + part_off[j]);
@@ -208,7 +207,7 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
         return la > lb;
     });
     g->nunits = (int)hu.size();
-    g->grid = std::max(1, std::min(g->nunits, 2 * sms));
+    g->sms = sms;
     cudaError_t e;
     if ((e = cudaMalloc(&g->d_probs, std::max<size_t>(1, idx.size()) * sizeof(GroupProblem))) != cudaSuccess ||
         (e = cudaMalloc(&g->d_units, std::max<size_t>(1, hu.size()) * sizeof(GroupUnit))) != cudaSuccess ||
@@ -444,7 +443,7 @@ maxmulsk_status capture_group(maxmulsk_grouped_s* g, const maxmulsk_problem* pro
         if (g->d_scratch && g->counter_bytes) cudaMemsetAsync(g->d_scratch, 0, g->counter_bytes, g->cap);
         if (g->nunits > 0)
             simt_grouped_launch(g->d_probs, g->d_units, g->nunits, g->d_next, g->simt_plan.tile_m,
-                                g->simt_plan.tile_n, g->simt_plan.variant, g->grid, g->cap);
+                                g->simt_plan.tile_n, g->simt_plan.variant, g->sms, g->cap);
         for (const auto& sg : g->singles) {
             const maxmulsk_problem& p = problems[sg.problem];
             maxmulsk_status s1 = run_plan_dev(p.A, p.B, p.C, p.M, p.K, p.N, sg.plan, g->d_single_ws,

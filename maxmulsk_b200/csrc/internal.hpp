@@ -40,10 +40,22 @@ struct SimtArgs {
     int64_t kchunk;        // slice length (multiple of kSliceAlign) or K
     int splits;            // slices actually run (>= 1)
     float* partial;        // splits * M * N floats when splits > 1
-    unsigned* counters;    // one per output tile when splits > 1 (zero on entry)
+    unsigned* counters;    // grouped launches: one per output tile when splits > 1 (zero on entry)
     int reduce_after;      // set by simt_launch: slices only write partials, a
                            // separate kernel sums them (zero everywhere else)
+    int wa, wb, wc;        // set by simt_set_widths: floats A, B and C move at a time
 };
+// The widest accesses (4, 2 or 1 floats) that every row of an operand allows:
+// rows start on multiples of that size. C takes 4 or 1.
+inline void simt_set_widths(SimtArgs& a) {
+    auto width = [](int64_t ld, const void* p) {
+        if (ld % 4 == 0 && (uintptr_t)p % 16 == 0) return 4;
+        return ld % 2 == 0 && (uintptr_t)p % 8 == 0 ? 2 : 1;
+    };
+    a.wa = width(a.K, a.A);
+    a.wb = width(a.N, a.B);
+    a.wc = width(a.N, a.C) == 4 ? 4 : 1;
+}
 // Workspace bytes for the SIMT path with this tile/split choice.
 size_t simt_workspace_bytes(int64_t M, int64_t K, int64_t N, int tile_m, int tile_n, int split_k);
 // Lays out ws into SimtArgs fields. Returns false if ws is too small.
@@ -53,17 +65,16 @@ cudaError_t simt_launch(const SimtArgs& a, int tile_m, int tile_n, int variant, 
 struct GroupProblem {
     SimtArgs a;            // one problem: pointers, sizes, its K slicing and scratch
     int32_t tiles_n;       // tiles along N (numbers the split-K counters)
-    int32_t vec;           // 128-bit loads allowed for this problem
 };
 struct GroupUnit {
     int32_t problem, tm, tn, z;
 };
 cudaError_t simt_grouped_launch(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,
-                                int tile_m, int tile_n, int variant, int grid, cudaStream_t s);
+                                int tile_m, int tile_n, int variant, int sms, cudaStream_t s);
 // Runs an FP32 plan whose split-K scratch (counters, then partials) is at
 // `scratch` (>= simt_workspace_bytes; may be null without a K split): lays it
-// out, clears the counters on `s`, launches. Both the workspace entry and the
-// static-scratch entry go through here.
+// out and launches (the counters are unused, their place kept). Both the
+// workspace entry and the static-scratch entry go through here.
 maxmulsk_status simt_run(const float* dA, const float* dB, float* dC, size_t M, size_t K, size_t N,
                          const maxmulsk_plan& plan, void* scratch, size_t scratch_bytes, cudaStream_t s);
 // The SIMT plan with its split-K scratch in a static device array (no allocation).

@@ -1,12 +1,10 @@
 // FP32 SIMT GEMM for sm_100a: C = A*B, row-major, on the CUDA cores.
 //
 // Replaces the reference's blocked SME driver (sme/v3/sme-1x4-acc-kcout.cpp:427-567)
-// as the FP32-accurate path. The SME packers (pack_A_streaming :39-136 with
-// its ZA transpose, pack_B_streaming :145-193) become shared-memory staging:
-// A is stored k-major (transposed on the way in, like the ZA transpose), B
-// row-major; both double-buffered, fed by 128-bit global loads. The 16x64 ZA
-// micro-tile becomes a CTA tile of tile_m x tile_n with an 8x8 (or 4x4)
-// register tile per thread.
+// as the FP32-accurate path. The SME packers (pack_A_streaming :39-136,
+// pack_B_streaming :145-193) become a ring of shared-memory stages filled by
+// cp.async; the 16x64 ZA micro-tile becomes a CTA tile of tile_m x tile_n with
+// a register tile of packed FP32 pairs per thread.
 //
 // Arithmetic: every output is ONE sequential chain over k in increasing order
 // (a fused multiply-add per step, or multiply-then-add in the SCALAR variant,
@@ -35,29 +33,6 @@
 
 namespace mmsk {
 namespace {
-
-constexpr int kThreads = 256;
-constexpr int kBK = 16;
-
-template <bool FUSED>
-__device__ __forceinline__ float mac(float a, float b, float c) {
-    if constexpr (FUSED) return __fmaf_rn(a, b, c);
-    else return __fadd_rn(c, __fmul_rn(a, b));
-}
-
-// Shared-memory stages of one CTA.
-//
-// A is stored k-major: As[k][m ^ swz(k)]. A warp's transposing stores write
-// 8 rows for each of the k's kq, kq+4, kq+8, kq+12 of its float4 loads; with
-// rows of BM + 4 floats, k and k + 8 fall on the same banks, so rows of k >= 8
-// are stored with bit 3 of the row index flipped. Groups of four rows stay
-// contiguous and 16-byte aligned for the float4 reads of the product loop.
-template <int BM, int BN>
-struct SimtSmem {
-    float As[2][kBK][BM + 4];                       // k-major A, padded rows, swizzled
-    float Bs[2][kBK][BN];
-    int last;
-};
 
 // The end of one tile: without a K split the sums go to C; with one, this
 // slice's partial tile is written and, unless a separate reduction kernel
@@ -156,212 +131,120 @@ __device__ __forceinline__ void simt_epilogue(const SimtArgs& p, float (&acc)[TM
     if (tid == 0) p.counters[tile] = 0u;   // leave the counter ready for the next call
 }
 
-// One CTA computes the BM x BN tile at (m0, n0) of K slice z; `tile` numbers
-// the tile for the split-K arrival counters. VM selects 128-bit loads and
-// stores: 0 never, 1 always (both fixed at compile time), 2 at run time by
-// `vec_rt` (one body for problems of either kind, as in grouped launches).
-template <int BM, int BN, bool FUSED, int VM>
-__device__ __forceinline__ void simt_tile(const SimtArgs& p, int64_t m0, int64_t n0, int z, unsigned tile,
-                                          SimtSmem<BM, BN>& sm, bool vec_rt = false) {
-    const bool VEC = (VM == 2) ? vec_rt : (VM == 1);
-    constexpr int TM = BM / 16, TN = BN / 16;       // per-thread outputs
-    constexpr int GM = TM / 4, GN = TN / 4;         // 4-wide groups per thread
-    constexpr int A_F4 = BM * kBK / 4 / kThreads;   // float4 loads per thread
-    constexpr int B_F4 = BN * kBK / 4 / kThreads;
-    auto& As = sm.As;
-    auto& Bs = sm.Bs;
-
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int64_t kbeg = (int64_t)z * p.kchunk;
-    const int64_t kend = min(p.K, kbeg + p.kchunk);
-    const int64_t M = p.M, N = p.N, K = p.K;
-    const float* __restrict__ A = p.A;
-    const float* __restrict__ B = p.B;
-
-    float4 ra[A_F4], rb[B_F4];
-
-    auto load_tile = [&](int64_t k0) {
-#pragma unroll
-        for (int j = 0; j < A_F4; j++) {
-            const int f = tid + j * kThreads;
-            const int row = f / (kBK / 4);
-            const int kq = (f % (kBK / 4)) * 4;
-            const int64_t gm = m0 + row, gk = k0 + kq;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (gm < M) {
-                const float* src = A + gm * K + gk;
-                if (VEC) {
-                    if (gk < kend) v = __ldg(reinterpret_cast<const float4*>(src));
-                } else {
-                    if (gk + 0 < kend) v.x = __ldg(src + 0);
-                    if (gk + 1 < kend) v.y = __ldg(src + 1);
-                    if (gk + 2 < kend) v.z = __ldg(src + 2);
-                    if (gk + 3 < kend) v.w = __ldg(src + 3);
-                }
-            }
-            ra[j] = v;
-        }
-#pragma unroll
-        for (int j = 0; j < B_F4; j++) {
-            const int f = tid + j * kThreads;
-            const int kr = f / (BN / 4);
-            const int nq = (f % (BN / 4)) * 4;
-            const int64_t gk = k0 + kr, gn = n0 + nq;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (gk < kend) {
-                const float* src = B + gk * N + gn;
-                if (VEC) {
-                    if (gn < N) v = __ldg(reinterpret_cast<const float4*>(src));
-                } else {
-                    if (gn + 0 < N) v.x = __ldg(src + 0);
-                    if (gn + 1 < N) v.y = __ldg(src + 1);
-                    if (gn + 2 < N) v.z = __ldg(src + 2);
-                    if (gn + 3 < N) v.w = __ldg(src + 3);
-                }
-            }
-            rb[j] = v;
-        }
-    };
-    auto store_tile = [&](int buf) {
-#pragma unroll
-        for (int j = 0; j < A_F4; j++) {
-            const int f = tid + j * kThreads;
-            const int row = f / (kBK / 4);
-            const int kq = (f % (kBK / 4)) * 4;
-            const int srow = row ^ (kq & 8);
-            As[buf][kq + 0][srow] = ra[j].x;
-            As[buf][kq + 1][srow] = ra[j].y;
-            As[buf][kq + 2][srow] = ra[j].z;
-            As[buf][kq + 3][srow] = ra[j].w;
-        }
-#pragma unroll
-        for (int j = 0; j < B_F4; j++) {
-            const int f = tid + j * kThreads;
-            const int kr = f / (BN / 4);
-            const int nq = (f % (BN / 4)) * 4;
-            *reinterpret_cast<float4*>(&Bs[buf][kr][nq]) = rb[j];
-        }
-    };
-
-    float acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; i++)
-#pragma unroll
-        for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
-
-    const int64_t ntiles = (kend - kbeg + kBK - 1) / kBK;
-    if (ntiles > 0) {
-        load_tile(kbeg);
-        store_tile(0);
-        __syncthreads();
-        for (int64_t t = 0; t < ntiles; t++) {
-            const int buf = (int)(t & 1);
-            if (t + 1 < ntiles) load_tile(kbeg + (t + 1) * kBK);
-            // Fragments of step k + 1 are read from shared memory while the
-            // products of step k run (two register sets, fully unrolled).
-            float a[2][TM], b[2][TN];
-            auto load_frag = [&](int set, int k) {
-#pragma unroll
-                for (int g = 0; g < GM; g++) {
-                    float4 v = *reinterpret_cast<const float4*>(&As[buf][k][(g * 64 + ty * 4) ^ (k & 8)]);
-                    a[set][g * 4 + 0] = v.x; a[set][g * 4 + 1] = v.y; a[set][g * 4 + 2] = v.z; a[set][g * 4 + 3] = v.w;
-                }
-#pragma unroll
-                for (int g = 0; g < GN; g++) {
-                    float4 v = *reinterpret_cast<const float4*>(&Bs[buf][k][g * 64 + tx * 4]);
-                    b[set][g * 4 + 0] = v.x; b[set][g * 4 + 1] = v.y; b[set][g * 4 + 2] = v.z; b[set][g * 4 + 3] = v.w;
-                }
-            };
-            load_frag(0, 0);
-#pragma unroll
-            for (int k = 0; k < kBK; k++) {
-                if (k + 1 < kBK) load_frag((k + 1) & 1, k + 1);
-#pragma unroll
-                for (int i = 0; i < TM; i++)
-#pragma unroll
-                    for (int j = 0; j < TN; j++) acc[i][j] = mac<FUSED>(a[k & 1][i], b[k & 1][j], acc[i][j]);
-            }
-            if (t + 1 < ntiles) store_tile(buf ^ 1);
-            __syncthreads();
-        }
-    }
-
-    // Steps past kend multiply by a zero operand. The product is +-0 and adding
-    // it leaves the chain unchanged (the chain never holds -0: it starts at +0
-    // and an exact zero sum rounds to +0), so the padded steps keep the result
-    // identical to a chain over [kbeg, kend) alone.
-
-    auto out_row = [&](int i) { return m0 + (i / 4) * 64 + ty * 4 + (i % 4); };
-    auto out_col = [&](int g) { return n0 + g * 64 + tx * 4; };
-    simt_epilogue<TM, GN>(p, acc, out_row, out_col, VEC, z, tile, sm.last);
-}
-
-template <int BM, int BN, bool FUSED, bool VEC>
-__global__ void __launch_bounds__(kThreads, 2)
-sgemm_simt_kernel(SimtArgs p) {
-    __shared__ __align__(16) SimtSmem<BM, BN> sm;
-    simt_tile<BM, BN, FUSED, VEC ? 1 : 0>(p, (int64_t)blockIdx.y * BM, (int64_t)blockIdx.x * BN, blockIdx.z,
-                                          blockIdx.y * gridDim.x + blockIdx.x, sm);
-}
-
 // ---------------------------------------------------------------------------
-// 128 x 128 tiles on a cp.async pipeline (the plan's 128 x 128 FP32 tile).
+// The tile kernel: packed multiply-adds on a cp.async ring.
 //
-// 128 threads (four warps of 64 x 64), each owning 8 x 16 outputs: rows
-// wm*64 + lm + 8i (i < 8), columns wn*64 + 4 ln + 16 j + {0..3} (j < 4), with
-// lane = 4 lm + ln. Two CTAs per SM. Tiles of A (128 rows x 32 k, row-major,
-// rows padded to 36 floats) and B (32 k x 128 columns) arrive by cp.async
-// (16-byte copies where K and N are multiples of 4 and A, B, C are 16-byte
-// aligned; 4-byte copies otherwise) into a ring of three stages, so no thread
-// stages operands through registers or transposes them. Per four k's a
-// thread reads its 8 rows of A as 128-bit loads (4 k's each; a warp's eight
-// rows fall on eight bank groups) and, per k, 16 values of B (four 128-bit
-// loads, 64 contiguous bytes per warp): 512 multiply-adds per 24 shared loads.
+// A warp owns 8 RT x 4 LT outputs; lane = 4 lm + ln holds rows lm + 8 i (i <
+// RT) and columns 4 ln + 16 j + {0..3} (j < LT / 4) of them as RT x LT / 2
+// packed pairs. Stages of BK k's of A (rows padded to BK + 4 floats, so a
+// warp's eight rows fall on eight bank groups) and B arrive by cp.async in the
+// widest copies the operand's alignment allows (SimtArgs::wa, wb).
 //
-// Arithmetic: as in the kernel above, every output is one chain over k in
-// increasing order (the stage loop, then four k's per A load, in order), so
-// C is the same bit for bit; copies outside the matrix fill zeros.
+// Bound by the FMA pipe: 128 multiply-adds per clock and SM, 74.4 TFLOP/s at
+// 1965 MHz. fma.rn.f32x2 issues half as many instructions for the same pipe
+// cycles, which leaves issue slots for the shared loads; operands are
+// duplicated into pairs from A, RT moves per RT LT / 2 instructions. Register
+// operand conflicts hold a loop of nothing but these instructions to 88-91 %
+// of the peak by the order they come in. Measured at 4096^3, 128 x 128 tiles,
+// no K split: 2358 us (58.3 TFLOP/s) against 3011 us with scalar multiply-adds
+// and fragments read from shared memory where they are used; 2620 us with
+// packed ones alone, 2477 us with fragments read one k ahead across stage
+// boundaries, 2397 us with the column-snake order below (row by row 2477,
+// row snake 2459, 2 x 2 blocks 2479), 2358 us with bounds tested per stage
+// rather than per copy. A sizes of K and N that are not multiples of 4 cost 12 %
+// over their aligned neighbours (776 x 1531 x 899 and 776 x 1532 x 900: 75.2
+// and 67.4 us; 108.6 and 101.7 us before, 94.7 us with bounds per copy).
+//
+// Arithmetic: every output is one chain over k in increasing order, so C is
+// the same bit for bit whatever the tile; copies past kend write zeros.
 // ---------------------------------------------------------------------------
-namespace cpk {
-constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3;
-constexpr int AST = BK + 4;                    // A row stride (floats): eight rows on eight bank groups
-constexpr int A_FLOATS = BM * AST;
-constexpr int B_FLOATS = BK * BN;
-constexpr int STAGE_FLOATS = A_FLOATS + B_FLOATS;
-constexpr int SMEM = STAGES * STAGE_FLOATS * 4;
-// LT = outputs per thread along N: 16 (128 threads, warps of 64 x 64) or 8
-// (256 threads, warps of 64 x 32); eight rows per thread either way.
-template <int LT> struct Shape {
-    static constexpr int THREADS = LT == 16 ? 128 : 256;
-    static constexpr int WARPS_N = LT == 16 ? 2 : 4;
-    static constexpr int WN = BN / WARPS_N;    // warp tile columns
+template <int BM_, int BN_, int RT_, int LT_, int BK_, int STAGES_, int CTAS_>
+struct CpCfg {
+    static constexpr int BM = BM_, BN = BN_, RT = RT_, LT = LT_, BK = BK_, STAGES = STAGES_, CTAS = CTAS_;
+    static constexpr int WM = 8 * RT, WN = 4 * LT;  // warp tile
+    static constexpr int WARPS_N = BN / WN;
+    static constexpr int THREADS = 32 * (BM / WM) * WARPS_N;
+    static constexpr int AST = BK + 4;             // A row stride (floats): eight rows on eight bank groups
+    static constexpr int A_FLOATS = BM * AST;
+    static constexpr int B_FLOATS = BK * BN;
+    static constexpr int STAGE_FLOATS = A_FLOATS + B_FLOATS;
+    static constexpr int SMEM = STAGES * STAGE_FLOATS * 4;
+    static_assert(THREADS >= BN && THREADS >= BK && BK % 2 == 0 && STAGES >= 3, "tile configuration");
 };
-}  // namespace cpk
 
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, int src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+// The plans' tiles. 128 x 128: 8 x 16 outputs a thread (255 registers, two
+// CTAs an SM). 128 x 64: 8 x 8 a thread. 64 x 64: 4 x 8 a thread and four CTAs
+// an SM, which a small C needs to fill the GPU. Measured, per configuration
+// (4096^3 unsplit, 128 x 128: BK 16 x 4 stages 2358 us, 16 x 3 2377, 8 x 6
+// 2496; 2048^3 split 2, 128 x 64: 32 x 3, two CTAs 344, 16 x 4, three CTAs
+// 350; 2048^3 unsplit, 64 x 64: 32 x 3 354, 16 x 4 394, 4 x 4 a thread 475).
+template <int BM, int BN> struct CpTileSel;
+template <> struct CpTileSel<128, 128> { using T = CpCfg<128, 128, 8, 16, 16, 4, 2>; };
+template <> struct CpTileSel<128, 64> { using T = CpCfg<128, 64, 8, 8, 32, 3, 2>; };
+template <> struct CpTileSel<64, 64> { using T = CpCfg<64, 64, 4, 8, 32, 3, 4>; };
+template <int BM, int BN> using CpTile = typename CpTileSel<BM, BN>::T;
+
+// Two FP32 lanes in a 64-bit register: the packed arithmetic of sm_100
+// (fma.rn.f32x2), each lane rounded exactly as the scalar instruction rounds
+// it.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
-__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src, int src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+// c + a * b per lane: one fused multiply-add, or (SCALAR variant) a multiply,
+// then an add, each rounded. The latter stays on scalar instructions: the
+// compiler contracts a packed multiply and add into the fused form (seen in
+// results), which it never does to __fmul_rn and __fadd_rn.
+template <bool FUSED>
+__device__ __forceinline__ f32x2 mac2(f32x2 a, f32x2 b, f32x2 c) {
+    if constexpr (FUSED) {
+        f32x2 r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+        return r;
+    } else {
+        float a0, a1, b0, b1, c0, c1;
+        unpack2(a, a0, a1);
+        unpack2(b, b0, b1);
+        unpack2(c, c0, c1);
+        return pack2(__fadd_rn(c0, __fmul_rn(a0, b0)), __fadd_rn(c1, __fmul_rn(a1, b1)));
+    }
+}
+
+// W floats from global to shared memory; with `bytes`, that many are read and
+// the rest of the 4 W written as zeros.
+template <int W>
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, int bytes) {
+    if constexpr (W == 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;\n" ::"r"(dst), "l"(src), "r"(bytes), "n"(4 * W) : "memory");
+}
+template <int W>
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src) {
+    if constexpr (W == 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(dst), "l"(src), "n"(4 * W) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-template <bool FUSED, bool VEC, int LT>
-__global__ void __launch_bounds__(cpk::Shape<LT>::THREADS, 2)
-sgemm_simt_cp_kernel(SimtArgs p) {
-    using namespace cpk;
-    constexpr int THREADS = Shape<LT>::THREADS, WARPS_N = Shape<LT>::WARPS_N, WN = Shape<LT>::WN;
+template <class Cf, bool FUSED>
+__device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int64_t n0, int z, unsigned tile,
+                                             float* smem, int& last_flag) {
+    constexpr int BM = Cf::BM, BN = Cf::BN, BK = Cf::BK, STAGES = Cf::STAGES, THREADS = Cf::THREADS;
+    constexpr int LT = Cf::LT, RT = Cf::RT;
+    constexpr int AST = Cf::AST;
     constexpr int GN = LT / 4;                 // float4 groups per thread row
-    extern __shared__ __align__(16) float smem[];
-    __shared__ int last_flag;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp / WARPS_N, wn = warp % WARPS_N;
+    const int wm = warp / Cf::WARPS_N, wn = warp % Cf::WARPS_N;
     const int lm = lane >> 2, ln = lane & 3;
-    const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-    const int z = blockIdx.z;
     const int64_t M = p.M, N = p.N, K = p.K;
     const int64_t kbeg = (int64_t)z * p.kchunk;
     const int64_t kend = min(K, kbeg + p.kchunk);
@@ -370,130 +253,192 @@ sgemm_simt_cp_kernel(SimtArgs p) {
     const float* __restrict__ B = p.B;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
 
-    // Stage `buf` <- A[m0.., k0..k0+BK), B[k0..k0+BK, n0..); zeros outside the
-    // matrix and past kend (a copy of 0 source bytes reads nothing; its source
-    // address is kept inside the operand anyway).
-    auto load_stage = [&](int buf, int64_t k0) {
-        const uint32_t a_s = sbase + (uint32_t)(buf * STAGE_FLOATS) * 4u;
-        const uint32_t b_s = a_s + (uint32_t)A_FLOATS * 4u;
-        if constexpr (VEC) {
-#pragma unroll
-            for (int j = 0; j < BM * BK / 4 / THREADS; j++) {       // 16-byte chunks of A
-                const int c = tid + j * THREADS;
-                const int row = c >> 3, ch = c & 7;
-                const int64_t gm = m0 + row, gk = k0 + ch * 4;
-                const bool ok = gm < M && gk < kend;
-                cp_async_16(a_s + (uint32_t)(row * AST + ch * 4) * 4u, ok ? A + gm * K + gk : A, ok ? 16 : 0);
-            }
-#pragma unroll
-            for (int j = 0; j < BK * BN / 4 / THREADS; j++) {       // 16-byte chunks of B
-                const int c = tid + j * THREADS;
-                const int row = c >> 5, ch = c & 31;
-                const int64_t gk = k0 + row, gn = n0 + ch * 4;
-                const bool ok = gk < kend && gn < N;
-                cp_async_16(b_s + (uint32_t)(row * BN + ch * 4) * 4u, ok ? B + gk * N + gn : B, ok ? 16 : 0);
-            }
-        } else {
-#pragma unroll 8
-            for (int j = 0; j < BM * BK / THREADS; j++) {           // elements of A
-                const int c = tid + j * THREADS;
-                const int row = c >> 5, col = c & 31;
-                const int64_t gm = m0 + row, gk = k0 + col;
-                const bool ok = gm < M && gk < kend;
-                cp_async_4(a_s + (uint32_t)(row * AST + col) * 4u, ok ? A + gm * K + gk : A, ok ? 4 : 0);
-            }
-#pragma unroll 8
-            for (int j = 0; j < BK * BN / THREADS; j++) {           // elements of B
-                const int c = tid + j * THREADS;
-                const int row = c >> 7, col = c & 127;
-                const int64_t gk = k0 + row, gn = n0 + col;
-                const bool ok = gk < kend && gn < N;
-                cp_async_4(b_s + (uint32_t)(row * BN + col) * 4u, ok ? B + gk * N + gn : B, ok ? 4 : 0);
+    // Stage `buf` <- A[m0.., k0..k0+BK), B[k0..k0+BK, n0..) in copies of W
+    // floats, the widest that every row start allows. A stage wholly inside the
+    // slice and the matrix needs no bounds; otherwise copies outside read
+    // nothing and write zeros (their source address is kept inside the operand).
+    const bool inside = m0 + BM <= M && n0 + BN <= N;
+    auto load_a_stage = [&]<int W, bool EDGE>(uint32_t a_s, int64_t k0) {
+        constexpr int CPR = BK / W, RPP = THREADS / CPR;            // copies per row, rows per pass
+        const int row = tid / CPR, col = tid % CPR * W;
+        const float* src = A + (m0 + row) * K + k0 + col;
+        const uint32_t dst = a_s + (uint32_t)(row * AST + col) * 4u;
+        const int64_t step = (int64_t)RPP * K;
+#pragma unroll(W == 1 ? 8 : 16)
+        for (int j = 0; j < BM / RPP; j++, src += step) {
+            if constexpr (EDGE) {
+                const bool ok = k0 + col < kend && m0 + row + j * RPP < M;
+                cp_async<W>(dst + (uint32_t)(j * RPP * AST * 4), ok ? src : A, ok ? 4 * W : 0);
+            } else {
+                cp_async<W>(dst + (uint32_t)(j * RPP * AST * 4), src);
             }
         }
     };
+    auto load_b_stage = [&]<int W, bool EDGE>(uint32_t b_s, int64_t k0) {
+        constexpr int CPR = BN / W, RPP = THREADS / CPR;
+        const int row = tid / CPR, col = tid % CPR * W;
+        const float* src = B + (k0 + row) * N + n0 + col;
+        const uint32_t dst = b_s + (uint32_t)(row * BN + col) * 4u;
+        const int64_t step = (int64_t)RPP * N;
+#pragma unroll(W == 1 ? 8 : 16)
+        for (int j = 0; j < BK / RPP; j++, src += step) {
+            if constexpr (EDGE) {
+                const bool ok = k0 + row + j * RPP < kend && n0 + col < N;
+                cp_async<W>(dst + (uint32_t)(j * RPP * BN * 4), ok ? src : B, ok ? 4 * W : 0);
+            } else {
+                cp_async<W>(dst + (uint32_t)(j * RPP * BN * 4), src);
+            }
+        }
+    };
+    auto load_stage = [&](int buf, int64_t k0) {
+        const uint32_t a_s = sbase + (uint32_t)(buf * Cf::STAGE_FLOATS) * 4u;
+        const uint32_t b_s = a_s + (uint32_t)Cf::A_FLOATS * 4u;
+        if (inside && k0 + BK <= kend) {
+            if (p.wa == 4) load_a_stage.template operator()<4, false>(a_s, k0);
+            else if (p.wa == 2) load_a_stage.template operator()<2, false>(a_s, k0);
+            else load_a_stage.template operator()<1, false>(a_s, k0);
+            if (p.wb == 4) load_b_stage.template operator()<4, false>(b_s, k0);
+            else if (p.wb == 2) load_b_stage.template operator()<2, false>(b_s, k0);
+            else load_b_stage.template operator()<1, false>(b_s, k0);
+        } else {
+            if (p.wa == 4) load_a_stage.template operator()<4, true>(a_s, k0);
+            else if (p.wa == 2) load_a_stage.template operator()<2, true>(a_s, k0);
+            else load_a_stage.template operator()<1, true>(a_s, k0);
+            if (p.wb == 4) load_b_stage.template operator()<4, true>(b_s, k0);
+            else if (p.wb == 2) load_b_stage.template operator()<2, true>(b_s, k0);
+            else load_b_stage.template operator()<1, true>(b_s, k0);
+        }
+    };
 
-    float acc[8][LT];
+    f32x2 acc[RT][LT / 2];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < RT; i++)
 #pragma unroll
-        for (int j = 0; j < LT; j++) acc[i][j] = 0.f;
+        for (int j = 0; j < LT / 2; j++) acc[i][j] = 0ull;
+
+    // Operand fragments of two k's: rows lm + 8 i of A, column quads of B.
+    float2 fa[2][RT];
+    f32x2 fb[2][LT / 2];
+    const int a_off = (wm * Cf::WM + lm) * AST, b_off = Cf::A_FLOATS + wn * Cf::WN + ln * 4;
+    auto load_a = [&](int set, const float* st, int k) {
+#pragma unroll
+        for (int i = 0; i < RT; i++) fa[set][i] = *reinterpret_cast<const float2*>(st + a_off + i * 8 * AST + k);
+    };
+    auto load_b = [&](int set, const float* st, int k) {
+#pragma unroll
+        for (int j = 0; j < GN; j++) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(st + b_off + k * BN + j * 16);
+            fb[set][2 * j] = v.x;
+            fb[set][2 * j + 1] = v.y;
+        }
+    };
 
 #pragma unroll
     for (int st = 0; st < STAGES - 1; st++) {
         if (st < ntiles) load_stage(st, kbeg + (int64_t)st * BK);
         cp_async_commit();
     }
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();
+    load_a(0, smem, 0);
+    load_b(0, smem, 0);
+    // Fragments of k + 1 are read while k's products run; the last k of a stage
+    // reads the next stage's first ones, after the barrier that says that stage
+    // has landed and that every warp has read the stage before it, whose buffer
+    // the next copies take. (Past the last stage it reads a stale buffer, unused.)
+    int buf = 0;
     for (int64_t t = 0; t < ntiles; t++) {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();                       // stage t landed; stage t - 1 is no longer read
-        const int64_t tn = t + STAGES - 1;
-        if (tn < ntiles) load_stage((int)(tn % STAGES), kbeg + tn * BK);
-        cp_async_commit();
-        const float* As = smem + (int)(t % STAGES) * STAGE_FLOATS;
-        const float* Bs = As + A_FLOATS;
-        const float* a_base = As + (wm * 64 + lm) * AST;
-        const float* b_base = Bs + wn * WN + ln * 4;
-        // Two of the eight four-k groups per loop body: a fully unrolled stage
-        // outgrows the instruction cache.
-#pragma unroll 2
-        for (int k4 = 0; k4 < BK / 4; k4++) {
-            float4 a[8];
+        const float* cur = smem + buf * Cf::STAGE_FLOATS;
+        const int nbuf = buf + 1 == STAGES ? 0 : buf + 1;
+        const float* nxt = smem + nbuf * Cf::STAGE_FLOATS;
 #pragma unroll
-            for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4*>(a_base + i * 8 * AST + k4 * 4);
-#pragma unroll
-            for (int kk = 0; kk < 4; kk++) {
-                float b[LT];
-#pragma unroll
-                for (int j = 0; j < GN; j++) {
-                    const float4 v = *reinterpret_cast<const float4*>(b_base + (k4 * 4 + kk) * BN + j * 16);
-                    b[4 * j + 0] = v.x; b[4 * j + 1] = v.y; b[4 * j + 2] = v.z; b[4 * j + 3] = v.w;
-                }
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float av = kk == 0 ? a[i].x : kk == 1 ? a[i].y : kk == 2 ? a[i].z : a[i].w;
-#pragma unroll
-                    for (int j = 0; j < LT; j++) acc[i][j] = mac<FUSED>(av, b[j], acc[i][j]);
-                }
+        for (int k = 0; k < BK; k++) {
+            if (k + 1 < BK) {
+                load_b((k + 1) & 1, cur, k + 1);
+                if ((k & 1) == 1) load_a(((k + 1) >> 1) & 1, cur, k + 1);
+            } else {
+                cp_async_wait<STAGES - 3>();
+                __syncthreads();
+                const int64_t tn = t + STAGES - 1;
+                if (tn < ntiles) load_stage(buf == 0 ? STAGES - 1 : buf - 1, kbeg + tn * BK);
+                cp_async_commit();
+                load_b(0, nxt, 0);
+                load_a(0, nxt, 0);
             }
+            f32x2 aa[RT];
+#pragma unroll
+            for (int i = 0; i < RT; i++) {
+                const float2 v = fa[(k >> 1) & 1][i];
+                aa[i] = (k & 1) ? pack2(v.y, v.y) : pack2(v.x, v.x);
+            }
+            // Column by column, rows down and up in turn: neighbouring
+            // instructions share an operand.
+#pragma unroll
+            for (int j = 0; j < LT / 2; j++)
+#pragma unroll
+                for (int q = 0; q < RT; q++) {
+                    const int i = (j & 1) ? RT - 1 - q : q;
+                    acc[i][j] = mac2<FUSED>(aa[i], fb[k & 1][j], acc[i][j]);
+                }
         }
+        buf = nbuf;
     }
     cp_async_wait<0>();
 
     // Steps past kend multiplied zeros: the chains are those over [kbeg, kend).
-    auto out_row = [&](int i) { return m0 + wm * 64 + lm + 8 * i; };
-    auto out_col = [&](int g) { return n0 + wn * WN + ln * 4 + 16 * g; };
-    simt_epilogue<8, GN>(p, acc, out_row, out_col, VEC, z, blockIdx.y * gridDim.x + blockIdx.x, last_flag);
+    float out[RT][LT];
+#pragma unroll
+    for (int i = 0; i < RT; i++)
+#pragma unroll
+        for (int j = 0; j < LT / 2; j++) unpack2(acc[i][j], out[i][2 * j], out[i][2 * j + 1]);
+    auto out_row = [&](int i) { return m0 + wm * Cf::WM + lm + 8 * i; };
+    auto out_col = [&](int g) { return n0 + wn * Cf::WN + ln * 4 + 16 * g; };
+    simt_epilogue<RT, GN>(p, out, out_row, out_col, p.wc == 4, z, tile, last_flag);
+}
+
+template <class Cf, bool FUSED>
+__global__ void __launch_bounds__(Cf::THREADS, Cf::CTAS)
+sgemm_simt_cp_kernel(SimtArgs p) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int last_flag;
+    simt_cp_tile<Cf, FUSED>(p, (int64_t)blockIdx.y * Cf::BM, (int64_t)blockIdx.x * Cf::BN, blockIdx.z,
+                            blockIdx.y * gridDim.x + blockIdx.x, smem, last_flag);
 }
 
 // Grouped launch: one persistent kernel over a list of (problem, tile, K
 // slice) units taken from an atomic counter, heaviest units first. Each unit
 // is exactly the tile a per-GEMM launch of that problem computes, so results
 // are identical to running the problems one by one.
-template <int BM, int BN, bool FUSED>
-__global__ void __launch_bounds__(kThreads, 2)
+template <class Cf, bool FUSED>
+__global__ void __launch_bounds__(Cf::THREADS, Cf::CTAS)
 sgemm_simt_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUnit* __restrict__ units, int nunits,
                           unsigned* next) {
-    __shared__ __align__(16) SimtSmem<BM, BN> sm;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int last_flag;
     __shared__ int s_unit;
+    // Thread 0 fetches the next unit's number while the current one runs.
+    unsigned fetched = threadIdx.x == 0 ? atomicAdd(next, 1u) : 0u;
     for (;;) {
-        if (threadIdx.x == 0) s_unit = (int)atomicAdd(next, 1u);
-        __syncthreads();
+        if (threadIdx.x == 0) s_unit = (int)min(fetched, (unsigned)nunits);
+        __syncthreads();                     // also: the last unit's stages are no longer read
         const int u = s_unit;
-        __syncthreads();
         if (u >= nunits) break;
+        if (threadIdx.x == 0) fetched = atomicAdd(next, 1u);
         const GroupUnit w = units[u];
-        const GroupProblem& P = probs[w.problem];
-        const unsigned tile = (unsigned)w.tm * (unsigned)P.tiles_n + (unsigned)w.tn;
-        simt_tile<BM, BN, FUSED, 2>(P.a, (int64_t)w.tm * BM, (int64_t)w.tn * BN, w.z, tile, sm, P.vec != 0);
+        const SimtArgs a = probs[w.problem].a;
+        const unsigned tile = (unsigned)w.tm * (unsigned)probs[w.problem].tiles_n + (unsigned)w.tn;
+        simt_cp_tile<Cf, FUSED>(a, (int64_t)w.tm * Cf::BM, (int64_t)w.tn * Cf::BN, w.z, tile, smem, last_flag);
     }
 }
 
-// Split-K reduction for plans of three or more K slices: the slices wrote
-// their partial products ([slice][M][N]); each thread sums one output (T =
+// Split-K reduction of the single launches (grouped launches sum in the last
+// CTA of a tile to arrive, simt_epilogue): the slices wrote their partial
+// products ([slice][M][N]); each thread sums one output (T =
 // float) or four adjacent ones (T = float4) over the slices in slice order --
 // the order of the in-kernel fixup and of the reference's panel sum
-// C = p0 + p1 + ... -- so C is the same bit for bit. Bound by the reads of the
+// C = p0 + p1 + ... -- so C is the same bit for bit. Two slices go this way too:
+// clearing and counting arrivals costs more than the second launch (128 x 64
+// tiles, two slices: 2048^3 344 -> 331 us, 1024^3 62 -> 53, 300^3 29 -> 13). Bound by the reads of the
 // partials, splits * M * N floats, from L2 while they fit (126 MB). Measured
 // (ncu): 1024^2 x 8 slices 7.8 us (4.8 TB/s), 777 x 901 x 8 6.3 us, 512^2 x 16
 // 5.4 us, 256^2 x 8 3.1 us; a grid-stride loop with a fixed batch of 64
@@ -513,7 +458,7 @@ cudaError_t launch_splitk_reduce(const float* partial, float* C, int64_t n, int 
     if (splits <= 4) simt_splitk_reduce_kernel<3><<<blocks, 256, 0, s>>>(src, dst, n, splits);
     else if (splits <= 8) simt_splitk_reduce_kernel<7><<<blocks, 256, 0, s>>>(src, dst, n, splits);
     else if (sizeof(T) > 4 || splits <= 16) simt_splitk_reduce_kernel<15><<<blocks, 256, 0, s>>>(src, dst, n, splits);
-    else simt_splitk_reduce_kernel<63><<<blocks, 256, 0, s>>>(src, dst, n, splits);
+    else simt_splitk_reduce_kernel<sizeof(T) > 4 ? 15 : 63><<<blocks, 256, 0, s>>>(src, dst, n, splits);
     return cudaGetLastError();
 }
 
@@ -529,9 +474,6 @@ cudaError_t splitk_reduce(const SimtArgs& a, cudaStream_t s) {
     return launch_splitk_reduce<float>(a.partial, a.C, n, a.splits, s);
 }
 
-// Slices at or above which the partials are summed by the reduction kernel.
-constexpr int kReduceAfterSplits = 3;
-
 // Raises a kernel's dynamic shared memory limit once per device.
 template <typename Kern>
 cudaError_t smem_limit_once(Kern kern, int bytes, std::atomic<uint64_t>& done) {
@@ -544,45 +486,26 @@ cudaError_t smem_limit_once(Kern kern, int bytes, std::atomic<uint64_t>& done) {
     return e;
 }
 
-template <bool FUSED, bool VEC, int LT>
-cudaError_t launch_cp_lt(const SimtArgs& a, dim3 grid, cudaStream_t s) {
-    static std::atomic<uint64_t> done{0};
-    cudaError_t e = smem_limit_once(sgemm_simt_cp_kernel<FUSED, VEC, LT>, cpk::SMEM, done);
-    if (e != cudaSuccess) return e;
-    sgemm_simt_cp_kernel<FUSED, VEC, LT><<<grid, cpk::Shape<LT>::THREADS, cpk::SMEM, s>>>(a);
-    return cudaGetLastError();
-}
-
-// 8 x 16 outputs per thread: measured at 4096^3 (45.7 against 44.7 TFLOP/s)
-// and 2048^3 (40.2 against 38.5) ahead of 8 x 8 with 256 threads.
-template <bool FUSED, bool VEC>
+template <class Cf, bool FUSED>
 cudaError_t launch_cp(const SimtArgs& a, dim3 grid, cudaStream_t s) {
-    return launch_cp_lt<FUSED, VEC, 16>(a, grid, s);
+    static std::atomic<uint64_t> done{0};
+    cudaError_t e = smem_limit_once(sgemm_simt_cp_kernel<Cf, FUSED>, Cf::SMEM, done);
+    if (e != cudaSuccess) return e;
+    sgemm_simt_cp_kernel<Cf, FUSED><<<grid, Cf::THREADS, Cf::SMEM, s>>>(a);
+    return cudaGetLastError();
 }
 
 template <int BM, int BN>
 cudaError_t launch_tile(const SimtArgs& args, int variant, cudaStream_t s) {
+    using Cf = CpTile<BM, BN>;
     SimtArgs a = args;
-    a.reduce_after = (a.splits >= kReduceAfterSplits) ? 1 : 0;
-    dim3 grid((unsigned)((a.N + BN - 1) / BN), (unsigned)((a.M + BM - 1) / BM), (unsigned)a.splits);
-    const bool vec = (a.K % 4 == 0) && (a.N % 4 == 0) &&
-                     ((uintptr_t)a.A % 16 == 0) && ((uintptr_t)a.B % 16 == 0) && ((uintptr_t)a.C % 16 == 0);
-    const bool fused = (variant != MAXMULSK_FP32_SCALAR);
+    a.reduce_after = a.splits > 1 ? 1 : 0;
+    simt_set_widths(a);
+    const dim3 grid((unsigned)((a.N + BN - 1) / BN), (unsigned)((a.M + BM - 1) / BM), (unsigned)a.splits);
     cudaError_t e;
     {
         PhaseScope ps(kPhaseGemm, s);
-        if constexpr (BM == cpk::BM && BN == cpk::BN) {
-            if (fused && vec) e = launch_cp<true, true>(a, grid, s);
-            else if (fused) e = launch_cp<true, false>(a, grid, s);
-            else if (vec) e = launch_cp<false, true>(a, grid, s);
-            else e = launch_cp<false, false>(a, grid, s);
-        } else {
-            if (fused && vec) sgemm_simt_kernel<BM, BN, true, true><<<grid, kThreads, 0, s>>>(a);
-            else if (fused) sgemm_simt_kernel<BM, BN, true, false><<<grid, kThreads, 0, s>>>(a);
-            else if (vec) sgemm_simt_kernel<BM, BN, false, true><<<grid, kThreads, 0, s>>>(a);
-            else sgemm_simt_kernel<BM, BN, false, false><<<grid, kThreads, 0, s>>>(a);
-            e = cudaGetLastError();
-        }
+        e = variant != MAXMULSK_FP32_SCALAR ? launch_cp<Cf, true>(a, grid, s) : launch_cp<Cf, false>(a, grid, s);
     }
     if (e != cudaSuccess || !a.reduce_after) return e;
     PhaseScope ps(kPhaseReduce, s);
@@ -628,34 +551,35 @@ maxmulsk_status simt_run(const float* dA, const float* dB, float* dC, size_t M, 
         set_error_message("workspace too small for the SIMT plan");
         return MAXMULSK_ERR_INVALID;
     }
-    if (a.splits > 1 && a.splits < kReduceAfterSplits) {
-        // The split-K arrival counters must start at zero on every call (with
-        // more slices, simt_splitk_reduce_kernel sums them and no counter is read).
-        const size_t tiles = (size_t)((M + plan.tile_m - 1) / plan.tile_m) * ((N + plan.tile_n - 1) / plan.tile_n);
-        maxmulsk_status st =
-            cuda_status(cudaMemsetAsync(a.counters, 0, tiles * sizeof(unsigned), s), "cudaMemsetAsync(counters)");
-        if (st != MAXMULSK_OK) return st;
-    }
     return cuda_status(simt_launch(a, plan.tile_m, plan.tile_n, plan.variant, s), "sgemm_simt launch");
 }
 
 namespace {
+template <class Cf, bool FUSED>
+cudaError_t launch_grouped(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next, int sms,
+                           cudaStream_t s) {
+    static std::atomic<uint64_t> done{0};
+    cudaError_t e = smem_limit_once(sgemm_simt_grouped_kernel<Cf, FUSED>, Cf::SMEM, done);
+    if (e != cudaSuccess) return e;
+    const int slots = Cf::CTAS * sms;
+    sgemm_simt_grouped_kernel<Cf, FUSED><<<nunits < slots ? nunits : slots, Cf::THREADS, Cf::SMEM, s>>>(probs, units,
+                                                                                                      nunits, next);
+    return cudaGetLastError();
+}
 template <int BM, int BN>
 cudaError_t launch_grouped_tile(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,
-                                int grid, int variant, cudaStream_t s) {
-    if (variant == MAXMULSK_FP32_SCALAR)
-        sgemm_simt_grouped_kernel<BM, BN, false><<<grid, kThreads, 0, s>>>(probs, units, nunits, next);
-    else
-        sgemm_simt_grouped_kernel<BM, BN, true><<<grid, kThreads, 0, s>>>(probs, units, nunits, next);
-    return cudaGetLastError();
+                                int variant, int sms, cudaStream_t s) {
+    using Cf = CpTile<BM, BN>;
+    return variant != MAXMULSK_FP32_SCALAR ? launch_grouped<Cf, true>(probs, units, nunits, next, sms, s)
+                                           : launch_grouped<Cf, false>(probs, units, nunits, next, sms, s);
 }
 }  // namespace
 
 cudaError_t simt_grouped_launch(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,
-                                int tile_m, int tile_n, int variant, int grid, cudaStream_t s) {
-    if (tile_m == 128 && tile_n == 128) return launch_grouped_tile<128, 128>(probs, units, nunits, next, grid, variant, s);
-    if (tile_m == 128 && tile_n == 64) return launch_grouped_tile<128, 64>(probs, units, nunits, next, grid, variant, s);
-    if (tile_m == 64 && tile_n == 64) return launch_grouped_tile<64, 64>(probs, units, nunits, next, grid, variant, s);
+                                int tile_m, int tile_n, int variant, int sms, cudaStream_t s) {
+    if (tile_m == 128 && tile_n == 128) return launch_grouped_tile<128, 128>(probs, units, nunits, next, variant, sms, s);
+    if (tile_m == 128 && tile_n == 64) return launch_grouped_tile<128, 64>(probs, units, nunits, next, variant, sms, s);
+    if (tile_m == 64 && tile_n == 64) return launch_grouped_tile<64, 64>(probs, units, nunits, next, variant, sms, s);
     return cudaErrorInvalidValue;
 }
 
@@ -682,8 +606,8 @@ cudaError_t simt_grouped_launch(const GroupProblem* probs, const GroupUnit* unit
 //     before any stream capture. The address is kept per CUDA context, so a
 //     context made after cudaDeviceReset resolves it again (its first call,
 //     too, belongs before any capture);
-//   * the array keeps the last call's contents; the arrival counters that
-//     must start at zero are cleared on the stream before every launch.
+//   * the array keeps the last call's contents; every launch writes what it
+//     reads.
 // ---------------------------------------------------------------------------
 static __device__ __align__(256) unsigned char g_simt_static_scratch[MAXMULSK_STATIC_SCRATCH_BYTES];
 

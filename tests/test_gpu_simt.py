@@ -243,3 +243,20 @@ def test_row_shards_reassemble_the_product(cuda, oracle_mod, world):
     st, whole, _ = run_plan(torch, A, B, M, K, N, plan, dA=dA, dB=dB)
     assert st == 0 and mm.stream_status() == 0
     assert np.array_equal(bits(dC.cpu().numpy()), bits(whole.ravel()))
+
+
+# Copies of 4, 2 and 1 floats per operand (row lengths and pointer offsets),
+# stages wholly inside the matrix and at its edges, both multiply-add forms.
+@pytest.mark.parametrize("tile", TILES)
+@pytest.mark.parametrize("variant", [mm.FP32_FMA, mm.FP32_SCALAR])
+@pytest.mark.parametrize("K,N,off", [(96, 160, 0), (98, 160, 0), (96, 162, 0), (99, 161, 0), (96, 160, 1), (96, 160, 2)])
+def test_copy_widths_bit_exact(cuda, oracle_mod, tile, variant, K, N, off):
+    M = 161
+    A, B = _inputs(oracle_mod, M, K, N, seed=70)
+    pad = np.zeros(off, np.float32)
+    bA, bB = to_dev(cuda, np.concatenate([pad, A.ravel()])), to_dev(cuda, np.concatenate([pad, B.ravel()]))
+    plan = mm.make_plan(mm.Precision.FP32, tile[0], tile[1], 1, variant)
+    st, C, bands = run_plan(cuda, A, B, M, K, N, plan, dA=bA[off:], dB=bB[off:], offset=off)
+    assert st == 0 and bands, mm.last_error_message()
+    ref = oracle_mod.sgemm_panels(A, B, M, K, N, fma=variant == mm.FP32_FMA)
+    assert np.array_equal(bits(C), bits(ref))
