@@ -458,7 +458,7 @@ cudaError_t launch_splitk_reduce(const float* partial, float* C, int64_t n, int 
     if (splits <= 4) simt_splitk_reduce_kernel<3><<<blocks, 256, 0, s>>>(src, dst, n, splits);
     else if (splits <= 8) simt_splitk_reduce_kernel<7><<<blocks, 256, 0, s>>>(src, dst, n, splits);
     else if (sizeof(T) > 4 || splits <= 16) simt_splitk_reduce_kernel<15><<<blocks, 256, 0, s>>>(src, dst, n, splits);
-    else simt_splitk_reduce_kernel<sizeof(T) > 4 ? 15 : 63><<<blocks, 256, 0, s>>>(src, dst, n, splits);
+    else simt_splitk_reduce_kernel<(sizeof(T) > 4 ? 15 : 63)><<<blocks, 256, 0, s>>>(src, dst, n, splits);
     return cudaGetLastError();
 }
 
