@@ -11,6 +11,7 @@
 //                   exhaustive search (autotune.cpp) runs instead; the
 //                   reference's counterpart is the MAXMULSK_BLOCKING sweep
 //                   that overrides its table (gemm_tuning.cpp:66-78, 96-100)
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -144,6 +145,41 @@ bool parse_config_env(maxmulsk_plan& out) {
     return true;
 }
 
+// The tile for an FP32 plan's K split. C is the same bit for bit on every tile,
+// so the learned model's say is kept for the K split, which sets the rounding,
+// and the tile follows the kernels' cost: with q = ceil(tiles * slices / SMs)
+// units on the busiest SM, rounds of `ctas` resident units take
+//     per_round + slice length * resident * tile_m tile_n / (128 FMA per clock * rate)
+// with the FMA-pipe share `rate` that a full SM, or a partly filled one,
+// reaches. Constants fitted to 208 shapes x 8 K splits timed on B200 (M, N, K
+// log-uniform in [1, 16384] and [32, 4096]): the tile chosen costs 0.14 % over
+// the best of the three on average (9.6 % at most), against 1.4 % / 27 % / 75 %
+// for 64x64 / 128x64 / 128x128 everywhere. On the model's own tiles, chosen for
+// slower kernels, those shapes took 7.2 % over the exhaustive best in total
+// time, with this rule 2.6 %; 4096^3 (two slices) 2535 -> 2381 us.
+maxmulsk_plan with_best_fp32_tile(size_t M, size_t K, size_t N, maxmulsk_plan p, int sms) {
+    struct Tile { int m, n, ctas; double part, full, per_round_us; };
+    static const Tile tiles[3] = {{128, 128, 2, 0.74, 0.81, 3.4}, {128, 64, 2, 0.69, 0.75, 2.0}, {64, 64, 4, 0.68, 0.66, 1.3}};
+    if (sms <= 0) sms = 148;
+    const double us_per_mac = 1.0 / (128.0 * 1965.0);
+    const double len = (double)slice_len(K, p.split_k), slices = (double)slice_count(K, p.split_k);
+    double best = -1.0;
+    maxmulsk_plan out = p;
+    for (const Tile& t : tiles) {
+        maxmulsk_plan c = p;
+        c.tile_m = t.m;
+        c.tile_n = t.n;
+        if (classify_plan(M, K, N, &c) != MAXMULSK_OK) continue;
+        const double units = (double)((M + t.m - 1) / t.m) * (double)((N + t.n - 1) / t.n) * slices;
+        const double q = std::ceil(units / sms), rounds = std::floor(q / t.ctas), rest = q - rounds * t.ctas;
+        const double mac = len * t.m * t.n * us_per_mac;
+        double us = rounds * (t.ctas * mac / t.full + t.per_round_us);
+        if (rest > 0) us += rest * mac / t.part + t.per_round_us;
+        if (best < 0 || us < best) { best = us; out = c; }
+    }
+    return out;
+}
+
 // Tuning database entry for this exact shape, else the learned cost model,
 // else the rule. BF16X9 has no candidates or model class of its own: it
 // takes the model's BF16X6 plan for the shape (the same tiles, K splits and
@@ -155,6 +191,7 @@ maxmulsk_plan choose_tuned(size_t M, size_t K, size_t N, int precision, int sms)
     const int model_precision = precision == MAXMULSK_PREC_BF16X9 ? MAXMULSK_PREC_BF16X6 : precision;
     if (tuning_predict(M, K, N, model_precision, &p)) {
         if (precision == MAXMULSK_PREC_BF16X9) p.precision = MAXMULSK_PREC_BF16X9;
+        if (precision == MAXMULSK_PREC_FP32) p = with_best_fp32_tile(M, K, N, p, sms);
         return p;
     }
     return choose_rule(M, K, N, precision, sms);

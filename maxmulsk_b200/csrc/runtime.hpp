@@ -21,6 +21,8 @@ const char* last_error_message();
 maxmulsk_status classify_plan(size_t M, size_t K, size_t N, const maxmulsk_plan* plan);
 size_t workspace_bytes(size_t M, size_t K, size_t N, const maxmulsk_plan& plan);
 maxmulsk_plan choose_rule(size_t M, size_t K, size_t N, int precision, int sms);
+// `p` with the tile that its K split runs fastest on (FP32 plans).
+maxmulsk_plan with_best_fp32_tile(size_t M, size_t K, size_t N, maxmulsk_plan p, int sms);
 maxmulsk_plan choose_tuned(size_t M, size_t K, size_t N, int precision, int sms);
 bool parse_config_env(maxmulsk_plan& out);
 // Exhaustive search as the picker's fallback. picker_doubt says why the

@@ -205,3 +205,26 @@ def test_close_calls_on_held_out_shapes(built_lib, monkeypatch):
             close += 1
     print("close calls in 200 held-out FP32 shapes:", close)
     assert 0 <= close <= 200
+
+
+def test_fp32_tile_follows_the_k_split(built_lib, monkeypatch):
+    # The learned model's K split is kept; the tile is the kernels' rule and
+    # always one the library accepts, over tiny, skinny, large and odd shapes.
+    monkeypatch.delenv("MAXMULSK_CONFIG", raising=False)
+    _load_shipped_model()
+    mm.lib().maxmulsk_tuning_clear()
+    cands = (mm.Plan * 48)()
+    n = mm.lib().maxmulsk_candidates(0, cands, 48)
+    out = (ctypes.c_float * 48)()
+    rng = np.random.default_rng(3)
+    shapes = [(1, 1, 1), (1, 16384, 1), (16384, 1, 16384), (5000000, 64, 1), (1, 64, 5000000), (4096, 4096, 4096)]
+    shapes += [tuple(int(x) for x in np.exp(rng.uniform(0, np.log(16385), 3))) for _ in range(200)]
+    for M, K, N in shapes:
+        p = mm.choose(M, K, N)
+        assert mm.classify(M, K, N, p) == 0 and p.precision == 0 and p.variant == 0
+        assert (p.tile_m, p.tile_n) in ((128, 128), (128, 64), (64, 64))
+        assert mm.lib().maxmulsk_mlp_predict_host(M, K, N, 0, out) == 0
+        cap = (64 << 20) + 16 * (M * K + K * N + M * N)
+        ok = [i for i in range(n) if mm.classify(M, K, N, cands[i]) == 0
+              and mm.workspace_bytes(M, K, N, cands[i]) <= cap]
+        assert p.split_k == cands[min(ok, key=lambda i: out[i])].split_k, (M, K, N)
