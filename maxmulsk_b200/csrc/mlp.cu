@@ -15,7 +15,9 @@
 // Every kernel is deterministic: reductions run in a fixed order, no atomics.
 #include <dlfcn.h>
 
+#include <atomic>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -138,24 +140,38 @@ struct Model {
 std::mutex g_model_mu;
 Model g_model;
 bool g_env_tried = false;
+std::atomic<uint64_t> g_model_gen{1};         // counts the models there have been
+
+// z[o] = bias[o] + sum_i x[i] W[i][o], i upward, one fused multiply-add a step
+// (the order and rounding of linear_fwd): a row of W at a time, so that the
+// outputs' chains fill vector registers instead of a library call per term.
+#define MMSK_ROWS_FMA(NAME, ATTR)                                                                 \
+    ATTR void NAME(const float* x, const float* w, const float* bias, int in, int out, float* z) { \
+        for (int o = 0; o < out; o++) z[o] = bias[o];                                             \
+        for (int i = 0; i < in; i++)                                                              \
+            for (int o = 0; o < out; o++) z[o] = __builtin_fmaf(x[i], w[i * out + o], z[o]);      \
+    }
+MMSK_ROWS_FMA(rows_fma_plain, )
+#if defined(__x86_64__)
+MMSK_ROWS_FMA(rows_fma_avx2, __attribute__((target("avx2,fma"))))
+#endif
+#undef MMSK_ROWS_FMA
+
+void host_linear(const float* x, const float* w, const float* bias, int in, int out, float* z) {
+#if defined(__x86_64__)
+    static const bool wide = __builtin_cpu_supports("avx2") && __builtin_cpu_supports("fma");
+    if (wide) return rows_fma_avx2(x, w, bias, in, out, z);
+#endif
+    rows_fma_plain(x, w, bias, in, out, z);
+}
 
 void host_forward(const float* w, const float* x, float* y) {
     float h1[H], h2[H];
-    for (int o = 0; o < H; o++) {
-        float z = w[OFF_B1 + o];
-        for (int i = 0; i < F; i++) z = fmaf(x[i], w[OFF_W1 + i * H + o], z);
-        h1[o] = gelu(z);
-    }
-    for (int o = 0; o < H; o++) {
-        float z = w[OFF_B2 + o];
-        for (int i = 0; i < H; i++) z = fmaf(h1[i], w[OFF_W2 + i * H + o], z);
-        h2[o] = gelu(z);
-    }
-    for (int o = 0; o < O; o++) {
-        float z = w[OFF_B3 + o];
-        for (int i = 0; i < H; i++) z = fmaf(h2[i], w[OFF_W3 + i * O + o], z);
-        y[o] = z;
-    }
+    host_linear(x, w + OFF_W1, w + OFF_B1, F, H, h1);
+    for (float& v : h1) v = gelu(v);
+    host_linear(h1, w + OFF_W2, w + OFF_B2, H, H, h2);
+    for (float& v : h2) v = gelu(v);
+    host_linear(h2, w + OFF_W3, w + OFF_B3, H, O, y);
 }
 
 // <directory of this library>/../data/picker_model.bin
@@ -204,6 +220,7 @@ int mlp_load(const char* path) {
     g_env_tried = true;
     g_model.w = std::move(w);
     g_model.loaded = true;
+    g_model_gen++;
     return 0;
 }
 
@@ -212,6 +229,7 @@ void mlp_unload() {
     g_env_tried = true;
     g_model.loaded = false;
     g_model.w.clear();
+    g_model_gen++;
 }
 
 bool mlp_predict_host(size_t M, size_t K, size_t N, int cls, float* y) {
@@ -236,9 +254,11 @@ bool mlp_predict_host(size_t M, size_t K, size_t N, int cls, float* y) {
     return true;
 }
 
-bool mlp_predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan* out, float* margin) {
+namespace {
+
+// The model's pick for a shape (mlp_predict_plan without its memory).
+bool predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan* out, float* margin) {
     const int cls = (precision == MAXMULSK_PREC_FP32) ? 0 : 1;
-    if (precision == MAXMULSK_PREC_BF16X9) return false;          // not among the candidates
     float y[O];
     if (!mlp_predict_host(M, K, N, cls, y)) return false;
     maxmulsk_plan cands[O];
@@ -259,7 +279,46 @@ bool mlp_predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan
     if (best < 0) return false;
     *out = cands[best];
     // Predicted log-time gap to the runner-up (infinite with one candidate).
-    if (margin) *margin = second < 0 ? INFINITY : y[second] - y[best];
+    *margin = second < 0 ? INFINITY : y[second] - y[best];
+    return true;
+}
+
+// The last picks of this thread, by shape: a program calls few shapes many
+// times, and a pick (forward pass, 24 or 48 candidates checked and sized) costs
+// 29-34 us on the host with scalar multiply-adds, several times a small
+// product on the GPU; 4.3-5.7 us with host_linear, 1 us or less found here. A
+// 256^3 matmul from Python 34 -> 16 us a call. Per thread, so no
+// lock; a direct-mapped table of fixed size; an entry holds for one model and
+// one device, whose work slots decide the workspaces.
+struct PickEntry {
+    uint64_t gen = 0;
+    size_t M = 0, K = 0, N = 0;
+    int precision = 0, device = 0;
+    bool ok = false;
+    float margin = 0.f;
+    maxmulsk_plan plan{};
+};
+constexpr size_t kPickEntries = 128;
+thread_local PickEntry t_picks[kPickEntries];
+
+}  // namespace
+
+bool mlp_predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan* out, float* margin) {
+    if (precision == MAXMULSK_PREC_BF16X9) return false;          // not among the candidates
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t h = (M * 0x9E3779B97F4A7C15ull) ^ (K * 0xC2B2AE3D27D4EB4Full) ^ (N * 0x165667B19E3779F9ull) ^ (uint64_t)precision;
+    PickEntry& e = t_picks[(h >> 32) % kPickEntries];
+    const uint64_t gen = g_model_gen.load(std::memory_order_acquire);
+    if (!(e.gen == gen && e.M == M && e.K == K && e.N == N && e.precision == precision && e.device == dev)) {
+        PickEntry f;
+        f.gen = gen; f.M = M; f.K = K; f.N = N; f.precision = precision; f.device = dev;
+        f.ok = predict_plan(M, K, N, precision, &f.plan, &f.margin);
+        e = f;
+    }
+    if (!e.ok) return false;
+    *out = e.plan;
+    if (margin) *margin = e.margin;
     return true;
 }
 

@@ -228,3 +228,41 @@ def test_fp32_tile_follows_the_k_split(built_lib, monkeypatch):
         ok = [i for i in range(n) if mm.classify(M, K, N, cands[i]) == 0
               and mm.workspace_bytes(M, K, N, cands[i]) <= cap]
         assert p.split_k == cands[min(ok, key=lambda i: out[i])].split_k, (M, K, N)
+
+
+def test_picks_follow_the_loaded_model(built_lib, tmp_path, monkeypatch):
+    # Picks are remembered per thread and shape: more shapes than are kept, in
+    # two orders and in another thread, give the picks of a first pass; another
+    # model, or none, shows at once.
+    import threading
+    monkeypatch.delenv("MAXMULSK_CONFIG", raising=False)
+    mm.lib().maxmulsk_tuning_clear()
+    _load_shipped_model()
+    rng = np.random.default_rng(8)
+    shapes = [tuple(int(x) for x in np.exp(rng.uniform(0, np.log(16385), 3))) for _ in range(300)]
+    precs = (mm.Precision.FP32, mm.Precision.BF16X6, mm.Precision.TF32X3, mm.Precision.SPLIT_AUTO)
+
+    def picks(order):
+        got = {(s, p): mm.choose(*s, p).as_tuple() for s in order for p in precs}
+        return [got[s, p] for s in shapes for p in precs]
+
+    first = picks(shapes)
+    assert picks(shapes[::-1]) == first and picks(shapes) == first
+    other = []
+    t = threading.Thread(target=lambda: other.append(picks(shapes)))
+    t.start()
+    t.join()
+    assert other[0] == first
+    # A model whose last candidate of each class wins everywhere it may.
+    p = np.zeros(picker.NPARAM, np.float32)
+    p[-48:] = np.arange(48, 0, -1)
+    path = str(tmp_path / "last.bin")
+    picker.save_params(path, p)
+    try:
+        assert mm.lib().maxmulsk_model_load(path.encode()) == 0
+        assert mm.choose(512, 512, 512, mm.Precision.BF16X6).as_tuple() == (2, 128, 64, 16, 0)
+        mm.lib().maxmulsk_model_load(None)
+        assert mm.choose(*shapes[0]).as_tuple() == mm.choose_rule(*shapes[0]).as_tuple()
+    finally:
+        _load_shipped_model()
+    assert picks(shapes) == first
