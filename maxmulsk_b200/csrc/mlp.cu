@@ -28,6 +28,7 @@
 #include "internal.hpp"
 #include "mlp.hpp"
 #include "runtime.hpp"
+#include "split_math.cuh"
 
 namespace mmsk {
 
@@ -46,61 +47,213 @@ __host__ __device__ inline float gelu_grad(float x) {
     return cdf + x * pdf;
 }
 
-// Z[b][o] = b[o] + sum_i X[b][i] W[i][o]; A = act(Z) (GELU when act != 0).
-__global__ void linear_fwd(const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ bias,
-                           int B, int in, int out, float* __restrict__ Z, float* __restrict__ A, int act) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= B * out) return;
-    const int b = idx / out, o = idx % out;
-    float z = bias[o];
-    for (int i = 0; i < in; i++) z = fmaf(X[b * in + i], W[i * out + o], z);
-    if (Z) Z[idx] = z;
-    if (A) A[idx] = act ? gelu(z) : z;
-}
-
-// dY = 2 (Y - T) / count over the entries with mask != 0 (else 0); the
-// per-row squared errors go to rowloss[b] (summed on the host).
-__global__ void mse_grad(const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ mask,
-                         int B, float inv_count, float* __restrict__ dY, float* __restrict__ rowloss) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    float l = 0.f;
-    for (int o = 0; o < O; o++) {
-        const int k = b * O + o;
-        const float m = mask[k];
-        const float d = (m != 0.f) ? (Y[k] - T[k]) : 0.f;
-        dY[k] = 2.f * d * inv_count;
-        l = fmaf(d, d, l);
+// Forward pass, all three layers: Z[b][o] = bias[o] + sum_i X[b][i] W[i][o], i
+// upward, and H = gelu(Z) after the first two. A block takes kFwdRows rows; the
+// weights (30 KB) and the rows' activations stay in shared memory between the
+// layers. Thread t computes output o = t % 64 of rows t / 64 + 4 j: a row of W
+// is read by consecutive lanes, four inputs of a row by broadcast. Bound by
+// latency (61 MFLOP at 4000 rows): one launch instead of three.
+constexpr int kFwdRows = 16;
+__global__ void __launch_bounds__(256)
+mlp_forward_kernel(const float* __restrict__ params, const float* __restrict__ X, int B, float* __restrict__ Z1,
+                   float* __restrict__ H1, float* __restrict__ Z2, float* __restrict__ H2, float* __restrict__ Y) {
+    __shared__ float w[NPARAM];
+    __shared__ __align__(16) float in[2][kFwdRows][H];           // X or H2, and H1
+    const int tid = threadIdx.x, o = tid & 63, rq = tid >> 6;
+    const int b0 = blockIdx.x * kFwdRows;
+    for (int i = tid; i < NPARAM; i += 256) w[i] = params[i];
+    for (int i = tid; i < kFwdRows * 8; i += 256) {
+        const int r = i >> 3, c = i & 7;
+        in[0][r][c] = (c < F && b0 + r < B) ? X[(size_t)(b0 + r) * F + c] : 0.f;   // an eighth, zero input
     }
-    rowloss[b] = l;
+    __syncthreads();
+    auto layer = [&](const float (*x)[H], int n, const float* W, const float* bias, int out, float (&z)[4]) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) z[j] = bias[o];
+        for (int i = 0; i < n; i += 4) {
+            float4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = *reinterpret_cast<const float4*>(&x[rq + 4 * j][i]);
+            const float w0 = W[i * out + o], w1 = W[(i + 1) * out + o], w2 = W[(i + 2) * out + o];
+#pragma unroll
+            for (int j = 0; j < 4; j++) z[j] = fmaf(v[j].z, w2, fmaf(v[j].y, w1, fmaf(v[j].x, w0, z[j])));
+            if (i + 3 < n) {
+                const float w3 = W[(i + 3) * out + o];
+#pragma unroll
+                for (int j = 0; j < 4; j++) z[j] = fmaf(v[j].w, w3, z[j]);
+            }
+        }
+    };
+    auto hidden = [&](const float (&z)[4], float (*dst)[H], float* Z, float* A) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int r = rq + 4 * j;
+            const float h = gelu(z[j]);
+            dst[r][o] = h;
+            if (b0 + r < B) {
+                const size_t k = (size_t)(b0 + r) * H + o;
+                if (Z) Z[k] = z[j];
+                A[k] = h;
+            }
+        }
+        __syncthreads();
+    };
+    float z[4];
+    layer(in[0], F, w + OFF_W1, w + OFF_B1, H, z);
+    hidden(z, in[1], Z1, H1);
+    layer(in[1], H, w + OFF_W2, w + OFF_B2, H, z);
+    hidden(z, in[0], Z2, H2);
+    if (o >= O) return;
+    layer(in[0], H, w + OFF_W3, w + OFF_B3, O, z);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (b0 + rq + 4 * j < B) Y[(size_t)(b0 + rq + 4 * j) * O + o] = z[j];
 }
 
-// dX[b][i] = sum_o dZ[b][o] W[i][o]; optionally times gelu'(Zprev[b][i]).
-__global__ void linear_bwd_x(const float* __restrict__ dZ, const float* __restrict__ W, const float* __restrict__ Zprev,
-                             int B, int in, int out, float* __restrict__ dX) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= B * in) return;
-    const int b = idx / in, i = idx % in;
-    float s = 0.f;
-    for (int o = 0; o < out; o++) s = fmaf(dZ[b * out + o], W[i * out + o], s);
-    dX[idx] = Zprev ? s * gelu_grad(Zprev[idx]) : s;
-}
+// Backward pass. dY = 2 (Y - T) / count over the entries with mask != 0 (else
+// 0), rowloss[b] the row's squared errors; through each layer
+//   dX[b][i] = sum_o dZ[b][o] W[i][o], times gelu'(Zprev[b][i]);
+//   dW[i][o] = sum_b X[b][i] dZ[b][o],  db[o] = sum_b dZ[b][o].
+// A block takes a contiguous range of rows, 8 at a time through shared memory
+// (W2 and W3 padded so that lanes walking i hit distinct banks), and keeps its
+// sums of all weight gradients in registers: thread t owns 12 of dW3, 16 of dW2,
+// 2 of dW1. They go to parts[block][NPARAM] and mlp_grad_sum adds the blocks in
+// block order (with one block, parts is grads). Two launches and chains of rows
+// / blocks terms; one thread per weight walking all rows, layer by layer in six
+// launches, took 840 us at 4000 rows.
+constexpr int kBwdRows = 8;
+__global__ void __launch_bounds__(256)
+mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ X, const float* __restrict__ Z1,
+                    const float* __restrict__ H1, const float* __restrict__ Z2, const float* __restrict__ H2,
+                    const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ mask, int B,
+                    int rows, float inv_count, float* __restrict__ parts, float* __restrict__ rowloss) {
+    constexpr int R = kBwdRows;
+    __shared__ float w3[H][O + 1], w2[H][H + 1];
+    __shared__ __align__(16) float dy[R][O], h2[R][H], dz2[R][H], h1[R][H], dz1[R][H];
+    __shared__ float xs[R][F];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < H * O; i += 256) w3[i / O][i % O] = params[OFF_W3 + i];
+    for (int i = tid; i < H * H; i += 256) w2[i / H][i % H] = params[OFF_W2 + i];
+    const int wi = tid >> 2, o3 = (tid & 3) * 12, o2 = (tid & 3) * 16;   // dW3[wi][o3 ..], dW2[wi][o2 ..]
+    const int hi = tid & 63, hr = tid >> 6;                              // dZ[hr + 4 j][hi]
+    const int i1 = tid / 32, o1 = (tid & 31) * 2;                        // dW1[i1][o1 ..], i1 < F
+    float g3[12], g2[16], g1[2], gb = 0.f;                               // gb: db3, db2 or db1 by thread range
+#pragma unroll
+    for (int j = 0; j < 12; j++) g3[j] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16; j++) g2[j] = 0.f;
+    g1[0] = g1[1] = 0.f;
 
-// dW[i][o] = sum_b X[b][i] dZ[b][o] (b upward), db[o] = sum_b dZ[b][o].
-__global__ void linear_bwd_w(const float* __restrict__ X, const float* __restrict__ dZ, int B, int in, int out,
-                             float* __restrict__ dW, float* __restrict__ db) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < in * out) {
-        const int i = idx / out, o = idx % out;
-        float s = 0.f;
-        for (int b = 0; b < B; b++) s = fmaf(X[b * in + i], dZ[b * out + o], s);
-        dW[idx] = s;
-    } else if (idx < in * out + out) {
-        const int o = idx - in * out;
-        float s = 0.f;
-        for (int b = 0; b < B; b++) s += dZ[b * out + o];
-        db[o] = s;
+    const int row_end = min(B, (int)(blockIdx.x + 1) * rows);
+    for (int r0 = blockIdx.x * rows; r0 < row_end; r0 += R) {
+        // Rows past the range count as zeros.
+        {
+            const int b = r0 + warp;
+            float l = 0.f;
+            for (int o = lane; o < O; o += 32) {
+                float d = 0.f;
+                if (b < row_end) {
+                    const size_t k = (size_t)b * O + o;
+                    d = mask[k] != 0.f ? Y[k] - T[k] : 0.f;
+                }
+                dy[warp][o] = 2.f * d * inv_count;
+                l = fmaf(d, d, l);
+            }
+#pragma unroll
+            for (int m = 16; m; m >>= 1) l += __shfl_xor_sync(0xffffffffu, l, m);
+            if (lane == 0 && b < row_end) rowloss[b] = l;
+        }
+        float z2[2], z1[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int b = r0 + hr + 4 * j;
+            const size_t k = (size_t)b * H + hi;
+            const bool ok = b < row_end;
+            h2[hr + 4 * j][hi] = ok ? H2[k] : 0.f;
+            h1[hr + 4 * j][hi] = ok ? H1[k] : 0.f;
+            z2[j] = ok ? Z2[k] : 0.f;
+            z1[j] = ok ? Z1[k] : 0.f;
+        }
+        if (tid < R * F) xs[tid / F][tid % F] = r0 + tid / F < row_end ? X[(size_t)r0 * F + tid] : 0.f;
+        __syncthreads();
+        {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll 8
+            for (int o = 0; o < O; o++) {
+                s0 = fmaf(dy[hr][o], w3[hi][o], s0);
+                s1 = fmaf(dy[hr + 4][o], w3[hi][o], s1);
+            }
+            dz2[hr][hi] = s0 * gelu_grad(z2[0]);
+            dz2[hr + 4][hi] = s1 * gelu_grad(z2[1]);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const float x = h2[r][wi];
+#pragma unroll
+                for (int j = 0; j < 12; j += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(&dy[r][o3 + j]);
+                    g3[j] = fmaf(x, v.x, g3[j]);
+                    g3[j + 1] = fmaf(x, v.y, g3[j + 1]);
+                    g3[j + 2] = fmaf(x, v.z, g3[j + 2]);
+                    g3[j + 3] = fmaf(x, v.w, g3[j + 3]);
+                }
+            }
+        }
+        __syncthreads();
+        {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll 8
+            for (int o = 0; o < H; o++) {
+                s0 = fmaf(dz2[hr][o], w2[hi][o], s0);
+                s1 = fmaf(dz2[hr + 4][o], w2[hi][o], s1);
+            }
+            dz1[hr][hi] = s0 * gelu_grad(z1[0]);
+            dz1[hr + 4][hi] = s1 * gelu_grad(z1[1]);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const float x = h1[r][wi];
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(&dz2[r][o2 + j]);
+                    g2[j] = fmaf(x, v.x, g2[j]);
+                    g2[j + 1] = fmaf(x, v.y, g2[j + 1]);
+                    g2[j + 2] = fmaf(x, v.z, g2[j + 2]);
+                    g2[j + 3] = fmaf(x, v.w, g2[j + 3]);
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            if (i1 < F) {
+                const float x = xs[r][i1];
+                g1[0] = fmaf(x, dz1[r][o1], g1[0]);
+                g1[1] = fmaf(x, dz1[r][o1 + 1], g1[1]);
+            }
+            if (tid < O) gb += dy[r][tid];
+            else if (tid >= 64 && tid < 64 + H) gb += dz2[r][tid - 64];
+            else if (tid >= 128 && tid < 128 + H) gb += dz1[r][tid - 128];
+        }
+        __syncthreads();                     // the next rows overwrite these
     }
+    float* out = parts + (size_t)blockIdx.x * NPARAM;
+#pragma unroll
+    for (int j = 0; j < 12; j++) out[OFF_W3 + wi * O + o3 + j] = g3[j];
+#pragma unroll
+    for (int j = 0; j < 16; j++) out[OFF_W2 + wi * H + o2 + j] = g2[j];
+    if (i1 < F) {
+        out[OFF_W1 + i1 * H + o1] = g1[0];
+        out[OFF_W1 + i1 * H + o1 + 1] = g1[1];
+    }
+    if (tid < O) out[OFF_B3 + tid] = gb;
+    else if (tid >= 64 && tid < 64 + H) out[OFF_B2 + tid - 64] = gb;
+    else if (tid >= 128 && tid < 128 + H) out[OFF_B1 + tid - 128] = gb;
+}
+
+// grads[i] = parts[0][i] + parts[1][i] + ..., in block order.
+__global__ void __launch_bounds__(128)
+mlp_grad_sum(const float* __restrict__ parts, int n, float* __restrict__ grads) {
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i < NPARAM) grads[i] = ordered_sum<31>(parts + i, (size_t)NPARAM, n);
 }
 
 // Adam (bias-corrected), elementwise.
@@ -333,9 +486,8 @@ maxmulsk_status maxmulsk_mlp_forward_dev(const float* params, const float* X, in
     if (!params || !X || !H1 || !H2 || !Y || B < 0) return MAXMULSK_ERR_INVALID;
     if (B == 0) return MAXMULSK_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    linear_fwd<<<blocks(B * H), 256, 0, s>>>(X, params + OFF_W1, params + OFF_B1, B, F, H, Z1, H1, 1);
-    linear_fwd<<<blocks(B * H), 256, 0, s>>>(H1, params + OFF_W2, params + OFF_B2, B, H, H, Z2, H2, 1);
-    linear_fwd<<<blocks(B * O), 256, 0, s>>>(H2, params + OFF_W3, params + OFF_B3, B, H, O, nullptr, Y, 0);
+    const unsigned grid = (unsigned)(((int64_t)B + kFwdRows - 1) / kFwdRows);
+    mlp_forward_kernel<<<grid, 256, 0, s>>>(params, X, B, Z1, H1, Z2, H2, Y);
     return cuda_status(cudaGetLastError(), "mlp forward");
 }
 
@@ -347,15 +499,15 @@ maxmulsk_status maxmulsk_mlp_backward_dev(const float* params, const float* X, c
         !(count > 0))
         return MAXMULSK_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    float* dY = work;                    // B x O
-    float* dZ2 = dY + (size_t)B * O;     // B x H
-    float* dZ1 = dZ2 + (size_t)B * H;    // B x H
-    mse_grad<<<blocks(B), 256, 0, s>>>(Y, T, mask, B, 1.0f / count, dY, rowloss);
-    linear_bwd_w<<<blocks(H * O + O), 256, 0, s>>>(H2, dY, B, H, O, grads + OFF_W3, grads + OFF_B3);
-    linear_bwd_x<<<blocks(B * H), 256, 0, s>>>(dY, params + OFF_W3, Z2, B, H, O, dZ2);
-    linear_bwd_w<<<blocks(H * H + H), 256, 0, s>>>(H1, dZ2, B, H, H, grads + OFF_W2, grads + OFF_B2);
-    linear_bwd_x<<<blocks(B * H), 256, 0, s>>>(dZ2, params + OFF_W2, Z1, B, H, H, dZ1);
-    linear_bwd_w<<<blocks(F * H + H), 256, 0, s>>>(X, dZ1, B, F, H, grads + OFF_W1, grads + OFF_B1);
+    // As many row blocks as their gradient sums fit in `work` (B (O + 2 H)
+    // floats), of 45 rows or more: 90 at 4000 rows. One writes grads itself.
+    const int64_t fit = (int64_t)B * (O + 2 * H) / NPARAM;
+    const int64_t want = fit < 1 ? 1 : fit < 4 * (int64_t)device_sm_count() ? fit : 4 * (int64_t)device_sm_count();
+    const int rows = (int)(((B + want - 1) / want));
+    const int nb = (B + rows - 1) / rows;
+    mlp_backward_kernel<<<nb, 256, 0, s>>>(params, X, Z1, H1, Z2, H2, Y, T, mask, B, rows, 1.0f / count,
+                                           nb > 1 ? work : grads, rowloss);
+    if (nb > 1) mlp_grad_sum<<<(NPARAM + 127) / 128, 128, 0, s>>>(work, nb, grads);
     return cuda_status(cudaGetLastError(), "mlp backward");
 }
 
