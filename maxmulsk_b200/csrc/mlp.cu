@@ -13,8 +13,10 @@
 // Features of a shape (M, K, N, class):
 //   ln(M), ln(N), ln(K) / ln(16384); (M, N, K mod 16) / 16; class (0 FP32, 1 split)
 // Every kernel is deterministic: reductions run in a fixed order, no atomics.
+#include <cooperative_groups.h>
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdint>
@@ -29,6 +31,8 @@
 #include "mlp.hpp"
 #include "runtime.hpp"
 #include "split_math.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace mmsk {
 
@@ -61,7 +65,9 @@ mlp_forward_kernel(const float* __restrict__ params, const float* __restrict__ X
     __shared__ __align__(16) float in[2][kFwdRows][H];           // X or H2, and H1
     const int tid = threadIdx.x, o = tid & 63, rq = tid >> 6;
     const int b0 = blockIdx.x * kFwdRows;
-    for (int i = tid; i < NPARAM; i += 256) w[i] = params[i];
+#pragma unroll
+    for (int j = 0; j < (NPARAM + 255) / 256; j++)
+        if (tid + j * 256 < NPARAM) w[tid + j * 256] = params[tid + j * 256];
     for (int i = tid; i < kFwdRows * 8; i += 256) {
         const int r = i >> 3, c = i & 7;
         in[0][r][c] = (c < F && b0 + r < B) ? X[(size_t)(b0 + r) * F + c] : 0.f;   // an eighth, zero input
@@ -114,25 +120,35 @@ mlp_forward_kernel(const float* __restrict__ params, const float* __restrict__ X
 // 0), rowloss[b] the row's squared errors; through each layer
 //   dX[b][i] = sum_o dZ[b][o] W[i][o], times gelu'(Zprev[b][i]);
 //   dW[i][o] = sum_b X[b][i] dZ[b][o],  db[o] = sum_b dZ[b][o].
-// A block takes a contiguous range of rows, 8 at a time through shared memory
-// (W2 and W3 padded so that lanes walking i hit distinct banks), and keeps its
-// sums of all weight gradients in registers: thread t owns 12 of dW3, 16 of dW2,
-// 2 of dW1. They go to parts[block][NPARAM] and mlp_grad_sum adds the blocks in
-// block order (with one block, parts is grads). Two launches and chains of rows
-// / blocks terms; one thread per weight walking all rows, layer by layer in six
-// launches, took 840 us at 4000 rows.
-constexpr int kBwdRows = 8;
+// A block takes eight rows at a time through shared memory (W2 and W3 padded so
+// that lanes walking i hit distinct banks) and keeps its sums of all weight
+// gradients in registers: thread t owns 12 of dW3, 16 of dW2, 2 of dW1. Eight
+// blocks form a cluster; at the end each adds an eighth of the weights over the
+// cluster's shared memories, in block order, into parts[cluster][NPARAM], and
+// mlp_grad_sum adds the clusters in order (with one cluster, parts is grads).
+// Bound by latency, so the rows are spread thin. At 4000 rows 22.8 us (ncu, cold
+// caches) on 256 blocks; 89 blocks of 45 rows without clusters 44 us, one thread
+// per weight walking all rows, in six launches, 840 us. A whole training step
+// 893 -> 39 us.
+constexpr int kBwdRows = 8, kBwdCluster = 8;
 __global__ void __launch_bounds__(256)
 mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ X, const float* __restrict__ Z1,
                     const float* __restrict__ H1, const float* __restrict__ Z2, const float* __restrict__ H2,
                     const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ mask, int B,
-                    int rows, float inv_count, float* __restrict__ parts, float* __restrict__ rowloss) {
+                    float inv_count, float* __restrict__ parts, float* __restrict__ rowloss) {
     constexpr int R = kBwdRows;
-    __shared__ float w3[H][O + 1], w2[H][H + 1];
+    static_assert(R == 8, "one row a warp, two rows a thread");
+    constexpr int P3 = O + 4, P2 = H + 4;                  // row strides: quads of eight rows on distinct banks
+    __shared__ __align__(16) float buf[NPARAM];            // W3 and W2, then this block's gradient sums
+    static_assert(H * P3 + H * P2 <= NPARAM, "padded weights fit the gradients' buffer");
+    float (*w3)[P3] = reinterpret_cast<float (*)[P3]>(buf);
+    float (*w2)[P2] = reinterpret_cast<float (*)[P2]>(buf + H * P3);
     __shared__ __align__(16) float dy[R][O], h2[R][H], dz2[R][H], h1[R][H], dz1[R][H];
     __shared__ float xs[R][F];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
     for (int i = tid; i < H * O; i += 256) w3[i / O][i % O] = params[OFF_W3 + i];
+#pragma unroll
     for (int i = tid; i < H * H; i += 256) w2[i / H][i % H] = params[OFF_W2 + i];
     const int wi = tid >> 2, o3 = (tid & 3) * 12, o2 = (tid & 3) * 16;   // dW3[wi][o3 ..], dW2[wi][o2 ..]
     const int hi = tid & 63, hr = tid >> 6;                              // dZ[hr + 4 j][hi]
@@ -144,44 +160,58 @@ mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ 
     for (int j = 0; j < 16; j++) g2[j] = 0.f;
     g1[0] = g1[1] = 0.f;
 
-    const int row_end = min(B, (int)(blockIdx.x + 1) * rows);
-    for (int r0 = blockIdx.x * rows; r0 < row_end; r0 += R) {
-        // Rows past the range count as zeros.
-        {
-            const int b = r0 + warp;
-            float l = 0.f;
-            for (int o = lane; o < O; o += 32) {
-                float d = 0.f;
-                if (b < row_end) {
-                    const size_t k = (size_t)b * O + o;
-                    d = mask[k] != 0.f ? Y[k] - T[k] : 0.f;
-                }
-                dy[warp][o] = 2.f * d * inv_count;
-                l = fmaf(d, d, l);
-            }
-#pragma unroll
-            for (int m = 16; m; m >>= 1) l += __shfl_xor_sync(0xffffffffu, l, m);
-            if (lane == 0 && b < row_end) rowloss[b] = l;
-        }
-        float z2[2], z1[2];
+    // The next eight rows are read while the current ones are worked on; rows
+    // past B count as zeros.
+    float ny[2], nt[2], nm[2], nh2[2], nh1[2], nz2[2], nz1[2], nx;
+    auto fetch = [&](int r0) {
+        const int b = r0 + warp;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const int b = r0 + hr + 4 * j;
-            const size_t k = (size_t)b * H + hi;
-            const bool ok = b < row_end;
-            h2[hr + 4 * j][hi] = ok ? H2[k] : 0.f;
-            h1[hr + 4 * j][hi] = ok ? H1[k] : 0.f;
-            z2[j] = ok ? Z2[k] : 0.f;
-            z1[j] = ok ? Z1[k] : 0.f;
+            const int o = lane + 32 * j;
+            const bool ok = b < B && o < O;
+            const size_t k = (size_t)b * O + o;
+            ny[j] = ok ? Y[k] : 0.f;
+            nt[j] = ok ? T[k] : 0.f;
+            nm[j] = ok ? mask[k] : 0.f;
+            const int bh = r0 + hr + 4 * j;
+            const size_t kh = (size_t)bh * H + hi;
+            const bool okh = bh < B;
+            nh2[j] = okh ? H2[kh] : 0.f;
+            nh1[j] = okh ? H1[kh] : 0.f;
+            nz2[j] = okh ? Z2[kh] : 0.f;
+            nz1[j] = okh ? Z1[kh] : 0.f;
         }
-        if (tid < R * F) xs[tid / F][tid % F] = r0 + tid / F < row_end ? X[(size_t)r0 * F + tid] : 0.f;
+        nx = (tid < R * F && r0 + tid / F < B) ? X[(size_t)r0 * F + tid] : 0.f;
+    };
+    const int stride = (int)gridDim.x * R;
+    fetch((int)blockIdx.x * R);
+    for (int r0 = (int)blockIdx.x * R; r0 < B; r0 += stride) {
+        float l = 0.f, z2[2], z1[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float d = nm[j] != 0.f ? ny[j] - nt[j] : 0.f;
+            if (lane + 32 * j < O) dy[warp][lane + 32 * j] = 2.f * d * inv_count;
+            l = fmaf(d, d, l);
+            h2[hr + 4 * j][hi] = nh2[j];
+            h1[hr + 4 * j][hi] = nh1[j];
+            z2[j] = nz2[j];
+            z1[j] = nz1[j];
+        }
+        if (tid < R * F) xs[tid / F][tid % F] = nx;
+        if (r0 < B - stride) fetch(r0 + stride);
+#pragma unroll
+        for (int m = 16; m; m >>= 1) l += __shfl_xor_sync(0xffffffffu, l, m);
+        if (lane == 0 && r0 + warp < B) rowloss[r0 + warp] = l;
         __syncthreads();
         {
             float s0 = 0.f, s1 = 0.f;
-#pragma unroll 8
-            for (int o = 0; o < O; o++) {
-                s0 = fmaf(dy[hr][o], w3[hi][o], s0);
-                s1 = fmaf(dy[hr + 4][o], w3[hi][o], s1);
+#pragma unroll 4
+            for (int o = 0; o < O; o += 4) {
+                const float4 wv = *reinterpret_cast<const float4*>(&w3[hi][o]);
+                const float4 a = *reinterpret_cast<const float4*>(&dy[hr][o]);
+                const float4 c = *reinterpret_cast<const float4*>(&dy[hr + 4][o]);
+                s0 = fmaf(a.w, wv.w, fmaf(a.z, wv.z, fmaf(a.y, wv.y, fmaf(a.x, wv.x, s0))));
+                s1 = fmaf(c.w, wv.w, fmaf(c.z, wv.z, fmaf(c.y, wv.y, fmaf(c.x, wv.x, s1))));
             }
             dz2[hr][hi] = s0 * gelu_grad(z2[0]);
             dz2[hr + 4][hi] = s1 * gelu_grad(z2[1]);
@@ -201,10 +231,13 @@ mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ 
         __syncthreads();
         {
             float s0 = 0.f, s1 = 0.f;
-#pragma unroll 8
-            for (int o = 0; o < H; o++) {
-                s0 = fmaf(dz2[hr][o], w2[hi][o], s0);
-                s1 = fmaf(dz2[hr + 4][o], w2[hi][o], s1);
+#pragma unroll 4
+            for (int o = 0; o < H; o += 4) {
+                const float4 wv = *reinterpret_cast<const float4*>(&w2[hi][o]);
+                const float4 a = *reinterpret_cast<const float4*>(&dz2[hr][o]);
+                const float4 c = *reinterpret_cast<const float4*>(&dz2[hr + 4][o]);
+                s0 = fmaf(a.w, wv.w, fmaf(a.z, wv.z, fmaf(a.y, wv.y, fmaf(a.x, wv.x, s0))));
+                s1 = fmaf(c.w, wv.w, fmaf(c.z, wv.z, fmaf(c.y, wv.y, fmaf(c.x, wv.x, s1))));
             }
             dz1[hr][hi] = s0 * gelu_grad(z1[0]);
             dz1[hr + 4][hi] = s1 * gelu_grad(z1[1]);
@@ -235,18 +268,32 @@ mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ 
         }
         __syncthreads();                     // the next rows overwrite these
     }
-    float* out = parts + (size_t)blockIdx.x * NPARAM;
+    __syncthreads();                         // W2 and W3 are done with (and, in a block without rows, stored)
 #pragma unroll
-    for (int j = 0; j < 12; j++) out[OFF_W3 + wi * O + o3 + j] = g3[j];
+    for (int j = 0; j < 12; j++) buf[OFF_W3 + wi * O + o3 + j] = g3[j];
 #pragma unroll
-    for (int j = 0; j < 16; j++) out[OFF_W2 + wi * H + o2 + j] = g2[j];
+    for (int j = 0; j < 16; j++) buf[OFF_W2 + wi * H + o2 + j] = g2[j];
     if (i1 < F) {
-        out[OFF_W1 + i1 * H + o1] = g1[0];
-        out[OFF_W1 + i1 * H + o1 + 1] = g1[1];
+        buf[OFF_W1 + i1 * H + o1] = g1[0];
+        buf[OFF_W1 + i1 * H + o1 + 1] = g1[1];
     }
-    if (tid < O) out[OFF_B3 + tid] = gb;
-    else if (tid >= 64 && tid < 64 + H) out[OFF_B2 + tid - 64] = gb;
-    else if (tid >= 128 && tid < 128 + H) out[OFF_B1 + tid - 128] = gb;
+    if (tid < O) buf[OFF_B3 + tid] = gb;
+    else if (tid >= 64 && tid < 64 + H) buf[OFF_B2 + tid - 64] = gb;
+    else if (tid >= 128 && tid < 128 + H) buf[OFF_B1 + tid - 128] = gb;
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    float* out = parts + (size_t)(blockIdx.x / kBwdCluster) * NPARAM;
+    const int share = (NPARAM + kBwdCluster - 1) / kBwdCluster, first = (int)cluster.block_rank() * share;
+    for (int i = first + tid; i < min(NPARAM, first + share); i += 256) {
+        float v[kBwdCluster];
+#pragma unroll
+        for (int c = 0; c < kBwdCluster; c++) v[c] = cluster.map_shared_rank(buf, c)[i];
+        float g = v[0];
+#pragma unroll
+        for (int c = 1; c < kBwdCluster; c++) g += v[c];
+        out[i] = g;
+    }
+    cluster.sync();                          // no block leaves while another reads its sums
 }
 
 // grads[i] = parts[0][i] + parts[1][i] + ..., in block order.
@@ -499,15 +546,30 @@ maxmulsk_status maxmulsk_mlp_backward_dev(const float* params, const float* X, c
         !(count > 0))
         return MAXMULSK_ERR_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // As many row blocks as their gradient sums fit in `work` (B (O + 2 H)
-    // floats), of 45 rows or more: 90 at 4000 rows. One writes grads itself.
+    // Clusters for one wave of two blocks an SM with equal turns of eight rows a
+    // block (32 clusters, two turns at 4000 rows: 22.8 us; 63 clusters in two waves
+    // 28.0), as far as their gradient sums fit in `work` (B (O + 2 H) floats, NPARAM
+    // each). One cluster writes grads itself.
     const int64_t fit = (int64_t)B * (O + 2 * H) / NPARAM;
-    const int64_t want = fit < 1 ? 1 : fit < 4 * (int64_t)device_sm_count() ? fit : 4 * (int64_t)device_sm_count();
-    const int rows = (int)(((B + want - 1) / want));
-    const int nb = (B + rows - 1) / rows;
-    mlp_backward_kernel<<<nb, 256, 0, s>>>(params, X, Z1, H1, Z2, H2, Y, T, mask, B, rows, 1.0f / count,
-                                           nb > 1 ? work : grads, rowloss);
-    if (nb > 1) mlp_grad_sum<<<(NPARAM + 127) / 128, 128, 0, s>>>(work, nb, grads);
+    const int64_t turns = ((int64_t)B + kBwdRows - 1) / kBwdRows, wave = std::max(1, 2 * device_sm_count());
+    const int64_t each = (turns + wave - 1) / wave;
+    const int64_t want = (turns + each * kBwdCluster - 1) / (each * kBwdCluster);
+    const int nc = (int)std::max<int64_t>(1, std::min(want, fit));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nc * kBwdCluster));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kBwdCluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, mlp_backward_kernel, params, X, Z1, H1, Z2, H2, Y, T, mask, (int)B,
+                                             1.0f / count, nc > 1 ? work : grads, rowloss);
+    if (e != cudaSuccess) return cuda_status(e, "mlp backward");
+    if (nc > 1) mlp_grad_sum<<<(NPARAM + 127) / 128, 128, 0, s>>>(work, nc, grads);
     return cuda_status(cudaGetLastError(), "mlp backward");
 }
 
