@@ -131,39 +131,52 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// Arrives on `bar` once every tcgen05.mma this thread issued so far is done.
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 :: "r"(smem_u32(bar)) : "memory");
+// MMA issue. A whole warp runs the issue loop, so that its addresses and
+// descriptors stay in uniform registers; the instructions themselves are
+// predicated on `leader`, nonzero in one lane, the same one throughout.
+//
+// Waits as mbar_wait_bounded, the answer the same in all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long limit_cycles) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, limit_cycles));
 }
-// D[tmem] (+)= A[smem] * B[smem], TF32 inputs, FP32 accumulate.
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
+// Arrives on `bar` once every tcgen05.mma the leader issued so far is done.
+__device__ __forceinline__ void tc_commit(uint64_t* bar, uint32_t leader) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        :: "r"(smem_u32(bar)), "r"(leader) : "memory");
 }
+// D[tmem] (+)= A[smem] * B[smem], FP32 accumulate; TF32 or BF16 inputs, one CTA
+// (CTAS 1) or a pair (2). Descriptors by halves: only the address half differs
+// between the MMAs of a stage.
+#define MMSK_MMA(NAME, FORM)                                                                                     \
+    __device__ __forceinline__ void NAME(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, \
+                                         uint32_t idesc, uint32_t accumulate, uint32_t leader) {                 \
+        asm volatile(                                                                                            \
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"                                                      \
+            "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"                                                \
+            "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"                                                  \
+            "@q tcgen05.mma." FORM " [%0], a, b, %5, p;\n\t}"                                                    \
+            :: "r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)   \
+            : "memory");                                                                                         \
+    }
+MMSK_MMA(mma_tf32, "cta_group::1.kind::tf32")
+MMSK_MMA(mma_bf16, "cta_group::1.kind::f16")
+MMSK_MMA(mma_tf32_pair, "cta_group::2.kind::tf32")
+MMSK_MMA(mma_bf16_pair, "cta_group::2.kind::f16")
+#undef MMSK_MMA
 // D[tmem] (+)= A[tmem] * B[smem], BF16 inputs, FP32 accumulate. A is M rows
 // in M lanes from column a_tmem on, two consecutive k's per 32-bit column
 // (the lower k in the low half): 8 columns per 16 k.
-__device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
+__device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi,
+                                            uint32_t idesc, uint32_t accumulate, uint32_t leader) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        :: "r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// D[tmem] (+)= A[smem] * B[smem], BF16 inputs, FP32 accumulate.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+        :: "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
 // 32 lanes x 32 columns of 32-bit TMEM: thread i of the warp gets lane
 // (base lane + i), columns [col, col + 32).
@@ -267,45 +280,34 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(taddr), "r"(ncols) : "memory");
 }
 // Arrives on `bar` (same shared offset) in every CTA of `cta_mask` once the
-// pair MMAs this thread issued are done.
-__device__ __forceinline__ void tc_commit_pair_multicast(uint64_t* bar, uint16_t cta_mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 :: "r"(smem_u32(bar)), "h"(cta_mask) : "memory");
-}
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 :: "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mma_tf32_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
+// pair MMAs the leader issued are done.
+__device__ __forceinline__ void tc_commit_pair_multicast(uint64_t* bar, uint16_t cta_mask, uint32_t leader) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+        :: "r"(smem_u32(bar)), "h"(cta_mask), "r"(leader) : "memory");
 }
-__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint32_t leader) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        :: "r"(smem_u32(bar)), "r"(leader) : "memory");
 }
 
 // ---------------------------------------------------------------- descriptors
 // Shared-memory matrix descriptor (tcgen05 form): start address, leading and
 // stride byte offsets (all >> 4), version 1, base offset 0, swizzle mode.
 //   swizzle: 0 none, 2 = 128-byte, 4 = 64-byte, 6 = 32-byte.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes,
-                                                   uint32_t swizzle) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1u << 46;                         // descriptor version for tcgen05
-    d |= (uint64_t)(swizzle & 0x7u) << 61;
-    return d;
+// Low half: the address and the leading offset. An address further on (shared
+// addresses are below 256 KB, 14 bits of 16 bytes) is a plain add of bytes >> 4.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
+    return ((saddr >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
+}
+// High half: the stride offset, the version (1 for tcgen05) and the swizzle.
+__host__ __device__ constexpr uint32_t smem_desc_hi(uint32_t sbo_bytes, uint32_t swizzle) {
+    return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | ((swizzle & 0x7u) << 29);
 }
 
 // Instruction descriptor for kind::tf32 / kind::f16 with FP32 accumulation.

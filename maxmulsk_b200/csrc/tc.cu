@@ -425,7 +425,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __shared__ volatile int abort_s;
 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -489,54 +489,59 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int acc = 0;
-            uint32_t acc_phase = 0;
-            bool ok = true;
-            for (int64_t u = blockIdx.x; u < p.units && ok && !abort_s; u += gridDim.x) {
-                const int64_t nkb = kblocks(decode_unit(p, u));
-                for (int64_t kb0 = 0; kb0 < nkb && ok; kb0 += p.chunk_kb) {
-                    // one chunk of up to CHUNK_KB stages into accumulator `acc`
-                    if (!mbar_wait_bounded(&tempty_bar[acc], acc_phase ^ 1u, p.timeout)) { fail(); ok = false; break; }
+        // The whole warp, lane 0 issuing (sm100.cuh): with one lane in a branch
+        // of its own every MMA's descriptors were built in vector registers and
+        // moved over: about 108 clocks an MMA against the 64 that a 128-column
+        // one takes, and an empty MMA queue at every chunk boundary. GEMM alone
+        // at 2048^3 (chunks of 32): 128 x 256 3xTF32 86.7 -> 67.4 us, BF16x6 80.0 ->
+        // 68.5, BF16x9 105.7 -> 95.3; 128 x 128 BF16x6 127 -> 94.
+        const uint32_t leader = lane == 0;
+        const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), 16u);
+        const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem) + Cf::P * Cf::A_PLANE, Cf::B_KMAJOR ? 16u : (uint32_t)(Cf::BK * 128));
+        constexpr uint32_t A_HI = smem_desc_hi(512u, 4u);
+        constexpr uint32_t B_HI = Cf::B_KMAJOR ? smem_desc_hi(512u, 4u) : smem_desc_hi(1024u, 2u);
+        int stage = 0;
+        uint32_t phase = 0;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < p.units && ok && !__any_sync(0xffffffffu, abort_s); u += gridDim.x) {
+            const int nkb = (int)kblocks(decode_unit(p, u));
+            for (int kb0 = 0; kb0 < nkb && ok; kb0 += p.chunk_kb) {
+                // one chunk of up to chunk_kb stages into accumulator `acc`
+                if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1u, p.timeout)) { fail(); ok = false; break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+                const int kb1 = min(nkb, kb0 + p.chunk_kb);
+                for (int kb = kb0; kb < kb1; kb++) {
+                    if (!mbar_wait_warp(&full_bar[stage], phase, p.timeout)) { fail(); ok = false; break; }
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-                    const int64_t kb1 = min(nkb, kb0 + (int64_t)p.chunk_kb);
-                    for (int64_t kb = kb0; kb < kb1; kb++) {
-                        if (!mbar_wait_bounded(&full_bar[stage], phase, p.timeout)) { fail(); ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t a_base = smem_u32(smem + (size_t)stage * Cf::STAGE);
-                        const uint32_t b_base = a_base + Cf::P * Cf::A_PLANE;
+                    const uint32_t a_lo = a_lo0 + (uint32_t)(stage * (Cf::STAGE >> 4));
+                    const uint32_t b_lo = b_lo0 + (uint32_t)(stage * (Cf::STAGE >> 4));
 #pragma unroll
-                        for (int ks = 0; ks < Cf::KSTEPS; ks++) {
+                    for (int ks = 0; ks < Cf::KSTEPS; ks++) {
 #pragma unroll
-                            for (int q = 0; q < Cf::NPROD; q++) {
-                                int pa, pb;
-                                product_planes(MODE, q, pa, pb);
-                                const uint64_t adesc = make_smem_desc(
-                                    a_base + (uint32_t)(pa * Cf::A_PLANE + ks * 32), 16u, 512u, 4u);
-                                const uint64_t bdesc = Cf::B_KMAJOR
-                                    ? make_smem_desc(b_base + (uint32_t)(pb * Cf::B_PLANE + ks * 32), 16u, 512u, 4u)
-                                    : make_smem_desc(b_base + (uint32_t)(pb * Cf::B_PLANE + ks * Cf::KSTEP * 128),
-                                                     (uint32_t)(Cf::BK * 128), 1024u, 2u);
-                                const uint32_t accum = (kb > kb0 || ks > 0 || q > 0) ? 1u : 0u;
-                                if constexpr (Cf::TF32) mma_tf32(d_tmem, adesc, bdesc, Cf::IDESC, accum);
-                                else mma_bf16(d_tmem, adesc, bdesc, Cf::IDESC, accum);
-                            }
+                        for (int q = 0; q < Cf::NPROD; q++) {
+                            int pa, pb;
+                            product_planes(MODE, q, pa, pb);
+                            const uint32_t ao = (uint32_t)(pa * Cf::A_PLANE + ks * 32) >> 4;
+                            const uint32_t bo = (uint32_t)(pb * Cf::B_PLANE + ks * (Cf::B_KMAJOR ? 32 : Cf::KSTEP * 128)) >> 4;
+                            const uint32_t accum = (ks > 0 || q > 0) ? 1u : (uint32_t)(kb > kb0);
+                            if constexpr (Cf::TF32) mma_tf32(d_tmem, a_lo + ao, A_HI, b_lo + bo, B_HI, Cf::IDESC, accum, leader);
+                            else mma_bf16(d_tmem, a_lo + ao, A_HI, b_lo + bo, B_HI, Cf::IDESC, accum, leader);
                         }
-                        tc_commit(&empty_bar[stage]);
-                        if (++stage == Cf::STAGES) { stage = 0; phase ^= 1u; }
                     }
-                    if (!ok) break;
-                    tc_commit(&tfull_bar[acc]);
-                    if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
+                    tc_commit(&empty_bar[stage], leader);
+                    if (++stage == Cf::STAGES) { stage = 0; phase ^= 1u; }
                 }
+                if (!ok) break;
+                tc_commit(&tfull_bar[acc], leader);
+                if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
             }
-            // No MMA may still be running when TMEM is freed.
-            tc_commit(&done_bar);
-            if (!mbar_wait_bounded(&done_bar, 0u, p.timeout)) { atomicOr(p.err, kErrTimeout); abort_s = 1; }
         }
+        // No MMA may still be running when TMEM is freed.
+        tc_commit(&done_bar, leader);
+        if (!mbar_wait_warp(&done_bar, 0u, p.timeout)) { atomicOr(p.err, kErrTimeout); abort_s = 1; }
     } else {
         // ------------------------------------------------------------ epilogue
         uint8_t* cbuf = (Cf::TMA_STORE && p.store_c) ? smem + Cf::RING + (warp - 2) * kStoreWarpBytes : nullptr;
@@ -611,9 +616,9 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     __shared__ volatile int abort_s;
 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler
     const int lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_ctarank() & 1u;
+    const uint32_t rank = __shfl_sync(0xffffffffu, cluster_ctarank() & 1u, 0);
     const bool leader = (rank == 0);
     const int64_t pair = blockIdx.x >> 1;
     const int64_t npairs = gridDim.x >> 1;
@@ -684,52 +689,53 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer (leader only)
-        if (lane == 0 && leader) {
+        // ------------------------------------------------------------ MMA issuer (leader CTA only; as above)
+        if (leader) {
+            const uint32_t lead = lane == 0;
+            const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), 16u);
+            const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem) + Cf::P * Cf::A_PLANE, Cf::B_KMAJOR ? 16u : (uint32_t)(Cf::BK * 128));
+            constexpr uint32_t A_HI = smem_desc_hi(512u, 4u);
+            constexpr uint32_t B_HI = Cf::B_KMAJOR ? smem_desc_hi(512u, 4u) : smem_desc_hi(1024u, 2u);
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
             uint32_t acc_phase = 0;
             bool ok = true;
-            for (int64_t u = pair; u < p.units && ok && !abort_s; u += npairs) {
-                const int64_t nkb = kblocks(decode_unit(p, u));
-                for (int64_t kb0 = 0; kb0 < nkb && ok; kb0 += p.chunk_kb) {
-                    if (!mbar_wait_bounded(&tempty_bar[acc], acc_phase ^ 1u, p.timeout)) { fail(); ok = false; break; }
+            for (int64_t u = pair; u < p.units && ok && !__any_sync(0xffffffffu, abort_s); u += npairs) {
+                const int nkb = (int)kblocks(decode_unit(p, u));
+                for (int kb0 = 0; kb0 < nkb && ok; kb0 += p.chunk_kb) {
+                    if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1u, p.timeout)) { fail(); ok = false; break; }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-                    const int64_t kb1 = min(nkb, kb0 + (int64_t)p.chunk_kb);
-                    for (int64_t kb = kb0; kb < kb1; kb++) {
-                        if (!mbar_wait_bounded(&full_bar[stage], phase, p.timeout)) { fail(); ok = false; break; }
+                    const int kb1 = min(nkb, kb0 + p.chunk_kb);
+                    for (int kb = kb0; kb < kb1; kb++) {
+                        if (!mbar_wait_warp(&full_bar[stage], phase, p.timeout)) { fail(); ok = false; break; }
                         tc_fence_after();
-                        const uint32_t a_base = smem_u32(smem + (size_t)stage * Cf::STAGE);
-                        const uint32_t b_base = a_base + Cf::P * Cf::A_PLANE;
+                        const uint32_t a_lo = a_lo0 + (uint32_t)(stage * (Cf::STAGE >> 4));
+                        const uint32_t b_lo = b_lo0 + (uint32_t)(stage * (Cf::STAGE >> 4));
 #pragma unroll
                         for (int ks = 0; ks < Cf::KSTEPS; ks++) {
 #pragma unroll
                             for (int q = 0; q < Cf::NPROD; q++) {
                                 int pa, pb;
                                 product_planes(MODE, q, pa, pb);
-                                const uint64_t adesc = make_smem_desc(
-                                    a_base + (uint32_t)(pa * Cf::A_PLANE + ks * 32), 16u, 512u, 4u);
-                                const uint64_t bdesc = Cf::B_KMAJOR
-                                    ? make_smem_desc(b_base + (uint32_t)(pb * Cf::B_PLANE + ks * 32), 16u, 512u, 4u)
-                                    : make_smem_desc(b_base + (uint32_t)(pb * Cf::B_PLANE + ks * Cf::KSTEP * 128),
-                                                     (uint32_t)(Cf::BK * 128), 1024u, 2u);
-                                const uint32_t accum = (kb > kb0 || ks > 0 || q > 0) ? 1u : 0u;
-                                if constexpr (Cf::TF32) mma_tf32_pair(d_tmem, adesc, bdesc, Cf::IDESC, accum);
-                                else mma_bf16_pair(d_tmem, adesc, bdesc, Cf::IDESC, accum);
+                                const uint32_t ao = (uint32_t)(pa * Cf::A_PLANE + ks * 32) >> 4;
+                                const uint32_t bo = (uint32_t)(pb * Cf::B_PLANE + ks * (Cf::B_KMAJOR ? 32 : Cf::KSTEP * 128)) >> 4;
+                                const uint32_t accum = (ks > 0 || q > 0) ? 1u : (uint32_t)(kb > kb0);
+                                if constexpr (Cf::TF32) mma_tf32_pair(d_tmem, a_lo + ao, A_HI, b_lo + bo, B_HI, Cf::IDESC, accum, lead);
+                                else mma_bf16_pair(d_tmem, a_lo + ao, A_HI, b_lo + bo, B_HI, Cf::IDESC, accum, lead);
                             }
                         }
-                        tc_commit_pair_multicast(&empty_bar[stage], (uint16_t)0x3);
+                        tc_commit_pair_multicast(&empty_bar[stage], (uint16_t)0x3, lead);
                         if (++stage == Cf::STAGES) { stage = 0; phase ^= 1u; }
                     }
                     if (!ok) break;
-                    tc_commit_pair_multicast(&tfull_bar[acc], (uint16_t)0x3);
+                    tc_commit_pair_multicast(&tfull_bar[acc], (uint16_t)0x3, lead);
                     if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
                 }
             }
-            tc_commit_pair(&done_bar);
-            if (!mbar_wait_bounded(&done_bar, 0u, p.timeout)) { atomicOr(p.err, kErrTimeout); abort_s = 1; }
+            tc_commit_pair(&done_bar, lead);
+            if (!mbar_wait_warp(&done_bar, 0u, p.timeout)) { atomicOr(p.err, kErrTimeout); abort_s = 1; }
         }
     } else {
         // ------------------------------------------------------------ epilogue (both CTAs)
@@ -1081,7 +1087,7 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* ops = smem;                                        // operand ring (1024-aligned stages)
     uint8_t* stg = smem + Cf::OP_STAGES * Cf::OP_STAGE;         // staging ring
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler
     const int lane = threadIdx.x & 31;
     constexpr int CONV0 = 2 + Cf::EPI;                          // first converter warp
 
@@ -1164,53 +1170,53 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int acc = 0;
-            uint32_t acc_phase = 0;
-            bool ok = true;
-            for (int64_t round = 0, u = src.unit_of(0); u < src.units() && ok && !abort_s; u = src.unit_of(++round)) {
-                UnitView v;
-                src.get(u, v);
-                const int64_t nkb = kblocks(v.w);
-                for (int64_t kb0 = 0; kb0 < nkb && ok; kb0 += v.chunk_kb) {
-                    if (!mbar_wait_bounded(&tempty_bar[acc], acc_phase ^ 1u, timeout)) { fail(); ok = false; break; }
+        // ------------------------------------------------------------ MMA issuer (as in tc_gemm_kernel)
+        const uint32_t leader = lane == 0;
+        const uint32_t b_lo0 = smem_desc_lo(smem_u32(ops), (uint32_t)(Cf::BK * 128));
+        constexpr uint32_t B_HI = smem_desc_hi(1024u, 2u);
+        int stage = 0;
+        uint32_t phase = 0;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        for (int64_t round = 0, u = src.unit_of(0); u < src.units() && ok && !__any_sync(0xffffffffu, abort_s);
+             u = src.unit_of(++round)) {
+            UnitView v;
+            src.get(u, v);
+            const int nkb = (int)kblocks(v.w);
+            for (int kb0 = 0; kb0 < nkb && ok; kb0 += v.chunk_kb) {
+                if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1u, timeout)) { fail(); ok = false; break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+                const int kb1 = min(nkb, kb0 + v.chunk_kb);
+                for (int kb = kb0; kb < kb1; kb++) {
+                    if (!mbar_wait_warp(&op_full[stage], phase, timeout)) { fail(); ok = false; break; }
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-                    const int64_t kb1 = min(nkb, kb0 + (int64_t)v.chunk_kb);
-                    for (int64_t kb = kb0; kb < kb1; kb++) {
-                        if (!mbar_wait_bounded(&op_full[stage], phase, timeout)) { fail(); ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t a_tm = tmem_base + Cf::A_COL + (uint32_t)stage * Cf::A_SLOT;
-                        const uint32_t b_base = smem_u32(ops + (size_t)stage * Cf::OP_STAGE);
+                    const uint32_t a_tm = tmem_base + Cf::A_COL + (uint32_t)stage * Cf::A_SLOT;
+                    const uint32_t b_lo = b_lo0 + (uint32_t)(stage * (Cf::OP_STAGE >> 4));
 #pragma unroll
-                        for (int ks = 0; ks < Cf::KSTEPS; ks++) {
+                    for (int ks = 0; ks < Cf::KSTEPS; ks++) {
 #pragma unroll
-                            for (int q = 0; q < Cf::NPROD; q++) {
-                                int pa, pb;
-                                product_planes(MODE, q, pa, pb);
-                                const uint32_t a_addr = a_tm + (uint32_t)(pa * (Cf::BK / 2) + ks * (Cf::KSTEP / 2));
-                                const uint64_t bdesc =
-                                    make_smem_desc(b_base + (uint32_t)(pb * Cf::B_PLANE + ks * Cf::KSTEP * 128),
-                                                   (uint32_t)(Cf::BK * 128), 1024u, 2u);
-                                const uint32_t accum = (kb > kb0 || ks > 0 || q > 0) ? 1u : 0u;
-                                mma_bf16_ta(d_tmem, a_addr, bdesc, Cf::IDESC, accum);
-                            }
+                        for (int q = 0; q < Cf::NPROD; q++) {
+                            int pa, pb;
+                            product_planes(MODE, q, pa, pb);
+                            const uint32_t ao = (uint32_t)(pa * (Cf::BK / 2) + ks * (Cf::KSTEP / 2));
+                            const uint32_t bo = (uint32_t)(pb * Cf::B_PLANE + ks * Cf::KSTEP * 128) >> 4;
+                            const uint32_t accum = (ks > 0 || q > 0) ? 1u : (uint32_t)(kb > kb0);
+                            mma_bf16_ta(d_tmem, a_tm + ao, b_lo + bo, B_HI, Cf::IDESC, accum, leader);
                         }
-                        tc_commit(&op_empty[stage]);
-                        if (++stage == Cf::OP_STAGES) { stage = 0; phase ^= 1u; }
                     }
-                    if (!ok) break;
-                    tc_commit(&tfull_bar[acc]);
-                    if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
+                    tc_commit(&op_empty[stage], leader);
+                    if (++stage == Cf::OP_STAGES) { stage = 0; phase ^= 1u; }
                 }
+                if (!ok) break;
+                tc_commit(&tfull_bar[acc], leader);
+                if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
             }
-            // No MMA may still be running when TMEM is freed.
-            tc_commit(&done_bar);
-            if (!mbar_wait_bounded(&done_bar, 0u, timeout)) { atomicOr(err, kErrTimeout); abort_s = 1; }
         }
+        // No MMA may still be running when TMEM is freed.
+        tc_commit(&done_bar, leader);
+        if (!mbar_wait_warp(&done_bar, 0u, timeout)) { atomicOr(err, kErrTimeout); abort_s = 1; }
     } else if (warp < CONV0) {
         // ------------------------------------------------------------ epilogue
         epilogue_role_tsum<Cf>(src, err, timeout, tmem_base, tfull_bar, tempty_bar, abort_s, warp, lane);
