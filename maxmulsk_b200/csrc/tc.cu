@@ -851,8 +851,10 @@ cudaError_t set_smem_once(Kern kern, int bytes, std::atomic<uint64_t>& done) {
 // Fused-split variant (BF16x6 / BF16x9, 128 x 128 tiles). The operands are
 // split inside the kernel instead of by the pre-pass. Warp 0 loads FP32 tiles
 // of A (128 rows x 32 k) and B (32 k x 128 n, as four 32-column boxes) with
-// TMA and the 128-byte swizzle into a staging ring, a few stages after an L2
-// prefetch of the same boxes; eight converter warps cut each staged element
+// TMA and the 128-byte swizzle into a staging ring of five stages (160 KB in
+// flight an SM; L2 prefetches of the boxes, which once ran ahead of it, cost more
+// TMA issue than they hid: 128 x 32768 x 512 32.5 -> 29.6 us without); eight
+// converter warps cut each staged element
 // into its three BF16 limbs (split_math.cuh, the pre-pass's arithmetic). A's
 // limbs go to tensor memory, one row per TMEM lane, where the MMA reads them
 // as its A operand; B's limb planes go to an operand ring in shared memory in
@@ -882,8 +884,6 @@ struct CfgFused {
     static constexpr int NBOX = BN / 32;
     static constexpr int ST_STAGE = ST_A + NBOX * ST_BOX;
     static constexpr int ST_STAGES = 5;
-    static constexpr int PREFETCH = 6;               // stages between a box's L2 prefetch and its load
-    static_assert(PREFETCH >= ST_STAGES, "prefetches run ahead of the staging ring");
     static constexpr int RING = OP_STAGES * OP_STAGE + ST_STAGES * ST_STAGE;
     static constexpr int NPROD = (MODE == MAXMULSK_PREC_BF16X6) ? 6 : 9;
     static constexpr uint32_t IDESC = make_idesc(1u, 128u, (uint32_t)BN, 1u);
@@ -1131,16 +1131,6 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
                 const void* mapB = src.map_b(v, tmB1);
                 src.acquire(mapA, mapB);
                 const int64_t nkb = kblocks(w);
-                // The FP32 boxes of stage j go to L2 PREFETCH stages before
-                // their load, which then waits for L2 instead of HBM. The
-                // first stages are loaded at once (their loads go to HBM
-                // themselves); each prefetch follows a load.
-                auto prefetch = [&](int64_t j) {
-                    const int32_t k = (int32_t)(w.kbeg + j * Cf::BK);
-                    tma_prefetch_l2_2d(mapA, k, w.tm * Cf::BM);
-#pragma unroll
-                    for (int b = 0; b < Cf::NBOX; b++) tma_prefetch_l2_2d(mapB, w.tn * BN + 32 * b, k);
-                };
                 bool ok = true;
                 for (int64_t kb = 0; kb < nkb; kb++) {
                     if (!mbar_wait_bounded(&st_empty[stage], phase ^ 1u, timeout)) { fail(); ok = false; break; }
@@ -1152,9 +1142,6 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
 #pragma unroll
                     for (int b = 0; b < Cf::NBOX; b++)
                         tma_load_2d(sa + Cf::ST_A + b * Cf::ST_BOX, mapB, &st_full[stage], w.tn * BN + 32 * b, k);
-                    // Stages the ring does not hold yet: prefetched behind this load.
-                    for (int64_t j = (kb == 0 ? Cf::ST_STAGES : kb + Cf::PREFETCH); j <= kb + Cf::PREFETCH && j < nkb; j++)
-                        prefetch(j);
                     issued++;
                     if (++stage == Cf::ST_STAGES) { stage = 0; phase ^= 1u; }
                 }
@@ -1240,77 +1227,64 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
             src.get(u, v);
             const int64_t nkb = kblocks(v.w);
             for (int64_t kb = 0; kb < nkb; kb++) {
-                int bad = abort_s;
-                if (!bad && lane == 0) {
-                    if (!mbar_wait_bounded(&op_empty[ostage], ophase ^ 1u, timeout) ||
-                        !mbar_wait_bounded(&st_full[stage], phase, timeout)) {
-                        fail();
-                        bad = 1;
-                    }
+                // The staged tile is read and cut before the operand slot is
+                // waited for, so only the stores follow the MMAs that last read
+                // it. BF16x6 at 128 x 32768 x 512 / 1024^3 with the reduction 36.8 /
+                // 29.3 us when the slot was waited for first; BF16x9 42.9 / 39.8 ->
+                // 35.4 / 27.9 (with the whole-warp MMA issue), 32.8 / 27.1 without
+                // L2 prefetches. Sixteen converter warps: 32.8 against 30.7.
+                if (!__all_sync(0xffffffffu, !abort_s && mbar_wait_bounded(&st_full[stage], phase, timeout))) {
+                    fail();
+                    stop = true;
+                    break;
                 }
-                bad = __shfl_sync(0xffffffffu, bad, 0);
-                if (bad) { stop = true; break; }
-                const uint8_t* sa = stg + (size_t)stage * Cf::ST_STAGE;
-                uint8_t* oa = ops + (size_t)ostage * Cf::OP_STAGE;
-                if (conv_a) {
-                    // A row r: 32 FP32 k's (128-byte row, 128-byte swizzle) ->
-                    // three limbs of 16 packed k pairs, stored in TMEM lane r at
-                    // columns A_COL + A_SLOT ostage + 16 p + pair.
-                    const int quarter = warp & 3;
-                    const int r = quarter * 32 + lane;
+                const int r = conv_a ? (warp & 3) * 32 + lane : lane;     // A row (its TMEM lane), or k row of box cw
+                const uint8_t* sx = stg + (size_t)stage * Cf::ST_STAGE + (conv_a ? 0 : Cf::ST_A + cw * Cf::ST_BOX) + r * 128;
+                uint32_t l0[16], l1[16], l2[16];
+                {
                     float x[32];
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
-                        const float4 v = *reinterpret_cast<const float4*>(sa + r * 128 + ((c ^ (r & 7)) << 4));
+                        const float4 v = *reinterpret_cast<const float4*>(sx + ((c ^ (r & 7)) << 4));
                         x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
                     }
-                    // The MMAs that read this slot (two stages back) are done.
+#pragma unroll
+                    for (int e = 0; e < 16; e++) bf16_limbs2(x[2 * e], x[2 * e + 1], l0[e], l1[e], l2[e]);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&st_empty[stage]);
+                if (!mbar_wait_warp(&op_empty[ostage], ophase ^ 1u, timeout)) { fail(); stop = true; break; }
+                if (conv_a) {
+                    // Three limbs of 16 packed k pairs, in TMEM lane r at columns
+                    // A_COL + A_SLOT ostage + 16 p + pair. The MMAs that read this
+                    // slot (two stages back) are done.
                     tc_fence_after();
-                    const uint32_t ta = tmem_base + ((uint32_t)(quarter * 32) << 16) + Cf::A_COL +
+                    const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + Cf::A_COL +
                                         (uint32_t)ostage * Cf::A_SLOT;
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        uint32_t l0[8], l1[8], l2[8];
-#pragma unroll
-                        for (int e = 0; e < 8; e++)
-                            bf16_limbs2(x[16 * h + 2 * e], x[16 * h + 2 * e + 1], l0[e], l1[e], l2[e]);
-                        tmem_st_32x32b_x8(ta + (uint32_t)(8 * h), l0);
-                        tmem_st_32x32b_x8(ta + (uint32_t)(16 + 8 * h), l1);
-                        tmem_st_32x32b_x8(ta + (uint32_t)(32 + 8 * h), l2);
-                    }
+                    tmem_st_32x32b_x16(ta, l0);
+                    tmem_st_32x32b_x16(ta + 16u, l1);
+                    tmem_st_32x32b_x16(ta + 32u, l2);
                     // The limbs are in TMEM before the MMA warp is told.
                     tmem_wait_st();
                     tc_fence_before();
                 } else {
-                    // B row k of box cw: 32 FP32 n's -> four 16-byte chunks of
-                    // 8 BF16 in column panel cw / 2, chunks 4 (cw % 2) .. +3.
-                    const int k = lane;
-                    const uint8_t* sb = sa + Cf::ST_A + cw * Cf::ST_BOX;
-                    float x[32];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        const float4 v = *reinterpret_cast<const float4*>(sb + k * 128 + ((c ^ (k & 7)) << 4));
-                        x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
-                    }
-                    uint8_t* ob = oa + (cw >> 1) * (Cf::BK * 128) + k * 128;
+                    // Four 16-byte chunks of 8 BF16 in column panel cw / 2,
+                    // chunks 4 (cw % 2) .. +3.
+                    uint8_t* ob = ops + (size_t)ostage * Cf::OP_STAGE + (cw >> 1) * (Cf::BK * 128) + r * 128;
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        uint32_t l0[4], l1[4], l2[4];
-#pragma unroll
-                        for (int e = 0; e < 4; e++) bf16_limbs2(x[8 * j + 2 * e], x[8 * j + 2 * e + 1], l0[e], l1[e], l2[e]);
-                        const int off = ((((cw & 1) * 4 + j) ^ (k & 7)) << 4);
-                        *reinterpret_cast<uint4*>(ob + off) = make_uint4(l0[0], l0[1], l0[2], l0[3]);
-                        *reinterpret_cast<uint4*>(ob + Cf::B_PLANE + off) = make_uint4(l1[0], l1[1], l1[2], l1[3]);
-                        *reinterpret_cast<uint4*>(ob + 2 * Cf::B_PLANE + off) = make_uint4(l2[0], l2[1], l2[2], l2[3]);
+                        const int off = ((((cw & 1) * 4 + j) ^ (r & 7)) << 4);
+                        *reinterpret_cast<uint4*>(ob + off) = make_uint4(l0[4 * j], l0[4 * j + 1], l0[4 * j + 2], l0[4 * j + 3]);
+                        *reinterpret_cast<uint4*>(ob + Cf::B_PLANE + off) =
+                            make_uint4(l1[4 * j], l1[4 * j + 1], l1[4 * j + 2], l1[4 * j + 3]);
+                        *reinterpret_cast<uint4*>(ob + 2 * Cf::B_PLANE + off) =
+                            make_uint4(l2[4 * j], l2[4 * j + 1], l2[4 * j + 2], l2[4 * j + 3]);
                     }
                     // The planes are read by the tensor cores (async proxy).
                     fence_proxy_async();
                 }
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&op_full[ostage]);
-                    mbar_arrive(&st_empty[stage]);
-                }
+                if (lane == 0) mbar_arrive(&op_full[ostage]);
                 if (++stage == Cf::ST_STAGES) { stage = 0; phase ^= 1u; }
                 if (++ostage == Cf::OP_STAGES) { ostage = 0; ophase ^= 1u; }
             }
