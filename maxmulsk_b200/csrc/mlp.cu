@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "internal.hpp"
+#include "launch.cuh"
 #include "mlp.hpp"
 #include "runtime.hpp"
 #include "split_math.cuh"
@@ -65,6 +66,7 @@ mlp_forward_kernel(const float* __restrict__ params, const float* __restrict__ X
     __shared__ __align__(16) float in[2][kFwdRows][H];           // X or H2, and H1
     const int tid = threadIdx.x, o = tid & 63, rq = tid >> 6;
     const int b0 = blockIdx.x * kFwdRows;
+    grid_wait();
 #pragma unroll
     for (int j = 0; j < (NPARAM + 255) / 256; j++)
         if (tid + j * 256 < NPARAM) w[tid + j * 256] = params[tid + j * 256];
@@ -146,6 +148,7 @@ mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ 
     __shared__ __align__(16) float dy[R][O], h2[R][H], dz2[R][H], h1[R][H], dz1[R][H];
     __shared__ float xs[R][F];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    grid_wait();
 #pragma unroll
     for (int i = tid; i < H * O; i += 256) w3[i / O][i % O] = params[OFF_W3 + i];
 #pragma unroll
@@ -299,6 +302,7 @@ mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ 
 // grads[i] = parts[0][i] + parts[1][i] + ..., in block order.
 __global__ void __launch_bounds__(128)
 mlp_grad_sum(const float* __restrict__ parts, int n, float* __restrict__ grads) {
+    grid_wait();
     const int i = blockIdx.x * 128 + threadIdx.x;
     if (i < NPARAM) grads[i] = ordered_sum<31>(parts + i, (size_t)NPARAM, n);
 }
@@ -306,6 +310,7 @@ mlp_grad_sum(const float* __restrict__ parts, int n, float* __restrict__ grads) 
 // Adam (bias-corrected), elementwise.
 __global__ void adam_step(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                           float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float c1, float c2) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -534,8 +539,8 @@ maxmulsk_status maxmulsk_mlp_forward_dev(const float* params, const float* X, in
     if (B == 0) return MAXMULSK_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)(((int64_t)B + kFwdRows - 1) / kFwdRows);
-    mlp_forward_kernel<<<grid, 256, 0, s>>>(params, X, B, Z1, H1, Z2, H2, Y);
-    return cuda_status(cudaGetLastError(), "mlp forward");
+    return cuda_status(launch_overlapped(mlp_forward_kernel, dim3(grid), 256, 0, s, 1, params, X, (int)B, Z1, H1, Z2, H2, Y),
+                       "mlp forward");
 }
 
 maxmulsk_status maxmulsk_mlp_backward_dev(const float* params, const float* X, const float* Z1, const float* H1,
@@ -555,31 +560,19 @@ maxmulsk_status maxmulsk_mlp_backward_dev(const float* params, const float* X, c
     const int64_t each = (turns + wave - 1) / wave;
     const int64_t want = (turns + each * kBwdCluster - 1) / (each * kBwdCluster);
     const int nc = (int)std::max<int64_t>(1, std::min(want, fit));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(nc * kBwdCluster));
-    cfg.blockDim = dim3(256);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kBwdCluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, mlp_backward_kernel, params, X, Z1, H1, Z2, H2, Y, T, mask, (int)B,
-                                             1.0f / count, nc > 1 ? work : grads, rowloss);
-    if (e != cudaSuccess) return cuda_status(e, "mlp backward");
-    if (nc > 1) mlp_grad_sum<<<(NPARAM + 127) / 128, 128, 0, s>>>(work, nc, grads);
-    return cuda_status(cudaGetLastError(), "mlp backward");
+    cudaError_t e = launch_overlapped(mlp_backward_kernel, dim3((unsigned)(nc * kBwdCluster)), 256, 0, s, kBwdCluster, params,
+                                      X, Z1, H1, Z2, H2, Y, T, mask, (int)B, 1.0f / count, nc > 1 ? work : grads, rowloss);
+    if (e == cudaSuccess && nc > 1)
+        e = launch_overlapped(mlp_grad_sum, dim3((NPARAM + 127) / 128), 128, 0, s, 1, (const float*)work, nc, grads);
+    return cuda_status(e, "mlp backward");
 }
 
 maxmulsk_status maxmulsk_mlp_adam_dev(float* params, const float* grads, float* m, float* v, float lr, float beta1,
                                       float beta2, float eps, int32_t step, void* stream) {
     if (!params || !grads || !m || !v || step < 1) return MAXMULSK_ERR_INVALID;
     const float c1 = 1.0f - std::pow(beta1, (float)step), c2 = 1.0f - std::pow(beta2, (float)step);
-    adam_step<<<blocks(NPARAM), 256, 0, static_cast<cudaStream_t>(stream)>>>(params, grads, m, v, NPARAM, lr, beta1,
-                                                                              beta2, eps, c1, c2);
-    return cuda_status(cudaGetLastError(), "mlp adam");
+    return cuda_status(launch_overlapped(adam_step, dim3(blocks(NPARAM)), 256, 0, static_cast<cudaStream_t>(stream), 1, params,
+                                         grads, m, v, (int)NPARAM, lr, beta1, beta2, eps, c1, c2), "mlp adam");
 }
 
 maxmulsk_status maxmulsk_mlp_predict_dev(const float* params, const float* X, const float* mask, int32_t B,

@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "internal.hpp"
+#include "launch.cuh"
 #include "phase.hpp"
 #include "runtime.hpp"
 #include "split_math.cuh"
@@ -401,6 +402,7 @@ __global__ void __launch_bounds__(Cf::THREADS, Cf::CTAS)
 sgemm_simt_cp_kernel(SimtArgs p) {
     extern __shared__ __align__(16) float smem[];
     __shared__ int last_flag;
+    grid_wait();
     simt_cp_tile<Cf, FUSED>(p, (int64_t)blockIdx.y * Cf::BM, (int64_t)blockIdx.x * Cf::BN, blockIdx.z,
                             blockIdx.y * gridDim.x + blockIdx.x, smem, last_flag);
 }
@@ -416,6 +418,7 @@ sgemm_simt_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUni
     extern __shared__ __align__(16) float smem[];
     __shared__ int last_flag;
     __shared__ int s_unit;
+    grid_wait();
     // Thread 0 fetches the next unit's number while the current one runs.
     unsigned fetched = threadIdx.x == 0 ? atomicAdd(next, 1u) : 0u;
     for (;;) {
@@ -446,6 +449,7 @@ sgemm_simt_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUni
 template <int BATCH, typename T>
 __global__ void __launch_bounds__(256)
 simt_splitk_reduce_kernel(const T* __restrict__ partial, T* __restrict__ C, int64_t n, int splits) {
+    grid_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) C[i] = ordered_sum<BATCH>(partial + i, (size_t)n, splits);
 }
@@ -455,11 +459,10 @@ cudaError_t launch_splitk_reduce(const float* partial, float* C, int64_t n, int 
     const unsigned blocks = (unsigned)((n + 255) / 256);
     const T* src = reinterpret_cast<const T*>(partial);
     T* dst = reinterpret_cast<T*>(C);
-    if (splits <= 4) simt_splitk_reduce_kernel<3><<<blocks, 256, 0, s>>>(src, dst, n, splits);
-    else if (splits <= 8) simt_splitk_reduce_kernel<7><<<blocks, 256, 0, s>>>(src, dst, n, splits);
-    else if (sizeof(T) > 4 || splits <= 16) simt_splitk_reduce_kernel<15><<<blocks, 256, 0, s>>>(src, dst, n, splits);
-    else simt_splitk_reduce_kernel<(sizeof(T) > 4 ? 15 : 63)><<<blocks, 256, 0, s>>>(src, dst, n, splits);
-    return cudaGetLastError();
+    auto kernel = splits <= 4 ? simt_splitk_reduce_kernel<3, T> : splits <= 8 ? simt_splitk_reduce_kernel<7, T>
+                : sizeof(T) > 4 || splits <= 16 ? simt_splitk_reduce_kernel<15, T>
+                                                : simt_splitk_reduce_kernel<(sizeof(T) > 4 ? 15 : 63), T>;
+    return launch_overlapped(kernel, dim3(blocks), 256, 0, s, 1, src, dst, n, splits);
 }
 
 // Four outputs per thread where rows of four stay 16-byte aligned in every
@@ -491,8 +494,7 @@ cudaError_t launch_cp(const SimtArgs& a, dim3 grid, cudaStream_t s) {
     static std::atomic<uint64_t> done{0};
     cudaError_t e = smem_limit_once(sgemm_simt_cp_kernel<Cf, FUSED>, Cf::SMEM, done);
     if (e != cudaSuccess) return e;
-    sgemm_simt_cp_kernel<Cf, FUSED><<<grid, Cf::THREADS, Cf::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_overlapped(sgemm_simt_cp_kernel<Cf, FUSED>, grid, Cf::THREADS, Cf::SMEM, s, 1, a);
 }
 
 template <int BM, int BN>
@@ -562,9 +564,8 @@ cudaError_t launch_grouped(const GroupProblem* probs, const GroupUnit* units, in
     cudaError_t e = smem_limit_once(sgemm_simt_grouped_kernel<Cf, FUSED>, Cf::SMEM, done);
     if (e != cudaSuccess) return e;
     const int slots = Cf::CTAS * sms;
-    sgemm_simt_grouped_kernel<Cf, FUSED><<<nunits < slots ? nunits : slots, Cf::THREADS, Cf::SMEM, s>>>(probs, units,
-                                                                                                      nunits, next);
-    return cudaGetLastError();
+    return launch_overlapped(sgemm_simt_grouped_kernel<Cf, FUSED>, dim3(nunits < slots ? nunits : slots), Cf::THREADS,
+                             Cf::SMEM, s, 1, probs, units, nunits, next);
 }
 template <int BM, int BN>
 cudaError_t launch_grouped_tile(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,

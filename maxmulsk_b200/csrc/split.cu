@@ -26,6 +26,7 @@
 #include <cstdint>
 
 #include "internal.hpp"
+#include "launch.cuh"
 #include "split_math.cuh"
 
 namespace mmsk {
@@ -40,6 +41,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256)
 split_kernel(const float* __restrict__ src, int64_t R, int64_t Cin, int64_t Cout, int64_t panel,
              void* __restrict__ planes, size_t plane_bytes) {
+    grid_wait();
     const int64_t quads_per_row = Cout / 4;
     const int64_t total = R * quads_per_row;
     const bool vec = (Cin % 4 == 0) && (((uintptr_t)src & 15) == 0);
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(256)
 split_bf16_panels_kernel(const float* __restrict__ src, int64_t R, int64_t Cin, int64_t Cout,
                          void* __restrict__ planes, size_t plane_bytes) {
     constexpr int PANEL = 64, ROWS = 64, QUADS = PANEL / 4, PER = ROWS * QUADS / 256;
+    grid_wait();
     const int64_t npan = Cout / PANEL;
     const int64_t units = npan * ((R + ROWS - 1) / ROWS);
     const bool vec = (Cin % 4 == 0) && (((uintptr_t)src & 15) == 0);
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(256)
 split_tf32_transpose_kernel(const float* __restrict__ B, int64_t K, int64_t N, int64_t Kp,
                             float* __restrict__ planes, size_t plane_bytes) {
     __shared__ float tile[32][33];
+    grid_wait();
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;     // 32 x 8
     const int64_t k0 = (int64_t)blockIdx.x * 32, n0 = (int64_t)blockIdx.y * 32;
 #pragma unroll
@@ -171,8 +175,8 @@ cudaError_t launch_tf32_transpose(const float* B, int64_t K, int64_t N, int64_t 
                                   size_t plane_bytes, cudaStream_t s) {
     if (K == 0 || N == 0) return cudaSuccess;
     dim3 grid((unsigned)((Kp + 31) / 32), (unsigned)((N + 31) / 32));
-    split_tf32_transpose_kernel<<<grid, 256, 0, s>>>(B, K, N, Kp, static_cast<float*>(planes), plane_bytes);
-    return cudaGetLastError();
+    return launch_overlapped(split_tf32_transpose_kernel, grid, 256, 0, s, 1, B, K, N, Kp, static_cast<float*>(planes),
+                             plane_bytes);
 }
 
 template <int MODE>
@@ -184,14 +188,14 @@ cudaError_t launch_one(const float* src, int64_t R, int64_t Cin, int64_t Cout, i
     if (MODE != MAXMULSK_PREC_3XTF32 && panel == 64) {
         const int64_t units = (Cout / 64) * ((R + 63) / 64);
         const int64_t blocks = units < (int64_t)sms * 8 ? units : (int64_t)sms * 8;
-        split_bf16_panels_kernel<<<(unsigned)blocks, 256, 0, s>>>(src, R, Cin, Cout, planes, plane_bytes);
-        return cudaGetLastError();
+        return launch_overlapped(split_bf16_panels_kernel, dim3((unsigned)blocks), 256, 0, s, 1, src, R, Cin, Cout, planes,
+                                 plane_bytes);
     }
     int64_t blocks = (total + 255) / 256;
     const int64_t cap = (int64_t)sms * 8;
     if (blocks > cap) blocks = cap;
-    split_kernel<MODE><<<(unsigned)blocks, 256, 0, s>>>(src, R, Cin, Cout, panel, planes, plane_bytes);
-    return cudaGetLastError();
+    return launch_overlapped(split_kernel<MODE>, dim3((unsigned)blocks), 256, 0, s, 1, src, R, Cin, Cout, panel, planes,
+                             plane_bytes);
 }
 
 }  // namespace

@@ -58,6 +58,7 @@
 #include <tuple>
 
 #include "internal.hpp"
+#include "launch.cuh"
 #include "phase.hpp"
 #include "sm100.cuh"
 #include "split_math.cuh"
@@ -446,6 +447,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
+    grid_wait();
 
     auto fail = [&]() {
         atomicOr(p.err, kErrTimeout);
@@ -539,6 +541,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
             }
         }
+        grid_release();
         // No MMA may still be running when TMEM is freed.
         tc_commit(&done_bar, leader);
         if (!mbar_wait_warp(&done_bar, 0u, p.timeout)) { atomicOr(p.err, kErrTimeout); abort_s = 1; }
@@ -641,6 +644,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     cluster_sync();                 // barriers of both CTAs initialised before any remote use
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
+    grid_wait();
 
     auto fail = [&]() {
         atomicOr(p.err, kErrTimeout);
@@ -734,6 +738,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
                 }
             }
+            grid_release();
             tc_commit_pair(&done_bar, lead);
             if (!mbar_wait_warp(&done_bar, 0u, p.timeout)) { atomicOr(p.err, kErrTimeout); abort_s = 1; }
         }
@@ -1110,6 +1115,7 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
+    grid_wait();
 
     auto fail = [&]() {
         atomicOr(err, kErrTimeout);
@@ -1201,6 +1207,7 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
                 if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
             }
         }
+        grid_release();
         // No MMA may still be running when TMEM is freed.
         tc_commit(&done_bar, leader);
         if (!mbar_wait_warp(&done_bar, 0u, timeout)) { atomicOr(err, kErrTimeout); abort_s = 1; }
@@ -1331,6 +1338,7 @@ tc_splitk_reduce_kernel(const TcParams p) {
     static_assert(E == 1 || E == 4, "columns per thread");
     constexpr int CB = 8 * E, CGROUPS = BN / CB;              // columns per block, blocks per tile row group
     __shared__ float sh[CB][33];
+    grid_wait();
     const int halves = p.bm / 128;
     const int64_t b = blockIdx.x;
     const int rg = (int)(b & 3), cg = (int)((b >> 2) % CGROUPS);
@@ -1371,11 +1379,11 @@ constexpr int kReduceAfterSplits = 3;
 template <int BN, int E>
 cudaError_t launch_reduce_e(const TcParams& prm, cudaStream_t s) {
     const unsigned blocks = (unsigned)(prm.tiles * (prm.bm / 128) * 4 * (BN / (8 * E)));
-    if (prm.main_splits <= 4) tc_splitk_reduce_kernel<BN, E, 3><<<blocks, 256, 0, s>>>(prm);
-    else if (prm.main_splits <= 8) tc_splitk_reduce_kernel<BN, E, 7><<<blocks, 256, 0, s>>>(prm);
-    else if (E > 1 || prm.main_splits <= 16) tc_splitk_reduce_kernel<BN, E, 15><<<blocks, 256, 0, s>>>(prm);
-    else tc_splitk_reduce_kernel<BN, E, 63><<<blocks, 256, 0, s>>>(prm);
-    return cudaGetLastError();
+    auto kernel = prm.main_splits <= 4 ? tc_splitk_reduce_kernel<BN, E, 3>
+                : prm.main_splits <= 8 ? tc_splitk_reduce_kernel<BN, E, 7>
+                : E > 1 || prm.main_splits <= 16 ? tc_splitk_reduce_kernel<BN, E, 15>
+                                                 : tc_splitk_reduce_kernel<BN, E, (E > 1 ? 15 : 63)>;
+    return launch_overlapped(kernel, dim3(blocks), 256, 0, s, 1, prm);
 }
 
 // 32-column blocks (whole 128-byte runs of C) when they number at least two an
@@ -1581,8 +1589,8 @@ cudaError_t launch_cfg(const TcArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     {
         PhaseScope ps(kPhaseGemm, s);
-        tc_gemm_kernel<MODE, BN><<<(unsigned)sc.grid, Cf::THREADS, Cf::SMEM, s>>>(tmA, tmB, tmC, prm);
-        e = cudaGetLastError();
+        e = launch_overlapped(tc_gemm_kernel<MODE, BN>, dim3((unsigned)sc.grid), Cf::THREADS, Cf::SMEM, s, 1, tmA, tmB, tmC,
+                              prm);
     }
     if (e != cudaSuccess || !prm.reduce_after) return e;
     PhaseScope ps(kPhaseReduce, s);
@@ -1640,22 +1648,10 @@ cudaError_t launch_cfg_pair(const TcArgs& a, cudaStream_t s) {
     static std::atomic<uint64_t> smem_set{0};
     cudaError_t e = set_smem_once(tc_gemm_pair_kernel<MODE, BN>, Cf::SMEM, smem_set);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * sc.grid), 1, 1);
-    cfg.blockDim = dim3(Cf::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cf::SMEM;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     {
         PhaseScope ps(kPhaseGemm, s);
-        e = cudaLaunchKernelEx(&cfg, tc_gemm_pair_kernel<MODE, BN>, tmA, tmB, tmC, prm);
-        if (e == cudaSuccess) e = cudaGetLastError();
+        e = launch_overlapped(tc_gemm_pair_kernel<MODE, BN>, dim3((unsigned)(2 * sc.grid)), Cf::THREADS, Cf::SMEM, s, 2, tmA,
+                              tmB, tmC, prm);
     }
     if (e != cudaSuccess || !prm.reduce_after) return e;
     PhaseScope ps(kPhaseReduce, s);
@@ -1711,8 +1707,8 @@ cudaError_t launch_fused(const TcArgs& a, cudaStream_t s) {
     TcGroupArgs none{};
     {
         PhaseScope ps(kPhaseGemm, s);
-        tc_fused_kernel<MODE, false><<<(unsigned)sc.grid, Cf::THREADS, Cf::SMEM, s>>>(tmA, tmB, tmC, prm, none);
-        e = cudaGetLastError();
+        e = launch_overlapped(tc_fused_kernel<MODE, false>, dim3((unsigned)sc.grid), Cf::THREADS, Cf::SMEM, s, 1, tmA, tmB,
+                              tmC, prm, none);
     }
     if (e != cudaSuccess || !prm.reduce_after) return e;
     PhaseScope ps(kPhaseReduce, s);
@@ -1855,17 +1851,17 @@ cudaError_t tc_grouped_launch(const TcGroupArgs& g, int precision, int grid, cud
         static std::atomic<uint64_t> smem_set{0};
         cudaError_t e = set_smem_once(tc_fused_kernel<MAXMULSK_PREC_BF16X6, true>, Cf::SMEM, smem_set);
         if (e != cudaSuccess) return e;
-        tc_fused_kernel<MAXMULSK_PREC_BF16X6, true><<<(unsigned)grid, Cf::THREADS, Cf::SMEM, s>>>(none, none, none, p, g);
+        return launch_overlapped(tc_fused_kernel<MAXMULSK_PREC_BF16X6, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1,
+                                 none, none, none, p, g);
     } else if (precision == MAXMULSK_PREC_BF16X9) {
         using Cf = CfgFused<MAXMULSK_PREC_BF16X9>;
         static std::atomic<uint64_t> smem_set{0};
         cudaError_t e = set_smem_once(tc_fused_kernel<MAXMULSK_PREC_BF16X9, true>, Cf::SMEM, smem_set);
         if (e != cudaSuccess) return e;
-        tc_fused_kernel<MAXMULSK_PREC_BF16X9, true><<<(unsigned)grid, Cf::THREADS, Cf::SMEM, s>>>(none, none, none, p, g);
-    } else {
-        return cudaErrorInvalidValue;
+        return launch_overlapped(tc_fused_kernel<MAXMULSK_PREC_BF16X9, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1,
+                                 none, none, none, p, g);
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 namespace {
