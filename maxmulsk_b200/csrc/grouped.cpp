@@ -60,10 +60,10 @@ struct maxmulsk_grouped_s {
     int sms = 0;
     // split-precision part
     void* d_tc = nullptr;                  // [problems][units][tensor maps][counters][partials]
-    mmsk::TcGroupArgs tc{};
+    mmsk::TcGroupArgs tc{}, slim{};        // units of the wide and of the slim kernel
     size_t tc_counter_bytes = 0;
     void* tc_counters = nullptr;
-    int tc_grid = 0;
+    int sms_tc = 0;
     struct Repack {                        // A copied to a 16-byte pitch before each launch
         float* dst;
         const float* src;
@@ -295,6 +295,7 @@ maxmulsk_status build_tc(maxmulsk_grouped_s* g, const maxmulsk_problem* problems
         q.kchunk = (int64_t)slice_len(p.K, sk[j]);
         q.tiles_n = (int32_t)((p.N + T - 1) / T);
         q.chunk_kb = tc_chunk_len((int64_t)p.K, q.splits) / 32;
+        q.mt = tc_slim_rows((int64_t)p.M);
         const int tm_n = (int)((p.M + T - 1) / T);
         for (int z = 0; z < q.splits; z++)
             for (int tm = 0; tm < tm_n; tm++)
@@ -303,6 +304,7 @@ maxmulsk_status build_tc(maxmulsk_grouped_s* g, const maxmulsk_problem* problems
     std::stable_sort(hu.begin(), hu.end(), [&](const TcGroupUnit& x, const TcGroupUnit& y) {
         const TcGroupProblem& a = hp[x.problem];
         const TcGroupProblem& b = hp[y.problem];
+        if ((a.mt == 0) != (b.mt == 0)) return a.mt == 0;     // the wide kernel's units, then the slim kernel's
         const int64_t la = std::min(a.kchunk, a.K - (int64_t)x.z * a.kchunk);
         const int64_t lb = std::min(b.kchunk, b.K - (int64_t)y.z * b.kchunk);
         return la > lb;
@@ -333,10 +335,13 @@ maxmulsk_status build_tc(maxmulsk_grouped_s* g, const maxmulsk_problem* problems
     g->tc.probs = reinterpret_cast<const TcGroupProblem*>(d_probs);
     g->tc.units = reinterpret_cast<const TcGroupUnit*>(d_units);
     g->tc.maps = d_maps;
-    g->tc.nunits = (int64_t)hu.size();
+    g->tc.nunits = (int64_t)std::count_if(hu.begin(), hu.end(), [&](const TcGroupUnit& u) { return hp[u.problem].mt == 0; });
     g->tc.err = device_error_word();
     g->tc.timeout = 2000000000LL;                             // about one second at B200 clocks
-    g->tc_grid = (int)std::max<int64_t>(1, std::min<int64_t>(g->tc.nunits, sms));
+    g->slim = g->tc;
+    g->slim.units += g->tc.nunits;
+    g->slim.nunits = (int64_t)hu.size() - g->tc.nunits;
+    g->sms_tc = sms;
     if (!g->tc.err) { set_error_message("device error word unavailable"); return MAXMULSK_ERR_ALLOC; }
     return MAXMULSK_OK;
 }
@@ -435,8 +440,9 @@ maxmulsk_status capture_group(maxmulsk_grouped_s* g, const maxmulsk_problem* pro
                                                r.cols * sizeof(float), r.rows, cudaMemcpyDeviceToDevice, g->cap);
             if (ec != cudaSuccess) e = ec;
         }
-        if (g->tc.nunits > 0) {
-            cudaError_t el = tc_grouped_launch(g->tc, g->plan.precision, g->tc_grid, g->cap);
+        for (const bool slim : {false, true}) {
+            const TcGroupArgs& t = slim ? g->slim : g->tc;
+            cudaError_t el = tc_grouped_launch(t, g->plan.precision, slim, (int)std::min<int64_t>(t.nunits, g->sms_tc), g->cap);
             if (el != cudaSuccess) e = el;
         }
         cudaMemsetAsync(g->d_next, 0, sizeof(unsigned), g->cap);
@@ -621,7 +627,7 @@ maxmulsk_status maxmulsk_grouped_info(maxmulsk_grouped g, maxmulsk_plan* group_p
     if (!g) return MAXMULSK_ERR_INVALID;
     if (group_plan) *group_plan = g->plan;
     if (split_k) std::memcpy(split_k, g->split_k.data(), g->count * sizeof(int32_t));
-    if (units) *units = (size_t)g->nunits + (size_t)g->tc.nunits + g->singles.size();
+    if (units) *units = (size_t)g->nunits + (size_t)(g->tc.nunits + g->slim.nunits) + g->singles.size();
     return MAXMULSK_OK;
 }
 

@@ -120,7 +120,7 @@ struct TcGroupProblem {
     int32_t tiles_n;       // tiles along N
     int32_t splits;        // K slices (1 = whole)
     int32_t chunk_kb;      // stages per TMEM accumulation chunk
-    int32_t pad;
+    int32_t mt;            // the slim kernel's rows (tc_slim_rows), 0 = the wide kernel
 };
 struct TcGroupUnit {
     int32_t problem, tm, tn, z;
@@ -137,9 +137,12 @@ struct TcGroupArgs {
 // (A: K-contiguous rows lda floats apart, B: N-contiguous rows) into
 // out[0..255]. lda and N multiples of 4, A and B 16-byte aligned.
 bool tc_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N, void* out);
+// Rows of the slim fused kernel's tile for an M-row product, or 0: the wide kernel.
+int tc_slim_rows(int64_t M);
 // Chunk length (k's per TMEM accumulation) the kernels use for K and a K split.
 int tc_chunk_len(int64_t K, int splits);
-cudaError_t tc_grouped_launch(const TcGroupArgs& g, int precision, int grid, cudaStream_t s);
+// One launch over units of problems that all run the slim kernel, or all the wide one.
+cudaError_t tc_grouped_launch(const TcGroupArgs& g, int precision, bool slim, int grid, cudaStream_t s);
 // Bytes of the partial tiles / counters of one split problem of a grouped launch.
 inline size_t tc_group_partial_floats(int64_t tiles, int splits) { return (size_t)tiles * splits * 128 * 128; }
 constexpr int kTcGroupCountersPerTile = 8;

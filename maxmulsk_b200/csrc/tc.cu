@@ -64,7 +64,6 @@
 #include "split_math.cuh"
 
 namespace mmsk {
-int tc_slots(int precision, int tile_m, int tile_n);
 
 namespace {
 
@@ -144,6 +143,7 @@ struct TcParams {
     int chunk_kb;            // stages per TMEM accumulation chunk
     int reduce_after;        // split tiles only write partials; tc_splitk_reduce_kernel sums them
     int store_c;             // whole tiles leave through the C tensor map (TMA stores)
+    int mt;                  // slim kernel: rows of the tile, a multiple of 16
     float* C;
     float* partial;          // [split tile][slice][BN columns x 128 rows], column-major, split tiles only
     unsigned* counters;      // EPI per split tile (one per epilogue warp)
@@ -217,6 +217,7 @@ struct UnitView {
     int max_splits;          // slices per split tile in the partial layout
     int chunk_kb;            // stages per TMEM accumulation chunk
     int reduce_after;        // partials are summed by tc_splitk_reduce_kernel
+    int mt;                  // slim kernel: rows of the tile, a multiple of 16
 };
 
 // Units of one GEMM (the schedule in TcParams).
@@ -232,6 +233,7 @@ struct SingleSrc {
         v.problem = 0;
         v.M = p.M; v.N = p.N; v.C = p.C; v.partial = p.partial; v.counters = p.counters;
         v.max_splits = p.max_splits; v.chunk_kb = p.chunk_kb; v.reduce_after = p.reduce_after;
+        v.mt = p.mt;
     }
     __device__ __forceinline__ const void* map_a(const UnitView&, const void* single) const { return single; }
     __device__ __forceinline__ const void* map_b(const UnitView&, const void* single) const { return single; }
@@ -899,7 +901,7 @@ struct CfgFused {
     static constexpr uint32_t TMEM_COLS = 512;
     static_assert(A_COL + OP_STAGES * A_SLOT <= TMEM_COLS, "TMEM columns");
     static constexpr int EPI = 4;                    // epilogue warps 2 .. 5, one per TMEM lane quarter
-    static constexpr int NCONV = 8;                  // converter warps 6 .. 13: four for A, four for B
+    static constexpr int NCONV = 8;                  // converter warps 6 .. 13: two sets of four
     static constexpr int THREADS = 64 + 32 * (EPI + NCONV);
     // C leaves from the TMEM sums 32 columns at a time through registers.
     static constexpr bool TMA_STORE = false;
@@ -934,6 +936,7 @@ struct GroupSrc {
         v.problem = gu.problem;
         v.M = P.M; v.N = P.N; v.C = P.C; v.partial = P.partial; v.counters = P.counters;
         v.max_splits = P.splits; v.chunk_kb = P.chunk_kb; v.reduce_after = 0;
+        v.mt = P.mt;
     }
     __device__ __forceinline__ const void* map_a(const UnitView& v, const void*) const {
         return static_cast<const char*>(g.maps) + 256 * (size_t)v.problem;
@@ -1097,8 +1100,8 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
     constexpr int CONV0 = 2 + Cf::EPI;                          // first converter warp
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < Cf::ST_STAGES; s++) { mbar_init(&st_full[s], 1); mbar_init(&st_empty[s], Cf::NCONV); }
-        for (int s = 0; s < Cf::OP_STAGES; s++) { mbar_init(&op_full[s], Cf::NCONV); mbar_init(&op_empty[s], 1); }
+        for (int s = 0; s < Cf::ST_STAGES; s++) { mbar_init(&st_full[s], 1); mbar_init(&st_empty[s], Cf::NCONV / 2); }
+        for (int s = 0; s < Cf::OP_STAGES; s++) { mbar_init(&op_full[s], Cf::NCONV / 2); mbar_init(&op_empty[s], 1); }
         for (int a = 0; a < Cf::NACC; a++) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], Cf::EPI); }
         mbar_init(&done_bar, 1);
         abort_s = 0;
@@ -1216,84 +1219,74 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
         epilogue_role_tsum<Cf>(src, err, timeout, tmem_base, tfull_bar, tempty_bar, abort_s, warp, lane);
     } else {
         // ------------------------------------------------------------ converters
-        // Warps cw = 0..3 split A rows 32q .. 32q+31 (one per lane), q = warp % 4
-        // the TMEM lane quarter the warp may write; warps 4..7 split the 32 k
-        // rows of B box cw - 4 (columns 32(cw-4) .. +31), one k row per lane:
-        // two converter warps per SM sub-partition, so one warp's memory
-        // traffic overlaps the other's arithmetic. Shared-memory accesses: a
-        // quarter-warp covers 8 consecutive rows, whose swizzled 16-byte chunks
-        // fall on distinct banks.
-        const int cwx = warp - CONV0;
-        const bool conv_a = cwx < Cf::NCONV / 2;
-        const int cw = conv_a ? cwx : cwx - Cf::NCONV / 2;
+        // Two sets of four warps cut alternate stages. A warp takes the 32 k rows
+        // of B box cw (one row a lane) and A rows 32 cw .. + 31 (one a lane), cw =
+        // the TMEM lane quarter it may write: quarter-warps cover 8 consecutive
+        // rows, whose swizzled 16-byte chunks fall on distinct banks. The staged
+        // tile is read and cut before the operand slot is waited for, so only the
+        // stores follow the MMAs that last read it. BF16x6 at 128 x 32768 x 512 /
+        // 1024^3 with the reduction 36.8 / 29.3 us when the slot was waited for
+        // first; BF16x9 42.9 / 39.8 -> 35.4 / 27.9 (with the whole-warp MMA issue),
+        // 32.8 / 27.1 without L2 prefetches. Four warps for A and four for B at
+        // every stage: 2 % slower; sixteen warps: 32.8 against 30.7.
+        const int set = (warp - CONV0) >> 2, cw = warp & 3;     // stages cut: even or odd ones; TMEM lane quarter and B box
+        int turn = 0;
         int stage = 0, ostage = 0;
         uint32_t phase = 0, ophase = 0;
+        auto advance = [&]() {
+            turn ^= 1;
+            if (++stage == Cf::ST_STAGES) { stage = 0; phase ^= 1u; }
+            if (++ostage == Cf::OP_STAGES) { ostage = 0; ophase ^= 1u; }
+        };
         bool stop = false;
         for (int64_t round = 0, u = src.unit_of(0); u < src.units() && !stop; u = src.unit_of(++round)) {
             UnitView v;
             src.get(u, v);
             const int64_t nkb = kblocks(v.w);
-            for (int64_t kb = 0; kb < nkb; kb++) {
-                // The staged tile is read and cut before the operand slot is
-                // waited for, so only the stores follow the MMAs that last read
-                // it. BF16x6 at 128 x 32768 x 512 / 1024^3 with the reduction 36.8 /
-                // 29.3 us when the slot was waited for first; BF16x9 42.9 / 39.8 ->
-                // 35.4 / 27.9 (with the whole-warp MMA issue), 32.8 / 27.1 without
-                // L2 prefetches. Sixteen converter warps: 32.8 against 30.7.
+            for (int64_t kb = 0; kb < nkb; kb++, advance()) {
+                if (turn != set) continue;
                 if (!__all_sync(0xffffffffu, !abort_s && mbar_wait_bounded(&st_full[stage], phase, timeout))) {
                     fail();
                     stop = true;
                     break;
                 }
-                const int r = conv_a ? (warp & 3) * 32 + lane : lane;     // A row (its TMEM lane), or k row of box cw
-                const uint8_t* sx = stg + (size_t)stage * Cf::ST_STAGE + (conv_a ? 0 : Cf::ST_A + cw * Cf::ST_BOX) + r * 128;
                 uint32_t l0[16], l1[16], l2[16];
-                {
+                auto cut = [&](const uint8_t* sx, int r) {
                     float x[32];
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
-                        const float4 v = *reinterpret_cast<const float4*>(sx + ((c ^ (r & 7)) << 4));
-                        x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
+                        const float4 f = *reinterpret_cast<const float4*>(sx + r * 128 + ((c ^ (r & 7)) << 4));
+                        x[4 * c] = f.x; x[4 * c + 1] = f.y; x[4 * c + 2] = f.z; x[4 * c + 3] = f.w;
                     }
 #pragma unroll
                     for (int e = 0; e < 16; e++) bf16_limbs2(x[2 * e], x[2 * e + 1], l0[e], l1[e], l2[e]);
+                };
+                const uint8_t* sa = stg + (size_t)stage * Cf::ST_STAGE;
+                cut(sa + Cf::ST_A + cw * Cf::ST_BOX, lane);
+                if (!mbar_wait_warp(&op_empty[ostage], ophase ^ 1u, timeout)) { fail(); stop = true; break; }
+                uint8_t* ob = ops + (size_t)ostage * Cf::OP_STAGE + (cw >> 1) * (Cf::BK * 128) + lane * 128;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int off = ((((cw & 1) * 4 + j) ^ (lane & 7)) << 4);
+                    *reinterpret_cast<uint4*>(ob + off) = make_uint4(l0[4 * j], l0[4 * j + 1], l0[4 * j + 2], l0[4 * j + 3]);
+                    *reinterpret_cast<uint4*>(ob + Cf::B_PLANE + off) =
+                        make_uint4(l1[4 * j], l1[4 * j + 1], l1[4 * j + 2], l1[4 * j + 3]);
+                    *reinterpret_cast<uint4*>(ob + 2 * Cf::B_PLANE + off) =
+                        make_uint4(l2[4 * j], l2[4 * j + 1], l2[4 * j + 2], l2[4 * j + 3]);
                 }
+                cut(sa, cw * 32 + lane);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&st_empty[stage]);
-                if (!mbar_wait_warp(&op_empty[ostage], ophase ^ 1u, timeout)) { fail(); stop = true; break; }
-                if (conv_a) {
-                    // Three limbs of 16 packed k pairs, in TMEM lane r at columns
-                    // A_COL + A_SLOT ostage + 16 p + pair. The MMAs that read this
-                    // slot (two stages back) are done.
-                    tc_fence_after();
-                    const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + Cf::A_COL +
-                                        (uint32_t)ostage * Cf::A_SLOT;
-                    tmem_st_32x32b_x16(ta, l0);
-                    tmem_st_32x32b_x16(ta + 16u, l1);
-                    tmem_st_32x32b_x16(ta + 32u, l2);
-                    // The limbs are in TMEM before the MMA warp is told.
-                    tmem_wait_st();
-                    tc_fence_before();
-                } else {
-                    // Four 16-byte chunks of 8 BF16 in column panel cw / 2,
-                    // chunks 4 (cw % 2) .. +3.
-                    uint8_t* ob = ops + (size_t)ostage * Cf::OP_STAGE + (cw >> 1) * (Cf::BK * 128) + r * 128;
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int off = ((((cw & 1) * 4 + j) ^ (r & 7)) << 4);
-                        *reinterpret_cast<uint4*>(ob + off) = make_uint4(l0[4 * j], l0[4 * j + 1], l0[4 * j + 2], l0[4 * j + 3]);
-                        *reinterpret_cast<uint4*>(ob + Cf::B_PLANE + off) =
-                            make_uint4(l1[4 * j], l1[4 * j + 1], l1[4 * j + 2], l1[4 * j + 3]);
-                        *reinterpret_cast<uint4*>(ob + 2 * Cf::B_PLANE + off) =
-                            make_uint4(l2[4 * j], l2[4 * j + 1], l2[4 * j + 2], l2[4 * j + 3]);
-                    }
-                    // The planes are read by the tensor cores (async proxy).
-                    fence_proxy_async();
-                }
+                tc_fence_after();
+                const uint32_t ta = tmem_base + ((uint32_t)(cw * 32) << 16) + Cf::A_COL + (uint32_t)ostage * Cf::A_SLOT;
+                tmem_st_32x32b_x16(ta, l0);
+                tmem_st_32x32b_x16(ta + 16u, l1);
+                tmem_st_32x32b_x16(ta + 32u, l2);
+                tmem_wait_st();
+                tc_fence_before();
+                fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&op_full[ostage]);
-                if (++stage == Cf::ST_STAGES) { stage = 0; phase ^= 1u; }
-                if (++ostage == Cf::OP_STAGES) { ostage = 0; ophase ^= 1u; }
             }
         }
     }
@@ -1316,6 +1309,378 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const CUtensorMap* c = p.store_c ? &tmC : nullptr;
         fused_roles<MODE>(SingleSrc{p, c}, &tmA, &tmB, c, p.err, p.timeout);
     }
+}
+
+// ============================================================================
+// Slim variant of the fused split, for products of at most 64 rows: the same
+// plan, units, products and order with the operands' places changed. The
+// 128-column tile of B (the weights) is cut into tensor memory, one column a
+// lane, and the few rows of A into K-major limb planes in shared memory, so an
+// MMA is 128 x mt x 16 with mt = the rows rounded up to 16: per 32-k stage the
+// MMAs read 12 mt x 32 bytes of shared memory instead of 48 KB, B's planes are
+// not stored there at all, and nothing is staged, cut or multiplied for rows
+// that do not exist. Bound by HBM (16 KB of B a stage and SM) where the wide
+// kernel is bound by shared memory (136 KB a stage). Measured (BF16x6 / BF16x9 in
+// graphs, inputs from HBM, the wide kernel first): 1 x 32768 x 512 29.5 / 32.6 ->
+// 24.2 / 28.2 us, 16 x 16384 x 1024 30.7 / 34.1 -> 24.9 / 29.0, 64 x 32768 x 512
+// 30.0 / 33.5 -> 28.2 / 31.2; the grouped batch of 256 GEMMs 3.86 -> 3.55 ms.
+// (64 x 512 x 4096: 12.3 -> 12.7; above 64 rows the shared memory saved is gone.)
+//
+// Converters take whole stages in turn: with every warp at a part of every
+// stage the waits set the pace (1 x 32768 x 512 29.9 us); twelve B or four A warps
+// leave the epilogue too few registers (25.6 us).
+//
+// Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue (one column
+// of C a thread), warps 6-13 cut B (a TMEM lane quarter of every other stage each),
+// warps 14-15 cut A (rows lane and lane + 32). C^T leaves the accumulators, so that
+// consecutive lanes store consecutive columns of a row of C, and K slices go to
+// the column-major partial tiles a column a thread.
+// ============================================================================
+constexpr int kSlimRows = 64;
+
+template <int MODE>
+struct CfgSlim {
+    static constexpr int BN = 128;
+    static constexpr int BK = 32, KSTEP = 16, KSTEPS = 2;
+    static constexpr int X_PLANE = kSlimRows * 64;   // one limb plane of A: rows of 32 k x 2 bytes
+    static constexpr int OP_STAGE = 3 * X_PLANE;
+    static constexpr int OP_STAGES = 4;
+    static constexpr int ST_BOX = BK * 32 * 4;       // FP32 B box: 32 k x 32 n
+    static constexpr int NBOX = BN / 32;
+    static constexpr int ST_W = NBOX * ST_BOX;
+    static constexpr int ST_STAGE = ST_W + kSlimRows * BK * 4;
+    static constexpr int ST_STAGES = 7;
+    static constexpr int NPROD = (MODE == MAXMULSK_PREC_BF16X6) ? 6 : 9;
+    static constexpr uint32_t IDESC = make_idesc(1u, 128u, 0u, 0u);   // N is set per unit
+    static constexpr int NACC = 4;                   // TMEM accumulators of up to 64 columns
+    static constexpr uint32_t W_COL = NACC * kSlimRows;
+    static constexpr uint32_t W_SLOT = 3 * BK / 2;   // 48 columns per operand stage: limb p at 16 p
+    static constexpr uint32_t TMEM_COLS = 512;
+    static_assert(W_COL + OP_STAGES * W_SLOT <= TMEM_COLS, "TMEM columns");
+    static constexpr int EPI = 4, NCONV_W = 8, NCONV = NCONV_W + 2;
+    static constexpr int THREADS = 64 + 32 * (EPI + NCONV);
+    static constexpr int SMEM = OP_STAGES * OP_STAGE + ST_STAGES * ST_STAGE + 1024;
+    static_assert(SMEM <= kSmemCap, "shared memory");
+};
+
+// One thread's column of C (rows 0 .. M - 1, M <= 64) from its sums.
+__device__ __forceinline__ void store_col_regs(const float (&sum)[kSlimRows], float* C, int64_t col, int64_t M, int64_t N) {
+    if (col >= N) return;
+#pragma unroll
+    for (int m = 0; m < kSlimRows; m++)
+        if (m < (int)M) C[(size_t)m * (size_t)N + (size_t)col] = sum[m];
+}
+
+template <int MODE, class Src>
+__device__ __forceinline__ void slim_roles(const Src& src, const void* tmA1, const void* tmB1, int* err, long long timeout) {
+    using Cf = CfgSlim<MODE>;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t st_full[Cf::ST_STAGES];
+    __shared__ __align__(8) uint64_t st_empty[Cf::ST_STAGES];
+    __shared__ __align__(8) uint64_t op_full[Cf::OP_STAGES];
+    __shared__ __align__(8) uint64_t op_empty[Cf::OP_STAGES];
+    __shared__ __align__(8) uint64_t tfull_bar[Cf::NACC];
+    __shared__ __align__(8) uint64_t tempty_bar[Cf::NACC];
+    __shared__ __align__(8) uint64_t done_bar;
+    __shared__ uint32_t tmem_base_s;
+    __shared__ volatile int abort_s;
+
+    uint8_t* ops = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* stg = ops + Cf::OP_STAGES * Cf::OP_STAGE;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // uniform to the compiler
+    const int lane = threadIdx.x & 31;
+    constexpr int CONV0 = 2 + Cf::EPI;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < Cf::ST_STAGES; s++) { mbar_init(&st_full[s], 1); mbar_init(&st_empty[s], Cf::NCONV / 2); }
+        for (int s = 0; s < Cf::OP_STAGES; s++) { mbar_init(&op_full[s], Cf::NCONV / 2); mbar_init(&op_empty[s], 1); }
+        for (int a = 0; a < Cf::NACC; a++) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], Cf::EPI); }
+        mbar_init(&done_bar, 1);
+        abort_s = 0;
+        fence_mbar_init();
+        fence_proxy_async();
+    }
+    if (warp == 0 && lane == 0 && tmA1) {
+        prefetch_tmap(tmA1);
+        prefetch_tmap(tmB1);
+    }
+    if (warp == 1) { tmem_alloc(&tmem_base_s, Cf::TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_s;
+    grid_wait();
+
+    auto fail = [&]() {
+        atomicOr(err, kErrTimeout);
+        abort_s = 1;
+    };
+    auto kblocks = [&](const Unit& w) -> int { return (int)((w.kend - w.kbeg + Cf::BK - 1) / Cf::BK); };
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ producer (FP32 tiles)
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            int64_t issued = 0;
+            for (int64_t round = 0, u = src.unit_of(0); u < src.units() && !abort_s; u = src.unit_of(++round)) {
+                UnitView v;
+                src.get(u, v);
+                const void* mapA = src.map_a(v, tmA1);
+                const void* mapB = src.map_b(v, tmB1);
+                src.acquire(mapA, mapB);
+                const int nkb = kblocks(v.w);
+                const int32_t n0 = v.w.tn * Cf::BN;
+                bool ok = true;
+                for (int kb = 0; kb < nkb; kb++) {
+                    if (!mbar_wait_bounded(&st_empty[stage], phase ^ 1u, timeout)) { fail(); ok = false; break; }
+                    if (abort_s) { ok = false; break; }
+                    uint8_t* sw = stg + (size_t)stage * Cf::ST_STAGE;
+                    mbar_arrive_expect_tx(&st_full[stage], (uint32_t)(Cf::ST_W + v.mt * Cf::BK * 4));
+                    const int32_t k = (int32_t)(v.w.kbeg + (int64_t)kb * Cf::BK);
+#pragma unroll
+                    for (int b = 0; b < Cf::NBOX; b++)
+                        tma_load_2d(sw + b * Cf::ST_BOX, mapB, &st_full[stage], n0 + 32 * b, k);
+                    tma_load_2d(sw + Cf::ST_W, mapA, &st_full[stage], k, 0);
+                    issued++;
+                    if (++stage == Cf::ST_STAGES) { stage = 0; phase ^= 1u; }
+                }
+                if (!ok) break;
+            }
+            // No copy may still be landing in shared memory when the CTA exits.
+            const int64_t first = issued > Cf::ST_STAGES ? issued - Cf::ST_STAGES : 0;
+            for (int64_t j = first; j < issued; j++) {
+                if (!mbar_wait_bounded(&st_full[j % Cf::ST_STAGES], (uint32_t)((j / Cf::ST_STAGES) & 1), timeout)) {
+                    atomicOr(err, kErrTimeout);
+                    abort_s = 1;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer (as in tc_gemm_kernel)
+        const uint32_t leader = lane == 0;
+        const uint32_t x_lo0 = smem_desc_lo(smem_u32(ops), 16u);
+        constexpr uint32_t X_HI = smem_desc_hi(512u, 4u);
+        int stage = 0;
+        uint32_t phase = 0;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        for (int64_t round = 0, u = src.unit_of(0); u < src.units() && ok && !__any_sync(0xffffffffu, abort_s);
+             u = src.unit_of(++round)) {
+            UnitView v;
+            src.get(u, v);
+            const int nkb = kblocks(v.w);
+            const uint32_t idesc = Cf::IDESC | ((uint32_t)(v.mt >> 3) << 17);
+            for (int kb0 = 0; kb0 < nkb && ok; kb0 += v.chunk_kb) {
+                if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1u, timeout)) { fail(); ok = false; break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * kSlimRows);
+                const int kb1 = min(nkb, kb0 + v.chunk_kb);
+                for (int kb = kb0; kb < kb1; kb++) {
+                    if (!mbar_wait_warp(&op_full[stage], phase, timeout)) { fail(); ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t w_tm = tmem_base + Cf::W_COL + (uint32_t)stage * Cf::W_SLOT;
+                    const uint32_t x_lo = x_lo0 + (uint32_t)(stage * (Cf::OP_STAGE >> 4));
+#pragma unroll
+                    for (int ks = 0; ks < Cf::KSTEPS; ks++) {
+#pragma unroll
+                        for (int q = 0; q < Cf::NPROD; q++) {
+                            int pa, pb;
+                            product_planes(MODE, q, pa, pb);
+                            const uint32_t wo = (uint32_t)(pb * (Cf::BK / 2) + ks * (Cf::KSTEP / 2));
+                            const uint32_t xo = (uint32_t)(pa * Cf::X_PLANE + ks * 32) >> 4;
+                            const uint32_t accum = (ks > 0 || q > 0) ? 1u : (uint32_t)(kb > kb0);
+                            mma_bf16_ta(d_tmem, w_tm + wo, x_lo + xo, X_HI, idesc, accum, leader);
+                        }
+                    }
+                    tc_commit(&op_empty[stage], leader);
+                    if (++stage == Cf::OP_STAGES) { stage = 0; phase ^= 1u; }
+                }
+                if (!ok) break;
+                tc_commit(&tfull_bar[acc], leader);
+                if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
+            }
+        }
+        grid_release();
+        // No MMA may still be running when TMEM is freed.
+        tc_commit(&done_bar, leader);
+        if (!mbar_wait_warp(&done_bar, 0u, timeout)) { atomicOr(err, kErrTimeout); abort_s = 1; }
+    } else if (warp < CONV0) {
+        // ------------------------------------------------------------ epilogue
+        // Thread: column `ncol` of the tile; its sums over the chunks, round to
+        // nearest in k order, one per row.
+        const int ew = warp - 2, ncol = (warp & 3) * 32 + lane;
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        bool stop = false;
+        for (int64_t round = 0, u = src.unit_of(0); u < src.units() && !stop; u = src.unit_of(++round)) {
+            UnitView v;
+            src.get(u, v);
+            const Unit& w = v.w;
+            const int nkb = kblocks(w);
+            float sum[kSlimRows];
+            for (int kb0 = 0; kb0 < nkb; kb0 += v.chunk_kb) {
+                if (!__all_sync(0xffffffffu, !abort_s && mbar_wait_bounded(&tfull_bar[acc], acc_phase, timeout))) {
+                    fail();
+                    stop = true;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t tacc = tmem_base + lanes + (uint32_t)(acc * kSlimRows);
+#pragma unroll
+                for (int c = 0; c < kSlimRows; c += 16) {
+                    if (c < v.mt) {
+                        uint32_t r[16];
+                        tmem_ld_32x32b_x16(tacc + (uint32_t)c, r);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            sum[c + j] = kb0 == 0 ? __uint_as_float(r[j]) : __fadd_rn(sum[c + j], __uint_as_float(r[j]));
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+                if (++acc == Cf::NACC) { acc = 0; acc_phase ^= 1u; }
+            }
+            if (stop) break;
+            const int64_t col = (int64_t)w.tn * Cf::BN + ncol;
+            if (w.sti < 0) {
+                store_col_regs(sum, v.C, col, v.M, v.N);
+                continue;
+            }
+            // Partial tiles are column-major, 128 rows a column: this thread's
+            // column is contiguous (its first mt rows written).
+            constexpr size_t TILE = (size_t)128 * Cf::BN;
+            float* seg = v.partial + (size_t)w.sti * v.max_splits * TILE + (size_t)ncol * 128;
+            float* part = seg + (size_t)w.z * TILE;
+#pragma unroll
+            for (int m = 0; m < kSlimRows; m += 4)
+                if (m < v.mt)
+                    __stcg(reinterpret_cast<float4*>(part + m), make_float4(sum[m], sum[m + 1], sum[m + 2], sum[m + 3]));
+            if (v.reduce_after) continue;
+            unsigned* ctr = v.counters + (size_t)w.sti * Cf::EPI + ew;
+            __threadfence();
+            __syncwarp();
+            int last = 0;
+            if (lane == 0) last = (atomicAdd(ctr, 1u) == (unsigned)(w.nsplit - 1));
+            last = __shfl_sync(0xffffffffu, last, 0);
+            if (!last) continue;
+            __threadfence();
+#pragma unroll
+            for (int m = 0; m < kSlimRows; m += 4) {
+                if (m < v.mt) {
+                    const float4 t = ordered_sum<7>(reinterpret_cast<const float4*>(seg + m), TILE / 4, w.nsplit);
+                    sum[m] = t.x; sum[m + 1] = t.y; sum[m + 2] = t.z; sum[m + 3] = t.w;
+                }
+            }
+            store_col_regs(sum, v.C, col, v.M, v.N);
+            if (lane == 0) *ctr = 0u;
+        }
+    } else {
+        // ------------------------------------------------------------ converters
+        const int cw = warp - CONV0;
+        const bool conv_w = cw < Cf::NCONV_W;
+        const int set = conv_w ? cw >> 2 : cw - Cf::NCONV_W;    // the stages this warp cuts: even or odd ones
+        int turn = 0;
+        int stage = 0, ostage = 0;
+        uint32_t phase = 0, ophase = 0;
+        auto advance = [&]() {
+            turn ^= 1;
+            if (++stage == Cf::ST_STAGES) { stage = 0; phase ^= 1u; }
+            if (++ostage == Cf::OP_STAGES) { ostage = 0; ophase ^= 1u; }
+        };
+        bool stop = false;
+        for (int64_t round = 0, u = src.unit_of(0); u < src.units() && !stop; u = src.unit_of(++round)) {
+            UnitView v;
+            src.get(u, v);
+            const int nkb = kblocks(v.w);
+            for (int kb = 0; kb < nkb; kb++, advance()) {
+                if (turn != set) continue;
+                if (!__all_sync(0xffffffffu, !abort_s && mbar_wait_bounded(&st_full[stage], phase, timeout))) {
+                    fail();
+                    stop = true;
+                    break;
+                }
+                const uint8_t* sw = stg + (size_t)stage * Cf::ST_STAGE;
+                if (conv_w) {
+                    // Column `lane` of box q = this warp's TMEM lane quarter: a warp
+                    // reads whole 128-byte rows.
+                    const int q = warp & 3;
+                    const uint8_t* sx = sw + q * Cf::ST_BOX + (lane & 3) * 4;
+                    uint32_t l0[16], l1[16], l2[16];
+                    {
+                        float x[32];
+#pragma unroll
+                        for (int k = 0; k < 32; k++)
+                            x[k] = *reinterpret_cast<const float*>(sx + k * 128 + (((lane >> 2) ^ (k & 7)) << 4));
+#pragma unroll
+                        for (int e = 0; e < 16; e++) bf16_limbs2(x[2 * e], x[2 * e + 1], l0[e], l1[e], l2[e]);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&st_empty[stage]);
+                    if (!mbar_wait_warp(&op_empty[ostage], ophase ^ 1u, timeout)) { fail(); stop = true; break; }
+                    tc_fence_after();
+                    const uint32_t tw = tmem_base + ((uint32_t)(q * 32) << 16) + Cf::W_COL + (uint32_t)ostage * Cf::W_SLOT;
+                    tmem_st_32x32b_x16(tw, l0);
+                    tmem_st_32x32b_x16(tw + 16u, l1);
+                    tmem_st_32x32b_x16(tw + 32u, l2);
+                    tmem_wait_st();
+                    tc_fence_before();
+                } else {
+                    // Rows lane and lane + 32 of A: 32 k's -> 64 bytes in each limb
+                    // plane, 16-byte chunk c at c ^ (row / 2 % 4) (the 64-byte
+                    // swizzle).
+                    if (!mbar_wait_warp(&op_empty[ostage], ophase ^ 1u, timeout)) { fail(); stop = true; break; }
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int r = 32 * h + lane;
+                        if (r < v.mt) {
+                            uint8_t* ox = ops + (size_t)ostage * Cf::OP_STAGE + r * 64;
+#pragma unroll
+                            for (int c = 0; c < 4; c++) {
+                                const uint8_t* sx = sw + Cf::ST_W + r * 128;
+                                const float4 f = *reinterpret_cast<const float4*>(sx + (((2 * c) ^ (r & 7)) << 4));
+                                const float4 g = *reinterpret_cast<const float4*>(sx + (((2 * c + 1) ^ (r & 7)) << 4));
+                                uint4 l0, l1, l2;
+                                bf16_limbs2(f.x, f.y, l0.x, l1.x, l2.x);
+                                bf16_limbs2(f.z, f.w, l0.y, l1.y, l2.y);
+                                bf16_limbs2(g.x, g.y, l0.z, l1.z, l2.z);
+                                bf16_limbs2(g.z, g.w, l0.w, l1.w, l2.w);
+                                uint8_t* o = ox + ((c ^ ((r >> 1) & 3)) << 4);
+                                *reinterpret_cast<uint4*>(o) = l0;
+                                *reinterpret_cast<uint4*>(o + Cf::X_PLANE) = l1;
+                                *reinterpret_cast<uint4*>(o + 2 * Cf::X_PLANE) = l2;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&st_empty[stage]);
+                    // The planes are read by the tensor cores (async proxy).
+                    fence_proxy_async();
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&op_full[ostage]);
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, Cf::TMEM_COLS);
+    }
+}
+
+template <int MODE, bool GROUPED>
+__global__ void __launch_bounds__(CfgSlim<MODE>::THREADS, 1)
+tc_slim_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p,
+               const TcGroupArgs g) {
+    if constexpr (GROUPED) slim_roles<MODE>(GroupSrc{g}, nullptr, nullptr, g.err, g.timeout);
+    else slim_roles<MODE>(SingleSrc{p}, &tmA, &tmB, p.err, p.timeout);
 }
 
 // Split-K reduction for plans that cut every tile into K slices. The GEMM
@@ -1505,6 +1870,7 @@ TcParams make_params(const TcArgs& a, const Sched& sc, int bk) {
     prm.chunk_kb = (a.chunk > 0 ? a.chunk : chunk_len(a.K, sc.main_splits)) / bk;
     prm.reduce_after = (sc.main_splits >= kReduceAfterSplits) ? 1 : 0;
     prm.store_c = 0;
+    prm.mt = 0;
     prm.C = a.C;
     prm.partial = a.partial;
     prm.counters = a.counters;
@@ -1661,17 +2027,17 @@ cudaError_t launch_cfg_pair(const TcArgs& a, cudaStream_t s) {
 // The fused-split kernel reads the FP32 operands directly: A as K x M rows of
 // 4-byte elements, B as N x K; both need rows of a multiple of 16 bytes and a
 // 16-byte aligned start (checked by the caller).
-bool encode_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N,
+// `rows`: rows of an A box (128, or the slim kernel's).
+bool encode_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N, int rows,
                        CUtensorMap* tmA, CUtensorMap* tmB) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return false;
     constexpr int BK = CfgFused<MAXMULSK_PREC_BF16X6>::BK;
-    constexpr int BM = CfgFused<MAXMULSK_PREC_BF16X6>::BM;
     const cuuint32_t estr[2] = {1, 1};
     {
         const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
         const cuuint64_t strides[1] = {(cuuint64_t)lda * 4u};
-        const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)BM};
+        const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)rows};
         if (enc(tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(A), dims, strides, box, estr,
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -1694,10 +2060,26 @@ cudaError_t launch_fused(const TcArgs& a, cudaStream_t s) {
     using Cf = CfgFused<MODE>;
     constexpr int BN = Cf::BN;
     CUtensorMap tmA, tmB;
-    if (!encode_fused_maps(a.A, a.K, a.B, a.M, a.K, a.N, &tmA, &tmB)) return cudaErrorInvalidValue;
+    const int mt = tc_slim_rows(a.M);
+    if (!encode_fused_maps(a.A, a.K, a.B, a.M, a.K, a.N, mt ? mt : 128, &tmA, &tmB)) return cudaErrorInvalidValue;
     const Sched sc = make_sched(a.M, a.K, a.N, 128, BN, a.split_k, tc_slots(a.precision, 128, BN));
     TcParams prm = make_params(a, sc, Cf::BK);
     if (sc.split_tiles > 0 && (!a.partial || !a.counters)) return cudaErrorInvalidValue;
+    if (mt) {
+        using Sl = CfgSlim<MODE>;
+        prm.mt = mt;
+        static std::atomic<uint64_t> slim_set{0};
+        cudaError_t e = set_smem_once(tc_slim_kernel<MODE, false>, Sl::SMEM, slim_set);
+        if (e != cudaSuccess) return e;
+        {
+            PhaseScope ps(kPhaseGemm, s);
+            e = launch_overlapped(tc_slim_kernel<MODE, false>, dim3((unsigned)sc.grid), Sl::THREADS, Sl::SMEM, s, 1, tmA, tmB,
+                                  prm, TcGroupArgs{});
+        }
+        if (e != cudaSuccess || !prm.reduce_after) return e;
+        PhaseScope ps(kPhaseReduce, s);
+        return launch_reduce<BN>(prm, s);
+    }
     CUtensorMap tmC;
     prm.store_c = (encode_c_map(a.C, a.M, a.N, &tmC) && Cf::TMA_STORE) ? 1 : 0;
 
@@ -1755,6 +2137,10 @@ int pair_slots_for() {
 }
 
 }  // namespace
+
+// Rows of the slim kernel's tile for an M-row fused product, or 0 for the wide
+// kernel.
+int tc_slim_rows(int64_t M) { return M <= kSlimRows ? (int)((M + 15) / 16 * 16) : 0; }
 
 // Concurrently resident work slots of a configuration on the current device:
 // the SM count for one-CTA tiles, the number of CTA pairs that fit at once
@@ -1836,31 +2222,38 @@ cudaError_t tc_launch(const TcArgs& a, cudaStream_t s) {
 
 bool tc_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N, void* out) {
     CUtensorMap* m = static_cast<CUtensorMap*>(out);
-    return encode_fused_maps(A, lda, B, M, K, N, &m[0], &m[1]);
+    const int mt = tc_slim_rows(M);
+    return encode_fused_maps(A, lda, B, M, K, N, mt ? mt : 128, &m[0], &m[1]);
 }
 
 int tc_chunk_len(int64_t K, int splits) { return chunk_len(K, splits); }
 
-cudaError_t tc_grouped_launch(const TcGroupArgs& g, int precision, int grid, cudaStream_t s) {
+namespace {
+template <int MODE>
+cudaError_t grouped_launch_mode(const TcGroupArgs& g, bool slim, int grid, cudaStream_t s) {
+    const CUtensorMap none{};
+    const TcParams p{};
+    if (slim) {
+        using Cf = CfgSlim<MODE>;
+        static std::atomic<uint64_t> smem_set{0};
+        cudaError_t e = set_smem_once(tc_slim_kernel<MODE, true>, Cf::SMEM, smem_set);
+        if (e != cudaSuccess) return e;
+        return launch_overlapped(tc_slim_kernel<MODE, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1, none, none, p, g);
+    }
+    using Cf = CfgFused<MODE>;
+    static std::atomic<uint64_t> smem_set{0};
+    cudaError_t e = set_smem_once(tc_fused_kernel<MODE, true>, Cf::SMEM, smem_set);
+    if (e != cudaSuccess) return e;
+    return launch_overlapped(tc_fused_kernel<MODE, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1, none, none, none, p,
+                             g);
+}
+}  // namespace
+
+cudaError_t tc_grouped_launch(const TcGroupArgs& g, int precision, bool slim, int grid, cudaStream_t s) {
     static_assert(sizeof(CUtensorMap) == 128, "grouped tensor-map table stride");
     if (g.nunits <= 0) return cudaSuccess;
-    CUtensorMap none{};
-    const TcParams p{};
-    if (precision == MAXMULSK_PREC_BF16X6) {
-        using Cf = CfgFused<MAXMULSK_PREC_BF16X6>;
-        static std::atomic<uint64_t> smem_set{0};
-        cudaError_t e = set_smem_once(tc_fused_kernel<MAXMULSK_PREC_BF16X6, true>, Cf::SMEM, smem_set);
-        if (e != cudaSuccess) return e;
-        return launch_overlapped(tc_fused_kernel<MAXMULSK_PREC_BF16X6, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1,
-                                 none, none, none, p, g);
-    } else if (precision == MAXMULSK_PREC_BF16X9) {
-        using Cf = CfgFused<MAXMULSK_PREC_BF16X9>;
-        static std::atomic<uint64_t> smem_set{0};
-        cudaError_t e = set_smem_once(tc_fused_kernel<MAXMULSK_PREC_BF16X9, true>, Cf::SMEM, smem_set);
-        if (e != cudaSuccess) return e;
-        return launch_overlapped(tc_fused_kernel<MAXMULSK_PREC_BF16X9, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1,
-                                 none, none, none, p, g);
-    }
+    if (precision == MAXMULSK_PREC_BF16X6) return grouped_launch_mode<MAXMULSK_PREC_BF16X6>(g, slim, grid, s);
+    if (precision == MAXMULSK_PREC_BF16X9) return grouped_launch_mode<MAXMULSK_PREC_BF16X9>(g, slim, grid, s);
     return cudaErrorInvalidValue;
 }
 

@@ -244,3 +244,23 @@ def test_fill_split_is_the_slots_per_tile_split(cuda, oracle_mod, variant, shape
     assert st0 == 0 and st1 == 0, mm.last_error_message()
     assert b0 and b1
     assert np.array_equal(bits(C0), bits(C1)), (shape, want)
+
+
+# The fused split's slim kernel (M <= 64: rows rounded up to 16, 32 and 64 cut by
+# one or two warps) and the wide one beside it, K and N edges, whole tiles, two
+# slices (summed in the kernel) and more (by the reduction): bit for bit the
+# split-inputs path.
+@pytest.mark.parametrize("prec", [mm.Precision.BF16X6, mm.Precision.BF16X9])
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33, 48, 49, 63, 64, 65])
+def test_slim_fused_equals_split_inputs(cuda, oracle_mod, prec, M):
+    for K, N, split in [(32, 4, 1), (100, 132, 1), (1028, 260, 2), (1028, 260, 5), (4100, 128, 1), (4100, 516, 0)]:
+        A, B = oracle_mod.fill_uniform(M * K, 21), oracle_mod.fill_wide(K * N, 22)
+        st, want, _ = run_plan(cuda, A, B, M, K, N, mm.make_plan(prec, 128, 128, split, mm.TC_SPLIT_INPUTS))
+        assert st == 0, mm.last_error_message()
+        for chunk in (0, 64):
+            if chunk:
+                st, want, _ = run_plan(cuda, A, B, M, K, N, mm.make_plan(prec, 128, 128, split, mm.TC_SPLIT_INPUTS, chunk))
+                assert st == 0
+            st, C, bands = run_plan(cuda, A, B, M, K, N, mm.make_plan(prec, 128, 128, split, mm.TC_FUSED_SPLIT, chunk))
+            assert st == 0 and bands, mm.last_error_message()
+            assert np.array_equal(bits(C), bits(want)), (M, K, N, split, chunk)
