@@ -239,7 +239,8 @@ typedef struct maxmulsk_grouped_s* maxmulsk_grouped;
  * group; NULL = chosen) and K split (split_k > 0 = that split for every
  * problem, 0 = chosen per problem) are what the caller gives; what is left
  * open is chosen by timing candidate configurations of the whole group (tile
- * shape x K-split policy), each captured and replayed, the fastest kept --
+ * shape, or each problem's own, x K-split policy), each captured and replayed,
+ * the fastest kept --
  * the group-level form of maxmulsk_autotune_dev. The search runs the group,
  * so C is written while the group is created.
  * A group_plan of precision MAXMULSK_PREC_BF16X6 / _BF16X9 / _SPLIT_AUTO runs
@@ -260,11 +261,12 @@ maxmulsk_status maxmulsk_grouped_launch(maxmulsk_grouped g, void* stream);
  * be NULL), number of work units. */
 maxmulsk_status maxmulsk_grouped_info(maxmulsk_grouped g, maxmulsk_plan* group_plan, int32_t* split_k,
                                       size_t* units);
-/* The plan each problem runs (count entries): FP32 problems the group's tile,
- * their K split and variant; fused problems (precision, 128, 128, K split,
- * MAXMULSK_TC_FUSED_SPLIT) -- for an A repacked to a padded pitch the result
- * is that of MAXMULSK_TC_SPLIT_INPUTS on the same tiles; problems run as their
- * own launches, their plan. Each problem's C equals a single launch of its
+/* The plan each problem runs (count entries): FP32 problems the group's tile
+ * (own tiles: the problem's, 64 x 64 standing for the 16 x 256 tile that no plan
+ * names), their K split and variant; fused problems (precision, 128, 128, K
+ * split, MAXMULSK_TC_FUSED_SPLIT) -- for an A repacked to a padded pitch the
+ * result is that of MAXMULSK_TC_SPLIT_INPUTS on the same tiles; problems run as
+ * their own launches, their plan. Each problem's C equals a single launch of its
  * plan bit for bit. */
 maxmulsk_status maxmulsk_grouped_plans(maxmulsk_grouped g, maxmulsk_plan* plans);
 void maxmulsk_grouped_destroy(maxmulsk_grouped g);

@@ -9,8 +9,9 @@
 // every GEMM is cut into (tile, K slice) units, the units are sorted heaviest
 // first, and one persistent kernel runs them:
 //   * FP32 groups: sgemm_simt_grouped_kernel (simt.cu), units taken from an
-//     atomic counter; one tile shape per group, the K split chosen per problem
-//     so that no unit is much longer than the average share of an SM;
+//     atomic counter; one tile shape per group, or each problem on the tile that
+//     suits it and a launch per tile shape; the K split chosen per problem so
+//     that no unit is much longer than the average share of an SM;
 //   * split-precision groups (BF16x6 / BF16x9): the fused-split tcgen05 kernel
 //     (tc.cu, tc_fused_kernel) over tables of problems, units and per-problem
 //     FP32 tensor maps, 128 x 128 tiles. TMA needs rows that start on 16-byte
@@ -53,8 +54,11 @@ struct maxmulsk_grouped_s {
     maxmulsk_plan simt_plan{};
     mmsk::GroupProblem* d_probs = nullptr;
     mmsk::GroupUnit* d_units = nullptr;
-    int nunits = 0;
-    unsigned* d_next = nullptr;
+    struct SimtPart {                      // units of one tile shape: one launch
+        int bm, bn, first, count;
+    };
+    std::vector<SimtPart> simt_parts;
+    unsigned* d_next = nullptr;            // a unit counter per part
     void* d_scratch = nullptr;             // [counters of all split problems][partials]
     size_t counter_bytes = 0;
     int sms = 0;
@@ -91,12 +95,19 @@ namespace {
 
 inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Relative throughput of the SIMT tile shapes (measured at 4096^3: 58, 54 and
-// 51 TFLOP/s for 128x128, 128x64, 64x64).
+// Tile shapes of the FP32 kernel and their relative throughput per padded
+// multiply-add (measured: 58, 54 and 51 TFLOP/s at 4096^3 for the three that
+// plans name; 16 x 256, for the few-row problems of a group: 33).
+struct SimtTile {
+    int bm, bn;
+    double rate;
+    int ctas;                              // resident CTAs an SM
+};
+constexpr SimtTile kSimtTiles[4] = {{128, 128, 1.0, 2}, {128, 64, 0.93, 2}, {64, 64, 0.87, 4}, {16, 256, 0.6, 2}};
 double tile_rate(int bm, int bn) {
-    if (bm == 128 && bn == 128) return 1.0;
-    if (bm == 128 && bn == 64) return 0.93;
-    return 0.87;
+    for (const SimtTile& t : kSimtTiles)
+        if (t.bm == bm && t.bn == bn) return t.rate;
+    return 1.0;
 }
 
 // Padded work of a problem on a tile shape, in multiply-adds.
@@ -118,13 +129,25 @@ void pick_tile(const maxmulsk_problem* probs, const std::vector<size_t>& idx, in
     }
 }
 
-// K split of each problem: units no longer than 1/share of a work slot's
-// average share of the group, slices at least 256 deep, at most 64 slices.
-// fixed > 0 imposes that split on every problem; share <= 0 splits none.
-std::vector<int> plan_splits(const maxmulsk_problem* probs, const std::vector<size_t>& idx, int bm, int bn,
-                             int slots, int fixed, double share) {
+// The tile shape with the least estimated time for one problem.
+SimtTile own_tile(const maxmulsk_problem& p) {
+    SimtTile best = kSimtTiles[0];
+    double t = -1;
+    for (const SimtTile& c : kSimtTiles) {
+        const double v = padded_work(p, c.bm, c.bn) / c.rate;
+        if (t < 0 || v < t) { t = v; best = c; }
+    }
+    return best;
+}
+
+// K split of each problem (problem idx[j] on tiles[j]): units no longer than
+// 1/share of a work slot's average share of the group, slices at least 256 deep,
+// at most 64 slices. fixed > 0 imposes that split on every problem; share <= 0
+// splits none.
+std::vector<int> plan_splits(const maxmulsk_problem* probs, const std::vector<size_t>& idx,
+                             const std::vector<SimtTile>& tiles, int slots, int fixed, double share) {
     double total = 0;
-    for (size_t i : idx) total += padded_work(probs[i], bm, bn);
+    for (size_t j = 0; j < idx.size(); j++) total += padded_work(probs[idx[j]], tiles[j].bm, tiles[j].bn);
     if (fixed <= 0 && share <= 0) return std::vector<int>(idx.size(), 1);
     const double cap = std::max(1.0, total / (share * slots));
     std::vector<int> out(idx.size(), 1);
@@ -135,7 +158,7 @@ std::vector<int> plan_splits(const maxmulsk_problem* probs, const std::vector<si
         if (fixed > 0) {
             s = fixed;
         } else {
-            const double unit = (double)bm * bn * (double)p.K;
+            const double unit = (double)tiles[j].bm * tiles[j].bn * (double)p.K;
             s = (int)std::min<double>(64.0, std::ceil(unit / cap));
             const int kmax = (int)std::max<size_t>(1, p.K / 256);
             s = std::max(1, std::min(s, kmax));
@@ -145,16 +168,32 @@ std::vector<int> plan_splits(const maxmulsk_problem* probs, const std::vector<si
     return out;
 }
 
-// FP32 part: the problems `idx` on the SIMT grouped kernel.
+// FP32 part: the problems `idx` on the SIMT grouped kernel, on the plan's tile
+// or (`mixed`) each on its own tile, one launch per tile shape.
 maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* problems, const std::vector<size_t>& idx,
-                           const maxmulsk_plan& plan, double share, int sms) {
-    const int bm = plan.tile_m, bn = plan.tile_n;
-    const std::vector<int> sk = plan_splits(problems, idx, bm, bn, 2 * sms, plan.split_k, share);   // 2 CTAs per SM
+                           const maxmulsk_plan& plan, bool mixed, double share, int sms) {
+    std::vector<SimtTile> tiles(idx.size(), SimtTile{plan.tile_m, plan.tile_n, 1.0, 2});
+    if (mixed)
+        for (size_t j = 0; j < idx.size(); j++) tiles[j] = own_tile(problems[idx[j]]);
+    std::vector<int> sk = plan_splits(problems, idx, tiles, 2 * sms, plan.split_k, share);   // 2 CTAs per SM
+    if (mixed) {
+        // Each tile shape is a launch of its own and has to balance by itself.
+        for (const SimtTile& t : kSimtTiles) {
+            std::vector<size_t> at, sub;
+            for (size_t j = 0; j < idx.size(); j++)
+                if (tiles[j].bm == t.bm && tiles[j].bn == t.bn) { at.push_back(j); sub.push_back(idx[j]); }
+            const std::vector<int> own = plan_splits(problems, sub, std::vector<SimtTile>(sub.size(), t), t.ctas * sms,
+                                                     plan.split_k, share);
+            for (size_t i = 0; i < at.size(); i++) sk[at[i]] = own[i];
+        }
+    }
     for (size_t j = 0; j < idx.size(); j++) {
         g->split_k[idx[j]] = sk[j];
         maxmulsk_plan& q = g->plans[idx[j]];
         q = plan;
         q.split_k = sk[j];
+        // A plan names 128 x 128, 128 x 64 or 64 x 64; C is the same on any tile.
+        if (tiles[j].bm >= 64) { q.tile_m = tiles[j].bm; q.tile_n = tiles[j].bn; }
     }
 
     std::vector<GroupProblem> hp(idx.size());
@@ -164,10 +203,10 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
     for (size_t j = 0; j < idx.size(); j++) {
         const maxmulsk_problem& p = problems[idx[j]];
         const int splits = (p.K ? slice_count(p.K, sk[j]) : 1);
-        const size_t tiles = (size_t)((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn);
+        const int bm = tiles[j].bm, bn = tiles[j].bn;
         if (splits > 1) {
             ctr_off[j] = counters;
-            counters += tiles * sizeof(unsigned);
+            counters += (size_t)((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn) * sizeof(unsigned);
             part_off[j] = partials;
             partials += align256((size_t)splits * p.M * p.N * sizeof(float));
         }
@@ -181,6 +220,7 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
     for (size_t j = 0; j < idx.size(); j++) {
         const maxmulsk_problem& p = problems[idx[j]];
         GroupProblem& q = hp[j];
+        const int bm = tiles[j].bm, bn = tiles[j].bn;
         std::memset(&q, 0, sizeof q);
         q.a.A = p.A; q.a.B = p.B; q.a.C = p.C;
         q.a.M = (int64_t)p.M; q.a.K = (int64_t)p.K; q.a.N = (int64_t)p.N;
@@ -198,20 +238,29 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
             for (int tm = 0; tm < tm_n; tm++)
                 for (int tn = 0; tn < tn_n; tn++) hu.push_back(GroupUnit{(int32_t)j, tm, tn, z});
     }
-    // Heaviest units first (K slice length), stable so slices stay grouped.
+    // By tile shape, largest first; then heaviest units first (K slice length),
+    // stable so slices stay grouped.
     std::stable_sort(hu.begin(), hu.end(), [&](const GroupUnit& x, const GroupUnit& y) {
+        const SimtTile &tx = tiles[x.problem], &ty = tiles[y.problem];
+        if (tx.bm != ty.bm) return tx.bm > ty.bm;
+        if (tx.bn != ty.bn) return tx.bn > ty.bn;
         const GroupProblem& a = hp[x.problem];
         const GroupProblem& b = hp[y.problem];
         const int64_t la = std::min(a.a.kchunk, a.a.K - (int64_t)x.z * a.a.kchunk);
         const int64_t lb = std::min(b.a.kchunk, b.a.K - (int64_t)y.z * b.a.kchunk);
         return la > lb;
     });
-    g->nunits = (int)hu.size();
+    for (size_t i = 0; i < hu.size(); i++) {
+        const SimtTile& t = tiles[hu[i].problem];
+        if (g->simt_parts.empty() || g->simt_parts.back().bm != t.bm || g->simt_parts.back().bn != t.bn)
+            g->simt_parts.push_back({t.bm, t.bn, (int)i, 0});
+        g->simt_parts.back().count++;
+    }
     g->sms = sms;
     cudaError_t e;
     if ((e = cudaMalloc(&g->d_probs, std::max<size_t>(1, idx.size()) * sizeof(GroupProblem))) != cudaSuccess ||
         (e = cudaMalloc(&g->d_units, std::max<size_t>(1, hu.size()) * sizeof(GroupUnit))) != cudaSuccess ||
-        (e = cudaMalloc(&g->d_next, sizeof(unsigned))) != cudaSuccess)
+        (e = cudaMalloc(&g->d_next, std::max<size_t>(1, g->simt_parts.size()) * sizeof(unsigned))) != cudaSuccess)
         return cuda_status(e, "cudaMalloc(grouped tables)");
     if (!idx.empty() && (e = cudaMemcpy(g->d_probs, hp.data(), idx.size() * sizeof(GroupProblem),
                                         cudaMemcpyHostToDevice)) != cudaSuccess)
@@ -227,7 +276,8 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
 maxmulsk_status build_tc(maxmulsk_grouped_s* g, const maxmulsk_problem* problems, const std::vector<size_t>& idx,
                          int precision, int fixed_split, double share, int sms) {
     constexpr int T = 128;                                    // tile rows and columns
-    const std::vector<int> sk = plan_splits(problems, idx, T, T, sms, fixed_split, share);   // 1 CTA per SM
+    const std::vector<SimtTile> tiles(idx.size(), SimtTile{T, T, 1.0, 1});
+    const std::vector<int> sk = plan_splits(problems, idx, tiles, sms, fixed_split, share);   // 1 CTA per SM
     const size_t n = idx.size();
     for (size_t j = 0; j < n; j++) {
         maxmulsk_plan& q = g->plans[idx[j]];
@@ -243,12 +293,12 @@ maxmulsk_status build_tc(maxmulsk_grouped_s* g, const maxmulsk_problem* problems
         const maxmulsk_problem& p = problems[idx[j]];
         g->split_k[idx[j]] = sk[j];
         const int splits = slice_count(p.K, sk[j]);
-        const int64_t tiles = (int64_t)((p.M + T - 1) / T) * (int64_t)((p.N + T - 1) / T);
+        const int64_t ntiles = (int64_t)((p.M + T - 1) / T) * (int64_t)((p.N + T - 1) / T);
         if (splits > 1) {
             ctr_off[j] = counters;
-            counters += (size_t)tiles * kTcGroupCountersPerTile * sizeof(unsigned);
+            counters += (size_t)ntiles * kTcGroupCountersPerTile * sizeof(unsigned);
             part_off[j] = partials;
-            partials += align256(tc_group_partial_floats(tiles, splits) * sizeof(float));
+            partials += align256(tc_group_partial_floats(ntiles, splits) * sizeof(float));
         }
     }
     // A operands that TMA cannot read in place: one zero-padded buffer, rows
@@ -355,6 +405,7 @@ bool fused_readable(const maxmulsk_problem& p) {
 struct GroupConfig {
     maxmulsk_plan simt{};          // FP32 part: tile, variant; split_k > 0 = that split for all
     double simt_share = 4.0;       // FP32 K-split policy (plan_splits) when split_k == 0
+    bool simt_mixed = false;       // each FP32 problem on its own tile
     int tc_precision = 0;          // 0: FP32 group; else BF16X6 / BF16X9 (the fused kernel)
     int tc_request = 0;            // the precision asked for (SPLIT_AUTO lets singles pick 3xTF32)
     int tc_fixed = 0;              // > 0: that split for every fused problem
@@ -403,7 +454,7 @@ maxmulsk_status build_group(maxmulsk_grouped_s* g, const maxmulsk_problem* probl
     } else {
         g->plan = cfg.simt;
     }
-    maxmulsk_status st = build_simt(g, problems, simt_idx, cfg.simt, cfg.simt_share, sms);
+    maxmulsk_status st = build_simt(g, problems, simt_idx, cfg.simt, cfg.simt_mixed, cfg.simt_share, sms);
     if (st == MAXMULSK_OK && !tc_idx.empty())
         st = build_tc(g, problems, tc_idx, cfg.tc_precision, cfg.tc_fixed, cfg.tc_share, sms);
     if (st != MAXMULSK_OK) return st;
@@ -445,11 +496,14 @@ maxmulsk_status capture_group(maxmulsk_grouped_s* g, const maxmulsk_problem* pro
             cudaError_t el = tc_grouped_launch(t, g->plan.precision, slim, (int)std::min<int64_t>(t.nunits, g->sms_tc), g->cap);
             if (el != cudaSuccess) e = el;
         }
-        cudaMemsetAsync(g->d_next, 0, sizeof(unsigned), g->cap);
+        if (!g->simt_parts.empty()) cudaMemsetAsync(g->d_next, 0, g->simt_parts.size() * sizeof(unsigned), g->cap);
         if (g->d_scratch && g->counter_bytes) cudaMemsetAsync(g->d_scratch, 0, g->counter_bytes, g->cap);
-        if (g->nunits > 0)
-            simt_grouped_launch(g->d_probs, g->d_units, g->nunits, g->d_next, g->simt_plan.tile_m,
-                                g->simt_plan.tile_n, g->simt_plan.variant, g->sms, g->cap);
+        for (size_t i = 0; i < g->simt_parts.size(); i++) {
+            const auto& t = g->simt_parts[i];
+            cudaError_t el = simt_grouped_launch(g->d_probs, g->d_units + t.first, t.count, g->d_next + i, t.bm, t.bn,
+                                                 g->simt_plan.variant, g->sms, g->cap);
+            if (el != cudaSuccess) e = el;
+        }
         for (const auto& sg : g->singles) {
             const maxmulsk_problem& p = problems[sg.problem];
             maxmulsk_status s1 = run_plan_dev(p.A, p.B, p.C, p.M, p.K, p.N, sg.plan, g->d_single_ws,
@@ -491,14 +545,16 @@ float time_group(maxmulsk_grouped_s* g) {
 // The candidates searched when the caller leaves the cut to the library.
 std::vector<GroupConfig> candidate_configs(const GroupConfig& base, bool search_tile, bool search_simt,
                                            bool search_tc) {
-    const int tiles[3][2] = {{128, 128}, {128, 64}, {64, 64}};
+    // Tile choices: every problem on its own tile, or one tile for the group (a
+    // batch of 128 uneven GEMMs: 3.61 ms on own tiles, 4.37 on 64 x 64).
+    const int tiles[3][2] = {{64, 64}, {128, 128}, {64, 64}};
     const double shares[4] = {0.0, 2.0, 4.0, 8.0};            // 0: no K split
     std::vector<GroupConfig> simt_opts;
     if (search_simt) {
         for (int t = 0; t < (search_tile ? 3 : 1); t++)
             for (double sh : shares) {
                 GroupConfig c = base;
-                if (search_tile) { c.simt.tile_m = tiles[t][0]; c.simt.tile_n = tiles[t][1]; }
+                if (search_tile) { c.simt.tile_m = tiles[t][0]; c.simt.tile_n = tiles[t][1]; c.simt_mixed = t == 0; }
                 c.simt_share = sh;
                 simt_opts.push_back(c);
             }
@@ -627,7 +683,9 @@ maxmulsk_status maxmulsk_grouped_info(maxmulsk_grouped g, maxmulsk_plan* group_p
     if (!g) return MAXMULSK_ERR_INVALID;
     if (group_plan) *group_plan = g->plan;
     if (split_k) std::memcpy(split_k, g->split_k.data(), g->count * sizeof(int32_t));
-    if (units) *units = (size_t)g->nunits + (size_t)(g->tc.nunits + g->slim.nunits) + g->singles.size();
+    size_t simt_units = 0;
+    for (const auto& t : g->simt_parts) simt_units += (size_t)t.count;
+    if (units) *units = simt_units + (size_t)(g->tc.nunits + g->slim.nunits) + g->singles.size();
     return MAXMULSK_OK;
 }
 

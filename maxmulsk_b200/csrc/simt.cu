@@ -159,10 +159,11 @@ __device__ __forceinline__ void simt_epilogue(const SimtArgs& p, float (&acc)[TM
 // Arithmetic: every output is one chain over k in increasing order, so C is
 // the same bit for bit whatever the tile; copies past kend write zeros.
 // ---------------------------------------------------------------------------
-template <int BM_, int BN_, int RT_, int LT_, int BK_, int STAGES_, int CTAS_>
+template <int BM_, int BN_, int RT_, int LT_, int BK_, int STAGES_, int CTAS_, int LM_ = 8>
 struct CpCfg {
     static constexpr int BM = BM_, BN = BN_, RT = RT_, LT = LT_, BK = BK_, STAGES = STAGES_, CTAS = CTAS_;
-    static constexpr int WM = 8 * RT, WN = 4 * LT;  // warp tile
+    static constexpr int LM = LM_, LN = 32 / LM;    // lanes along M and N
+    static constexpr int WM = LM * RT, WN = LN * LT;  // warp tile
     static constexpr int WARPS_N = BN / WN;
     static constexpr int THREADS = 32 * (BM / WM) * WARPS_N;
     static constexpr int AST = BK + 4;             // A row stride (floats): eight rows on eight bank groups
@@ -170,7 +171,7 @@ struct CpCfg {
     static constexpr int B_FLOATS = BK * BN;
     static constexpr int STAGE_FLOATS = A_FLOATS + B_FLOATS;
     static constexpr int SMEM = STAGES * STAGE_FLOATS * 4;
-    static_assert(THREADS >= BN && THREADS >= BK && BK % 2 == 0 && STAGES >= 3, "tile configuration");
+    static_assert(THREADS >= BK && BK % 2 == 0 && STAGES >= 3 && THREADS <= 4 * BN, "tile configuration");
 };
 
 // The plans' tiles. 128 x 128: 8 x 16 outputs a thread (255 registers, two
@@ -183,6 +184,11 @@ template <int BM, int BN> struct CpTileSel;
 template <> struct CpTileSel<128, 128> { using T = CpCfg<128, 128, 8, 16, 16, 4, 2>; };
 template <> struct CpTileSel<128, 64> { using T = CpCfg<128, 64, 8, 8, 32, 3, 2>; };
 template <> struct CpTileSel<64, 64> { using T = CpCfg<64, 64, 4, 8, 32, 3, 4>; };
+// Grouped launches only, for problems of few rows: 4 x 8 outputs a thread over
+// four by eight lanes, so a warp's B reads are whole 128-byte rows (the 74
+// problems of at most 32 rows of a 128-GEMM batch, 2.3 GB of B: 0.54 ms; BK 16 x
+// 4 stages and four CTAs an SM, or 16 x 128 tiles of 2 x 8 a thread, 0.93).
+template <> struct CpTileSel<16, 256> { using T = CpCfg<16, 256, 4, 8, 32, 3, 2, 4>; };
 template <int BM, int BN> using CpTile = typename CpTileSel<BM, BN>::T;
 
 // Two FP32 lanes in a 64-bit register: the packed arithmetic of sm_100
@@ -245,7 +251,7 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
     constexpr int GN = LT / 4;                 // float4 groups per thread row
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = warp / Cf::WARPS_N, wn = warp % Cf::WARPS_N;
-    const int lm = lane >> 2, ln = lane & 3;
+    const int lm = lane / Cf::LN, ln = lane % Cf::LN;
     const int64_t M = p.M, N = p.N, K = p.K;
     const int64_t kbeg = (int64_t)z * p.kchunk;
     const int64_t kend = min(K, kbeg + p.kchunk);
@@ -276,18 +282,31 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
         }
     };
     auto load_b_stage = [&]<int W, bool EDGE>(uint32_t b_s, int64_t k0) {
-        constexpr int CPR = BN / W, RPP = THREADS / CPR;
-        const int row = tid / CPR, col = tid % CPR * W;
-        const float* src = B + (k0 + row) * N + n0 + col;
-        const uint32_t dst = b_s + (uint32_t)(row * BN + col) * 4u;
-        const int64_t step = (int64_t)RPP * N;
+        if constexpr (BN / W > THREADS) {                           // several copies of one row per thread
+            for (int j = 0; j < BK; j++) {
+                const float* src = B + (k0 + j) * N + n0;
+#pragma unroll
+                for (int col = 0; col < BN / W; col += THREADS) {
+                    const int c = (col + tid) * W;
+                    const bool ok = !EDGE || (k0 + j < kend && n0 + c < N);
+                    cp_async<W>(b_s + (uint32_t)(j * BN + c) * 4u, ok ? src + c : B, ok ? 4 * W : 0);
+                }
+            }
+            return;
+        } else {
+            constexpr int CPR = BN / W, RPP = THREADS / CPR;
+            const int row = tid / CPR, col = tid % CPR * W;
+            const float* src = B + (k0 + row) * N + n0 + col;
+            const uint32_t dst = b_s + (uint32_t)(row * BN + col) * 4u;
+            const int64_t step = (int64_t)RPP * N;
 #pragma unroll(W == 1 ? 8 : 16)
-        for (int j = 0; j < BK / RPP; j++, src += step) {
-            if constexpr (EDGE) {
-                const bool ok = k0 + row + j * RPP < kend && n0 + col < N;
-                cp_async<W>(dst + (uint32_t)(j * RPP * BN * 4), ok ? src : B, ok ? 4 * W : 0);
-            } else {
-                cp_async<W>(dst + (uint32_t)(j * RPP * BN * 4), src);
+            for (int j = 0; j < BK / RPP; j++, src += step) {
+                if constexpr (EDGE) {
+                    const bool ok = k0 + row + j * RPP < kend && n0 + col < N;
+                    cp_async<W>(dst + (uint32_t)(j * RPP * BN * 4), ok ? src : B, ok ? 4 * W : 0);
+                } else {
+                    cp_async<W>(dst + (uint32_t)(j * RPP * BN * 4), src);
+                }
             }
         }
     };
@@ -323,12 +342,12 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
     const int a_off = (wm * Cf::WM + lm) * AST, b_off = Cf::A_FLOATS + wn * Cf::WN + ln * 4;
     auto load_a = [&](int set, const float* st, int k) {
 #pragma unroll
-        for (int i = 0; i < RT; i++) fa[set][i] = *reinterpret_cast<const float2*>(st + a_off + i * 8 * AST + k);
+        for (int i = 0; i < RT; i++) fa[set][i] = *reinterpret_cast<const float2*>(st + a_off + i * Cf::LM * AST + k);
     };
     auto load_b = [&](int set, const float* st, int k) {
 #pragma unroll
         for (int j = 0; j < GN; j++) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(st + b_off + k * BN + j * 16);
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(st + b_off + k * BN + j * 4 * Cf::LN);
             fb[set][2 * j] = v.x;
             fb[set][2 * j + 1] = v.y;
         }
@@ -392,8 +411,8 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
     for (int i = 0; i < RT; i++)
 #pragma unroll
         for (int j = 0; j < LT / 2; j++) unpack2(acc[i][j], out[i][2 * j], out[i][2 * j + 1]);
-    auto out_row = [&](int i) { return m0 + wm * Cf::WM + lm + 8 * i; };
-    auto out_col = [&](int g) { return n0 + wn * Cf::WN + ln * 4 + 16 * g; };
+    auto out_row = [&](int i) { return m0 + wm * Cf::WM + lm + Cf::LM * i; };
+    auto out_col = [&](int g) { return n0 + wn * Cf::WN + ln * 4 + 4 * Cf::LN * g; };
     simt_epilogue<RT, GN>(p, out, out_row, out_col, p.wc == 4, z, tile, last_flag);
 }
 
@@ -581,6 +600,7 @@ cudaError_t simt_grouped_launch(const GroupProblem* probs, const GroupUnit* unit
     if (tile_m == 128 && tile_n == 128) return launch_grouped_tile<128, 128>(probs, units, nunits, next, variant, sms, s);
     if (tile_m == 128 && tile_n == 64) return launch_grouped_tile<128, 64>(probs, units, nunits, next, variant, sms, s);
     if (tile_m == 64 && tile_n == 64) return launch_grouped_tile<64, 64>(probs, units, nunits, next, variant, sms, s);
+    if (tile_m == 16 && tile_n == 256) return launch_grouped_tile<16, 256>(probs, units, nunits, next, variant, sms, s);
     return cudaErrorInvalidValue;
 }
 

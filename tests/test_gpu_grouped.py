@@ -8,7 +8,7 @@ import pytest
 
 import maxmulsk_b200 as mm
 from maxmulsk_b200 import workloads
-from gpu_util import run_plan
+from gpu_util import bits, run_plan, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -219,3 +219,34 @@ def test_grouped_split_precision_big_problems_run_their_own_plans(cuda, oracle_m
     g2, _, _, _ = _group(cuda, oracle_mod, shapes, 900, mm.make_plan(mm.Precision.BF16X6, 128, 128, 3))
     assert all(p.variant == mm.TC_FUSED_SPLIT and p.split_k == 3 for p in g2.plans())
     g2.close()
+
+
+def test_few_row_problems_run_on_their_own_tiles(cuda, oracle_mod):
+    # With no plan given and only problems of few rows, the 16 x 256 tile does a
+    # fraction of the 64 x 64 tile's work, so the search keeps "own tiles": the
+    # units are 16 x 256 tiles times slices, and each C is the oracle's for the
+    # reported K split bit for bit, over rows, columns and row lengths that fit
+    # the tile and its copies or not.
+    torch = cuda
+    shapes = [(m, k, n) for m in (1, 3, 15, 16, 17, 32) for k, n in ((640, 512), (641, 513), (642, 514), (2048, 1024))]
+    shapes += [(m, k, n) for m in (1, 9, 16) for k, n in ((1, 257), (640, 260), (97, 259))]
+    shapes += [(16, 4096, 2048)] * 24
+    A = [oracle_mod.fill_uniform(m * k, 3 + i) for i, (m, k, n) in enumerate(shapes)]
+    B = [oracle_mod.fill_uniform(k * n, 90 + i) for i, (m, k, n) in enumerate(shapes)]
+    dA, dB = [to_dev(torch, a) for a in A], [to_dev(torch, b) for b in B]
+    dC = [torch.full((m * n,), float("nan"), device="cuda") for m, k, n in shapes]
+    g = mm.Grouped([(a, b, c, *s) for a, b, c, s in zip(dA, dB, dC, shapes)])
+    try:
+        plans = g.plans()
+        units = sum(-(-m // 16) * -(-n // 256) * mm.slice_count(k, p.split_k) for (m, k, n), p in zip(shapes, plans))
+        assert g.info()[2] == units
+        for c in dC:
+            c.fill_(float("nan"))
+        torch.cuda.synchronize()
+        assert g.launch() == 0
+        torch.cuda.synchronize()
+        for a, b, c, (m, k, n), p in list(zip(A, B, dC, shapes, plans))[:34]:
+            want = oracle_mod.sgemm_panels(a, b, m, k, n, kc=mm.slice_len(k, p.split_k), fma=True)
+            assert np.array_equal(bits(c.cpu().numpy().reshape(m, n)), bits(want)), (m, k, n, p)
+    finally:
+        g.close()
