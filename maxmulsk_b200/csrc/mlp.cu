@@ -340,7 +340,7 @@ inline unsigned blocks(int n) { return (unsigned)((n + 255) / 256); }
 // ----------------------------------------------------------------- host model
 struct Model {
     bool loaded = false;
-    std::vector<float> w;                     // NPARAM
+    std::vector<float> w;                     // NPARAM, or 2 NPARAM: the FP32 class's, then the split class's
 };
 std::mutex g_model_mu;
 Model g_model;
@@ -400,6 +400,10 @@ bool load_file(const char* path, std::vector<float>& w) {
     if (ok) {
         w.resize(NPARAM);
         ok = std::fread(w.data(), sizeof(float), NPARAM, f) == (size_t)NPARAM;
+        // Weights of the split class's own, if they follow whole.
+        std::vector<float> split(NPARAM);
+        if (ok && std::fread(split.data(), sizeof(float), NPARAM, f) == (size_t)NPARAM)
+            w.insert(w.end(), split.begin(), split.end());
     }
     std::fclose(f);
     return ok;
@@ -455,7 +459,7 @@ bool mlp_predict_host(size_t M, size_t K, size_t N, int cls, float* y) {
     if (!g_model.loaded) return false;
     float x[F];
     mlp_features(M, K, N, cls, x);
-    host_forward(g_model.w.data(), x, y);
+    host_forward(g_model.w.data() + (cls == 1 && g_model.w.size() > (size_t)NPARAM ? NPARAM : 0), x, y);
     return true;
 }
 

@@ -266,3 +266,30 @@ def test_picks_follow_the_loaded_model(built_lib, tmp_path, monkeypatch):
     finally:
         _load_shipped_model()
     assert picks(shapes) == first
+
+
+def test_model_file_with_split_weights(built_lib, tmp_path):
+    # Weights for the split class beside the FP32 class's: each class predicts
+    # with its own; a file with one set serves both, as does one whose second set
+    # is cut short.
+    rng = np.random.default_rng(1)
+    p, q = (rng.normal(0, 0.3, picker.NPARAM).astype(np.float32) for _ in range(2))
+    out = (ctypes.c_float * 48)()
+
+    def predict(path, cls):
+        assert mm.lib().maxmulsk_model_load(str(path).encode()) == 0
+        assert mm.lib().maxmulsk_mlp_predict_host(300, 700, 260, cls, out) == 0
+        return np.array(out)
+
+    one_p, one_q, two, cut = (tmp_path / n for n in ("p.bin", "q.bin", "two.bin", "cut.bin"))
+    picker.save_params(one_p, p)
+    picker.save_params(one_q, q)
+    picker.save_params(two, p, q)
+    cut.write_bytes(two.read_bytes()[:-4])
+    try:
+        assert np.array_equal(predict(two, 0), predict(one_p, 0))
+        assert np.array_equal(predict(two, 1), predict(one_q, 1))
+        assert np.array_equal(predict(cut, 1), predict(one_p, 1))
+        assert np.array_equal(picker.load_params(two), p)
+    finally:
+        _load_shipped_model()
