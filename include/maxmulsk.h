@@ -314,7 +314,8 @@ int32_t maxmulsk_tuning_save(const char* path);   /* entries written, or -1 */
 void maxmulsk_tuning_clear(void);
 
 /* Learned cost model: load weights (MAXMULSK_MODEL is read on first use);
- * NULL unloads. */
+ * NULL unloads. A file holds one set of weights for both plan classes, or two:
+ * the FP32 class's, then the split class's. */
 maxmulsk_status maxmulsk_model_load(const char* path);
 /* The model's features of a shape, and its predicted log-times on the host. */
 maxmulsk_status maxmulsk_mlp_features(size_t M, size_t K, size_t N, int32_t cls, float* out);

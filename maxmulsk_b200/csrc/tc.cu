@@ -1717,8 +1717,9 @@ tc_splitk_reduce_kernel(const TcParams p) {
     if (row0 >= p.M || col0 >= p.N) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* src = p.partial + (size_t)th * p.max_splits * TILE + (size_t)(cg * CB + warp) * 128 + rg * 32 + lane;
-    // Rows past M and columns past N are read too: every slice wrote its whole
-    // tile; they are not stored.
+    // Rows past M and columns past N are read too, inside the tile's memory
+    // (every slice writes its whole tile, the slim kernel its rows); they are not
+    // stored.
     if constexpr (E == 4) {
         const float4 v = ordered_sum<BATCH>(Strided4{src, (size_t)8 * 128}, TILE, p.main_splits);
         sh[warp][lane] = v.x;
