@@ -50,7 +50,9 @@ cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, unsigned threads,
         attr[1].val.clusterDim.z = 1;
         cfg.numAttrs = 2;
     }
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) cudaGetLastError();      // reported by the status alone, not by the next check too
+    return e;
 }
 
 }  // namespace mmsk
