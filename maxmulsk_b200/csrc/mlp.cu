@@ -441,7 +441,11 @@ void mlp_unload() {
     g_model_gen++;
 }
 
-bool mlp_predict_host(size_t M, size_t K, size_t N, int cls, float* y) {
+namespace {
+
+// mlp_predict_host, and what the first weights say (`y0`) where the file holds a
+// second set for the split class; `two` tells whether it does.
+bool predict_host(size_t M, size_t K, size_t N, int cls, float* y, float* y0, bool* two) {
     std::lock_guard<std::mutex> lk(g_model_mu);
     if (!g_env_tried) {
         // MAXMULSK_MODEL names the weights; unset, the model shipped beside
@@ -459,22 +463,35 @@ bool mlp_predict_host(size_t M, size_t K, size_t N, int cls, float* y) {
     if (!g_model.loaded) return false;
     float x[F];
     mlp_features(M, K, N, cls, x);
-    host_forward(g_model.w.data() + (cls == 1 && g_model.w.size() > (size_t)NPARAM ? NPARAM : 0), x, y);
+    *two = cls == 1 && g_model.w.size() > (size_t)NPARAM;
+    host_forward(g_model.w.data() + (*two ? NPARAM : 0), x, y);
+    if (*two && y0) host_forward(g_model.w.data(), x, y0);
     return true;
 }
 
-namespace {
-
 // The model's pick for a shape (mlp_predict_plan without its memory).
+//
+// Weights of the split class's own rank plans by time; how a product is summed is
+// not theirs to trade. The plan taken has the precision of the first weights' pick
+// (it matters under SPLIT_AUTO) and cuts K into no fewer slices, so that no chain
+// of adds is longer. Of 5,400 timed shapes SPLIT_AUTO would otherwise move 12 % to
+// 3xTF32's fewer bits, and 9 % would get longer chains, with up to 15 % more error
+// against FP64 (243 shapes); with the floor the worst of those has 3.3 % more (37 x
+// 664 x 17, twice the slices), the geometric mean is 0.3 % less. On the 800 shapes
+// held out the SPLIT_AUTO picks cost 7.1 % over the best plan with the first weights,
+// 3.3 % with the second alone, 4.1 % above the floor (geometric mean).
 bool predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan* out, float* margin) {
     const int cls = (precision == MAXMULSK_PREC_FP32) ? 0 : 1;
-    float y[O];
-    if (!mlp_predict_host(M, K, N, cls, y)) return false;
+    float y[O], y0[O];
+    bool two = false;
+    if (!predict_host(M, K, N, cls, y, y0, &two)) return false;
     maxmulsk_plan cands[O];
     const int n = candidate_plans(cls, cands, O);
     const size_t max_workspace = (64u << 20) + 4 * sizeof(float) * (M * K + K * N + M * N);
-    int best = -1, second = -1;
+    bool runs[O];
+    int first = -1;                                                // the first weights' pick
     for (int i = 0; i < n; i++) {
+        runs[i] = false;
         if (precision != MAXMULSK_PREC_FP32 && precision != MAXMULSK_PREC_SPLIT_AUTO &&
             cands[i].precision != precision)
             continue;                                              // an explicit split mode
@@ -482,6 +499,17 @@ bool predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan* ou
         // Plans with outsized split-K scratch were never timed (the autotuner
         // masks them), so the model's estimate for them means nothing.
         if (workspace_bytes(M, K, N, cands[i]) > max_workspace) continue;
+        runs[i] = true;
+        if (two && (first < 0 || y0[i] < y0[first])) first = i;
+    }
+    auto slices = [&](const maxmulsk_plan& p) {
+        return tc_slice_count((int64_t)M, (int64_t)K, (int64_t)N, p.precision, p.tile_m, p.tile_n, p.split_k);
+    };
+    const int floor_slices = first >= 0 ? slices(cands[first]) : 0;
+    int best = -1, second = -1;
+    for (int i = 0; i < n; i++) {
+        if (!runs[i]) continue;
+        if (first >= 0 && (cands[i].precision != cands[first].precision || slices(cands[i]) < floor_slices)) continue;
         if (best < 0 || y[i] < y[best]) { second = best; best = i; }
         else if (second < 0 || y[i] < y[second]) second = i;
     }
@@ -511,6 +539,11 @@ constexpr size_t kPickEntries = 128;
 thread_local PickEntry t_picks[kPickEntries];
 
 }  // namespace
+
+bool mlp_predict_host(size_t M, size_t K, size_t N, int cls, float* y) {
+    bool two = false;
+    return predict_host(M, K, N, cls, y, nullptr, &two);
+}
 
 bool mlp_predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan* out, float* margin) {
     if (precision == MAXMULSK_PREC_BF16X9) return false;          // not among the candidates

@@ -2167,6 +2167,11 @@ int tc_slots(int precision, int tile_m, int tile_n) {
     return n;
 }
 
+int tc_slice_count(int64_t M, int64_t K, int64_t N, int precision, int tile_m, int tile_n, int split_k) {
+    if (M == 0 || K == 0 || N == 0) return 1;
+    return make_sched(M, K, N, tile_m, tile_n, split_k, tc_slots(precision, tile_m, tile_n)).main_splits;
+}
+
 size_t tc_workspace_bytes(int64_t M, int64_t K, int64_t N, int precision, int tile_m, int tile_n, int split_k) {
     const PlaneGeom g = plane_geom(M, K, N, precision);
     const Sched sc = make_sched(M, K, N, tile_m, tile_n, split_k, tc_slots(precision, tile_m, tile_n));

@@ -3,6 +3,7 @@ differences, the model file read by the library's host forward pass, the
 features and the candidate lists."""
 import ctypes
 import math
+import os
 
 import numpy as np
 import pytest
@@ -291,5 +292,62 @@ def test_model_file_with_split_weights(built_lib, tmp_path):
         assert np.array_equal(predict(two, 1), predict(one_q, 1))
         assert np.array_equal(predict(cut, 1), predict(one_p, 1))
         assert np.array_equal(picker.load_params(two), p)
+    finally:
+        _load_shipped_model()
+
+
+def _slices(M, K, N, p, sms=148):
+    """K slices of a whole tile under a split-precision plan, as documented."""
+    sk = p[3]
+    if sk == 0:
+        sk = max(1, min(64, sms // (-(-M // p[1]) * -(-N // p[2]))))
+    return mm.slice_count(K, sk)
+
+
+def test_split_weights_keep_precision_and_slices(built_lib, tmp_path, monkeypatch):
+    # Weights of the split class's own choose among the plans that have the
+    # precision of the first weights' pick and cut K into no fewer slices: the best
+    # predicted of them, on the shipped file and on random weights; empty shapes
+    # pick too.
+    monkeypatch.delenv("MAXMULSK_CONFIG", raising=False)
+    mm.lib().maxmulsk_tuning_clear()
+    shipped = os.path.join(os.path.dirname(picker.__file__), "data", "picker_model.bin")
+    data = open(shipped, "rb").read()
+    rng = np.random.default_rng(17)
+    files = [(np.frombuffer(data[24 + 4 * i * picker.NPARAM:24 + 4 * (i + 1) * picker.NPARAM], np.float32)) for i in (0, 1)]
+    sets = [tuple(files), tuple(rng.normal(0, 0.4, picker.NPARAM).astype(np.float32) for _ in range(2))]
+    shapes = [tuple(int(x) for x in np.exp(rng.uniform(np.log(lo), np.log(hi + 1), 3)))
+              for lo, hi in [(1, 16384)] * 150 + [(256, 4096)] * 100]
+    shapes += [(2048,) * 3, (4096,) * 3, (1500, 2049, 1999)]
+    cands = [tuple(int(v) for v in r)
+             for r in np.load(os.path.join(os.path.dirname(shipped), "picker_timings_split.npz"))["cand_split"]]
+    out = (ctypes.c_float * 48)()
+    modes = (mm.Precision.SPLIT_AUTO, mm.Precision.TF32X3, mm.Precision.BF16X6, mm.Precision.BF16X9)
+
+    def load(*weights):
+        path = str(tmp_path / "m.bin")
+        picker.save_params(path, *weights)
+        assert mm.lib().maxmulsk_model_load(path.encode()) == 0
+
+    try:
+        for p, q in sets:
+            load(p)
+            first = {(s, m): mm.choose(*s, m).as_tuple() for s in shapes for m in modes}
+            load(p, q)
+            for s in shapes:
+                M, K, N = s
+                assert mm.lib().maxmulsk_mlp_predict_host(M, K, N, 1, out) == 0
+                cap = (64 << 20) + 16 * (M * K + K * N + M * N)
+                for m in modes:
+                    got, base = mm.choose(*s, m).as_tuple(), first[s, m]
+                    assert got[0] == base[0], (s, m, got, base)
+                    assert _slices(M, K, N, got) >= _slices(M, K, N, base), (s, m, got, base)
+                    ok = [i for i, c in enumerate(cands)
+                          if c[0] == min(base[0], 2) and _slices(M, K, N, c) >= _slices(M, K, N, base)
+                          and mm.classify(M, K, N, mm.make_plan(*c)) == 0
+                          and mm.workspace_bytes(M, K, N, mm.make_plan(*c)) <= cap]
+                    assert got[1:] == cands[min(ok, key=lambda i: out[i])][1:], (s, m, got, base)
+            assert mm.choose(0, 5, 7, mm.Precision.BF16X6).precision == mm.Precision.BF16X6
+            assert mm.choose(5, 0, 7, mm.Precision.SPLIT_AUTO).precision in (1, 2)
     finally:
         _load_shipped_model()
