@@ -156,13 +156,18 @@ bool parse_config_env(maxmulsk_plan& out) {
 // the best of the three on average (9.6 % at most), against 1.4 % / 27 % / 75 %
 // for 64x64 / 128x64 / 128x128 everywhere. On the model's own tiles, chosen for
 // slower kernels, those shapes took 7.2 % over the exhaustive best in total
-// time, with this rule 2.6 %; 4096^3 (two slices) 2535 -> 2381 us.
+// time, with this rule 2.6 %; 4096^3 (two slices) 2535 -> 2381 us. A tile whose
+// scratch (the arrival counters depend on the tile) would take a plan past the
+// static-scratch entry's limit is passed over, so that the entry runs what it runs
+// on the model's tile.
 maxmulsk_plan with_best_fp32_tile(size_t M, size_t K, size_t N, maxmulsk_plan p, int sms) {
     struct Tile { int m, n, ctas; double part, full, per_round_us; };
     static const Tile tiles[3] = {{128, 128, 2, 0.74, 0.81, 3.4}, {128, 64, 2, 0.69, 0.75, 2.0}, {64, 64, 4, 0.68, 0.66, 1.3}};
     if (sms <= 0) sms = 148;
     const double us_per_mac = 1.0 / (128.0 * 1965.0);
     const double len = (double)slice_len(K, p.split_k), slices = (double)slice_count(K, p.split_k);
+    const size_t limit = MAXMULSK_STATIC_SCRATCH_BYTES;
+    const bool static_fits = workspace_bytes(M, K, N, p) <= limit;
     double best = -1.0;
     maxmulsk_plan out = p;
     for (const Tile& t : tiles) {
@@ -170,6 +175,7 @@ maxmulsk_plan with_best_fp32_tile(size_t M, size_t K, size_t N, maxmulsk_plan p,
         c.tile_m = t.m;
         c.tile_n = t.n;
         if (classify_plan(M, K, N, &c) != MAXMULSK_OK) continue;
+        if (static_fits && workspace_bytes(M, K, N, c) > limit) continue;
         const double units = (double)((M + t.m - 1) / t.m) * (double)((N + t.n - 1) / t.n) * slices;
         const double q = std::ceil(units / sms), rounds = std::floor(q / t.ctas), rest = q - rounds * t.ctas;
         const double mac = len * t.m * t.n * us_per_mac;

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 import maxmulsk_b200 as mm
-from maxmulsk_b200 import picker
+from maxmulsk_b200 import autotune, picker
 
 
 def _oracle():
@@ -351,3 +351,31 @@ def test_split_weights_keep_precision_and_slices(built_lib, tmp_path, monkeypatc
             assert mm.choose(5, 0, 7, mm.Precision.SPLIT_AUTO).precision in (1, 2)
     finally:
         _load_shipped_model()
+
+
+def test_fp32_tile_keeps_plans_within_the_static_scratch(built_lib, monkeypatch):
+    # Shapes whose slices nearly fill the static entry's 16 MiB: where the plan on
+    # the model's own tile fits, the plan on the tile taken instead fits too.
+    monkeypatch.delenv("MAXMULSK_CONFIG", raising=False)
+    mm.lib().maxmulsk_tuning_clear()
+    _load_shipped_model()
+    limit = 16 << 20
+    out = (ctypes.c_float * 48)()
+    cands = autotune.candidates(0)
+    fits = 0
+    for M in list(range(6200, 6600, 3)) + list(range(250, 900, 13)):
+        for s in (2, 4, 8, 16):
+            N = (limit // 4 - 64) // (s * M)
+            for K in (1024, 2048, 4096):
+                got = mm.choose(M, K, N, mm.Precision.FP32)
+                if mm.slice_count(K, got.split_k) != s:
+                    continue
+                assert mm.lib().maxmulsk_mlp_predict_host(M, K, N, 0, out) == 0
+                cap = (64 << 20) + 16 * (M * K + K * N + M * N)
+                ok = [i for i, c in enumerate(cands) if mm.classify(M, K, N, c) == 0
+                      and mm.workspace_bytes(M, K, N, c) <= cap]
+                own = cands[min(ok, key=lambda i: out[i])]
+                if mm.workspace_bytes(M, K, N, own) <= limit:
+                    fits += 1
+                    assert mm.workspace_bytes(M, K, N, got) <= limit, (M, K, N, got, own)
+    assert fits > 50
