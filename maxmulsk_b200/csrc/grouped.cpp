@@ -327,7 +327,9 @@ maxmulsk_status build_tc(maxmulsk_grouped_s* g, const maxmulsk_problem* problems
             g->repack.push_back({dst, p.A, p.M, p.K, (size_t)lda});
             a = dst;
         }
-        if (!tc_fused_maps(a, lda, p.B, (int64_t)p.M, (int64_t)p.K, (int64_t)p.N, &maps[256 * j])) {
+        const int mt = tc_slim_rows((int64_t)p.M, slice_count(p.K, sk[j]), (int64_t)slice_len(p.K, sk[j]), true);
+        hp[j].mt = mt;
+        if (!tc_fused_maps(a, lda, p.B, (int64_t)p.M, (int64_t)p.K, (int64_t)p.N, mt, &maps[256 * j])) {
             set_error_message("grouped: tensor map encoding failed");
             return MAXMULSK_ERR_CUDA;
         }
@@ -338,14 +340,12 @@ maxmulsk_status build_tc(maxmulsk_grouped_s* g, const maxmulsk_problem* problems
     for (size_t j = 0; j < n; j++) {
         const maxmulsk_problem& p = problems[idx[j]];
         TcGroupProblem& q = hp[j];
-        std::memset(&q, 0, sizeof q);
         q.M = (int64_t)p.M; q.K = (int64_t)p.K; q.N = (int64_t)p.N;
         q.C = p.C;
         q.splits = slice_count(p.K, sk[j]);
         q.kchunk = (int64_t)slice_len(p.K, sk[j]);
         q.tiles_n = (int32_t)((p.N + T - 1) / T);
         q.chunk_kb = tc_chunk_len((int64_t)p.K, q.splits) / 32;
-        q.mt = tc_slim_rows((int64_t)p.M);
         const int tm_n = (int)((p.M + T - 1) / T);
         for (int z = 0; z < q.splits; z++)
             for (int tm = 0; tm < tm_n; tm++)

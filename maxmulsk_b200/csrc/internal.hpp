@@ -137,10 +137,11 @@ struct TcGroupArgs {
 };
 // Encodes the two FP32 tensor maps the fused split reads for one problem
 // (A: K-contiguous rows lda floats apart, B: N-contiguous rows) into
-// out[0..255]. lda and N multiples of 4, A and B 16-byte aligned.
-bool tc_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N, void* out);
-// Rows of the slim fused kernel's tile for an M-row product, or 0: the wide kernel.
-int tc_slim_rows(int64_t M);
+// out[0..255]. lda and N multiples of 4, A and B 16-byte aligned. `mt`: tc_slim_rows.
+bool tc_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N, int mt, void* out);
+// Rows of the slim fused kernel's tile for an M-row product in `splits` K slices of
+// `slice_k`, or 0: the wide kernel.
+int tc_slim_rows(int64_t M, int splits, int64_t slice_k, bool grouped);
 // Chunk length (k's per TMEM accumulation) the kernels use for K and a K split.
 int tc_chunk_len(int64_t K, int splits);
 // One launch over units of problems that all run the slim kernel, or all the wide one.

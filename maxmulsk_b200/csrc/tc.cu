@@ -1324,7 +1324,7 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // graphs, inputs from HBM, the wide kernel first): 1 x 32768 x 512 29.5 / 32.6 ->
 // 24.2 / 28.2 us, 16 x 16384 x 1024 30.7 / 34.1 -> 24.9 / 29.0, 64 x 32768 x 512
 // 30.0 / 33.5 -> 28.2 / 31.2; the grouped batch of 256 GEMMs 3.86 -> 3.55 ms.
-// (64 x 512 x 4096: 12.3 -> 12.7; above 64 rows the shared memory saved is gone.)
+// (Above 64 rows the shared memory saved is gone; tc_slim_rows has the line.)
 //
 // Converters take whole stages in turn: with every warp at a part of every
 // stage the waits set the pace (1 x 32768 x 512 29.9 us); twelve B or four A warps
@@ -1333,8 +1333,9 @@ tc_fused_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue (one column
 // of C a thread), warps 6-13 cut B (a TMEM lane quarter of every other stage each),
 // warps 14-15 cut A (rows lane and lane + 32). C^T leaves the accumulators, so that
-// consecutive lanes store consecutive columns of a row of C, and K slices go to
-// the column-major partial tiles a column a thread.
+// consecutive lanes store consecutive columns of a row of C. K slices go to the
+// reduction kernel's column-major partial tiles a column a thread, or, summed by
+// the last slice to arrive, to row-major ones.
 // ============================================================================
 constexpr int kSlimRows = 64;
 
@@ -1551,16 +1552,33 @@ __device__ __forceinline__ void slim_roles(const Src& src, const void* tmA1, con
                 store_col_regs(sum, v.C, col, v.M, v.N);
                 continue;
             }
-            // Partial tiles are column-major, 128 rows a column: this thread's
-            // column is contiguous (its first mt rows written).
             constexpr size_t TILE = (size_t)128 * Cf::BN;
-            float* seg = v.partial + (size_t)w.sti * v.max_splits * TILE + (size_t)ncol * 128;
+            float* tile = v.partial + (size_t)w.sti * v.max_splits * TILE;
+            if (v.reduce_after) {
+                // The reduction kernel's partial tiles are column-major, 128 rows a
+                // column: this thread's column is contiguous (its first mt rows
+                // written).
+                float* part = tile + (size_t)w.z * TILE + (size_t)ncol * 128;
+#pragma unroll
+                for (int m = 0; m < kSlimRows; m += 4)
+                    if (m < v.mt)
+                        __stcg(reinterpret_cast<float4*>(part + m), make_float4(sum[m], sum[m + 1], sum[m + 2], sum[m + 3]));
+                continue;
+            }
+            // Summed here: row-major partial tiles, so that the warp writes and reads
+            // 128-byte lines, and the rows' loads of a slice overlap. Read down its
+            // column by each thread (16-byte pieces, a round trip per four rows), two
+            // slices of 64 x 128 x 8192 took 22.5 us, now 16.4; a group of 47
+            // 48 x 2048 x 1024 in eight slices 578 us, now 483.
+            float* seg = tile + ncol;
             float* part = seg + (size_t)w.z * TILE;
 #pragma unroll
-            for (int m = 0; m < kSlimRows; m += 4)
-                if (m < v.mt)
-                    __stcg(reinterpret_cast<float4*>(part + m), make_float4(sum[m], sum[m + 1], sum[m + 2], sum[m + 3]));
-            if (v.reduce_after) continue;
+            for (int c = 0; c < kSlimRows; c += 16) {
+                if (c < v.mt) {
+#pragma unroll
+                    for (int m = c; m < c + 16; m++) __stcg(part + (size_t)m * Cf::BN, sum[m]);
+                }
+            }
             unsigned* ctr = v.counters + (size_t)w.sti * Cf::EPI + ew;
             __threadfence();
             __syncwarp();
@@ -1569,11 +1587,17 @@ __device__ __forceinline__ void slim_roles(const Src& src, const void* tmA1, con
             last = __shfl_sync(0xffffffffu, last, 0);
             if (!last) continue;
             __threadfence();
+            for (int q = 0; q < w.nsplit; q++) {
+                const float* bq = seg + (size_t)q * TILE;
 #pragma unroll
-            for (int m = 0; m < kSlimRows; m += 4) {
-                if (m < v.mt) {
-                    const float4 t = ordered_sum<7>(reinterpret_cast<const float4*>(seg + m), TILE / 4, w.nsplit);
-                    sum[m] = t.x; sum[m + 1] = t.y; sum[m + 2] = t.z; sum[m + 3] = t.w;
+                for (int c = 0; c < kSlimRows; c += 16) {
+                    if (c < v.mt) {
+#pragma unroll
+                        for (int m = c; m < c + 16; m++) {
+                            const float x = __ldcg(bq + (size_t)m * Cf::BN);
+                            sum[m] = q == 0 ? x : __fadd_rn(sum[m], x);
+                        }
+                    }
                 }
             }
             store_col_regs(sum, v.C, col, v.M, v.N);
@@ -2061,9 +2085,9 @@ cudaError_t launch_fused(const TcArgs& a, cudaStream_t s) {
     using Cf = CfgFused<MODE>;
     constexpr int BN = Cf::BN;
     CUtensorMap tmA, tmB;
-    const int mt = tc_slim_rows(a.M);
-    if (!encode_fused_maps(a.A, a.K, a.B, a.M, a.K, a.N, mt ? mt : 128, &tmA, &tmB)) return cudaErrorInvalidValue;
     const Sched sc = make_sched(a.M, a.K, a.N, 128, BN, a.split_k, tc_slots(a.precision, 128, BN));
+    const int mt = tc_slim_rows(a.M, sc.main_splits, sc.main_kchunk, false);
+    if (!encode_fused_maps(a.A, a.K, a.B, a.M, a.K, a.N, mt ? mt : 128, &tmA, &tmB)) return cudaErrorInvalidValue;
     TcParams prm = make_params(a, sc, Cf::BK);
     if (sc.split_tiles > 0 && (!a.partial || !a.counters)) return cudaErrorInvalidValue;
     if (mt) {
@@ -2139,9 +2163,19 @@ int pair_slots_for() {
 
 }  // namespace
 
-// Rows of the slim kernel's tile for an M-row fused product, or 0 for the wide
-// kernel.
-int tc_slim_rows(int64_t M) { return M <= kSlimRows ? (int)((M + 15) / 16 * 16) : 0; }
+// Rows of the slim kernel's tile for an M-row fused product cut into `splits` K
+// slices of `slice_k`, or 0 for the wide kernel. The wide one is the better of the
+// two where more than 48 rows' partial tiles for the reduction kernel (written in
+// 16-byte pieces) follow only one or two
+// 32-k stages. Times over the wide kernel's, BF16x6 and BF16x9, 3,900 sizes of 1 to
+// 64 rows, N 64 to 32768, K 96 to 32768, one to 64 slices, single and grouped:
+// there 0.99-1.07 (64 x 128 x 64 in four slices 7.5 us against 7.0), geometric mean
+// 1.03; elsewhere 0.26-1.06, 0.88 single and 0.75 grouped.
+int tc_slim_rows(int64_t M, int splits, int64_t slice_k, bool grouped) {
+    if (M > kSlimRows) return 0;
+    if (M > 48 && !grouped && splits >= kReduceAfterSplits && slice_k <= 64) return 0;
+    return (int)((M + 15) / 16 * 16);
+}
 
 // Concurrently resident work slots of a configuration on the current device:
 // the SM count for one-CTA tiles, the number of CTA pairs that fit at once
@@ -2226,9 +2260,8 @@ cudaError_t tc_launch(const TcArgs& a, cudaStream_t s) {
     }
 }
 
-bool tc_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N, void* out) {
+bool tc_fused_maps(const float* A, int64_t lda, const float* B, int64_t M, int64_t K, int64_t N, int mt, void* out) {
     CUtensorMap* m = static_cast<CUtensorMap*>(out);
-    const int mt = tc_slim_rows(M);
     return encode_fused_maps(A, lda, B, M, K, N, mt ? mt : 128, &m[0], &m[1]);
 }
 

@@ -250,3 +250,25 @@ def test_few_row_problems_run_on_their_own_tiles(cuda, oracle_mod):
             assert np.array_equal(bits(c.cpu().numpy().reshape(m, n)), bits(want)), (m, k, n, p)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("prec", [2, 3])
+@pytest.mark.parametrize("split", [1, 2, 3, 8, 64])
+def test_grouped_slim_slices_equal_split_inputs(cuda, oracle_mod, prec, split):
+    # Problems of at most 64 rows, whose slices the kernel sums itself, beside wide
+    # ones; two replays.
+    shapes = [(1, 512, 128), (16, 4096, 260), (17, 640, 132), (33, 1028, 516), (48, 320, 128), (49, 96, 260), (64, 64, 4),
+              (64, 2048, 512), (65, 512, 132), (200, 1024, 128)]
+    g, cbuf, host, offs = _group(cuda, oracle_mod, shapes, 700, mm.make_plan(prec, 128, 128, split))
+    try:
+        for _ in range(2):
+            cbuf.fill_(float("nan"))
+            cuda.cuda.synchronize()
+            assert g.launch() == 0 and mm.stream_status() == 0
+            c = cbuf.cpu().numpy()
+            for (M, K, N), (A, B), off in zip(shapes, host, offs):
+                st, want, _ = run_plan(cuda, A, B, M, K, N, mm.make_plan(prec, 128, 128, split, mm.TC_SPLIT_INPUTS))
+                assert st == 0
+                assert np.array_equal(c[off: off + M * N].view(np.uint32), want.ravel().view(np.uint32)), (M, K, N)
+    finally:
+        g.close()

@@ -264,3 +264,51 @@ def test_slim_fused_equals_split_inputs(cuda, oracle_mod, prec, M):
             st, C, bands = run_plan(cuda, A, B, M, K, N, mm.make_plan(prec, 128, 128, split, mm.TC_FUSED_SPLIT, chunk))
             assert st == 0 and bands, mm.last_error_message()
             assert np.array_equal(bits(C), bits(want)), (M, K, N, split, chunk)
+
+
+# The slim kernel's K slices summed in the kernel (two slices, tail waves) and by
+# the reduction, on both sides of the line between it and the wide kernel (more than
+# 48 rows, three slices of 64 or 96 k's): bit for bit the split-inputs path.
+@pytest.mark.parametrize("M", [1, 16, 33, 48, 49, 64])
+def test_slim_slices_equal_split_inputs(cuda, oracle_mod, M):
+    for K, N, split in [(64, 132, 2), (500, 8196, 2), (192, 260, 3), (288, 260, 3), (4096, 100, 64), (1024, 19200, 1)]:
+        A, B = oracle_mod.fill_uniform(M * K, 31), oracle_mod.fill_wide(K * N, 32)
+        st, want, _ = run_plan(cuda, A, B, M, K, N, mm.make_plan(2, 128, 128, split, mm.TC_SPLIT_INPUTS))
+        assert st == 0, mm.last_error_message()
+        st, C, bands = run_plan(cuda, A, B, M, K, N, mm.make_plan(2, 128, 128, split, mm.TC_FUSED_SPLIT))
+        assert st == 0 and bands, mm.last_error_message()
+        assert np.array_equal(bits(C), bits(want)), (M, K, N, split)
+
+
+@pytest.mark.parametrize("shape,split", [((64, 128, 8192), 2), ((33, 256, 8192), 2), ((64, 512, 8192), 2), ((64, 128, 64), 0)])
+def test_few_rows_take_no_longer_than_one_tile_more(cuda, shape, split):
+    # Products of at most 64 rows against 65 rows of the same sizes, which the wide
+    # kernel runs with more to load, store and multiply: no slower, 10 % allowed for
+    # the clock (two slices took 1.2 to 1.4 times as long when the slim kernel read
+    # partial tiles down their columns).
+    torch = cuda
+    M, K, N = shape
+
+    def us(rows):
+        A, B, C = torch.randn(rows, K, device="cuda"), torch.randn(K, N, device="cuda"), torch.empty(rows, N, device="cuda")
+        p = mm.make_plan(2, 128, 128, split, mm.TC_FUSED_SPLIT)
+        nb = mm.workspace_bytes(rows, K, N, p)
+        ws = torch.empty(nb + 256, dtype=torch.uint8, device="cuda")
+        wp = ws.data_ptr() + (-ws.data_ptr()) % 256
+        g = torch.cuda.CUDAGraph()
+        assert mm.sgemm_plan_dev(A, B, C, rows, K, N, p, wp, nb) == 0, mm.last_error_message()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g):
+            for _ in range(50):
+                mm.sgemm_plan_dev(A, B, C, rows, K, N, p, wp, nb)
+        times = []
+        for _ in range(5):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            g.replay()
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1) * 20)
+        return sorted(times)[2]
+
+    assert us(M) <= 1.1 * us(65)
