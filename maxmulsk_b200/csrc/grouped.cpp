@@ -473,12 +473,50 @@ maxmulsk_status build_group(maxmulsk_grouped_s* g, const maxmulsk_problem* probl
     return MAXMULSK_OK;
 }
 
+// A second stream to capture a parallel branch of a graph on.
+struct Branch {
+    cudaStream_t s = nullptr;
+    cudaEvent_t out = nullptr, in = nullptr;
+    cudaError_t create() {
+        cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&out, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&in, cudaEventDisableTiming);
+        return e;
+    }
+    cudaError_t fork(cudaStream_t from) {
+        cudaError_t e = cudaEventRecord(out, from);
+        return e == cudaSuccess ? cudaStreamWaitEvent(s, out, 0) : e;
+    }
+    cudaError_t join(cudaStream_t to) {
+        cudaError_t e = cudaEventRecord(in, s);
+        return e == cudaSuccess ? cudaStreamWaitEvent(to, in, 0) : e;
+    }
+    ~Branch() {
+        if (s) cudaStreamDestroy(s);
+        if (out) cudaEventDestroy(out);
+        if (in) cudaEventDestroy(in);
+    }
+};
+
 // Captures the group's work into its graph: K == 0 problems zero-filled, the
 // unit counter and split-K arrival counters reset, the A repacks, the
-// persistent kernel(s), then the single launches.
+// persistent kernel(s), then the single launches. The slim fused kernel runs on a
+// branch beside the wide one: one CTA an SM each, so the slim kernel's start where
+// the wide one's leave an SM or never took one, and the K splits, planned over
+// both, balance them together as they would one launch. One after the other, the
+// few long units of, say, two 64 x 32768 x 128 problems run on an otherwise idle
+// GPU: beside a 1024 x 4096 x 4096 275 us, 241 with the branch (one kernel for all,
+// which stages rows that are not there, 242); eight 256 x 2048 x 2048 and forty 16 x
+// 2048 x 512 220 / 201 / 212; the batch of 256 GEMMs 3.63 / 3.59 / 4.72 ms. Splits
+// planned for each kernel by itself cut three 64 x 32768 x 128 problems into 64
+// slices each, whose sums at the end cost more than they balance (394 us a group
+// with three 512 x 4096 x 3072, 261 now); the slim kernel first: 283.
 maxmulsk_status capture_group(maxmulsk_grouped_s* g, const maxmulsk_problem* problems) {
     cudaError_t e = cudaStreamCreateWithFlags(&g->cap, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_status(e, "cudaStreamCreate");
+    const bool beside = g->tc.nunits > 0 && g->slim.nunits > 0;
+    Branch branch;
+    if (beside && (e = branch.create()) != cudaSuccess) return cuda_status(e, "grouped: second capture stream");
     maxmulsk_status st = MAXMULSK_OK;
     e = cudaStreamBeginCapture(g->cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
@@ -491,11 +529,16 @@ maxmulsk_status capture_group(maxmulsk_grouped_s* g, const maxmulsk_problem* pro
                                                r.cols * sizeof(float), r.rows, cudaMemcpyDeviceToDevice, g->cap);
             if (ec != cudaSuccess) e = ec;
         }
+        auto run = [&](cudaError_t r) {
+            if (e == cudaSuccess) e = r;
+        };
+        if (beside) run(branch.fork(g->cap));
         for (const bool slim : {false, true}) {
             const TcGroupArgs& t = slim ? g->slim : g->tc;
-            cudaError_t el = tc_grouped_launch(t, g->plan.precision, slim, (int)std::min<int64_t>(t.nunits, g->sms_tc), g->cap);
-            if (el != cudaSuccess) e = el;
+            run(tc_grouped_launch(t, g->plan.precision, slim, (int)std::min<int64_t>(t.nunits, g->sms_tc),
+                                  slim && beside ? branch.s : g->cap));
         }
+        if (beside) run(branch.join(g->cap));
         if (!g->simt_parts.empty()) cudaMemsetAsync(g->d_next, 0, g->simt_parts.size() * sizeof(unsigned), g->cap);
         if (g->d_scratch && g->counter_bytes) cudaMemsetAsync(g->d_scratch, 0, g->counter_bytes, g->cap);
         for (size_t i = 0; i < g->simt_parts.size(); i++) {

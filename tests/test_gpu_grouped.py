@@ -272,3 +272,30 @@ def test_grouped_slim_slices_equal_split_inputs(cuda, oracle_mod, prec, split):
                 assert np.array_equal(c[off: off + M * N].view(np.uint32), want.ravel().view(np.uint32)), (M, K, N)
     finally:
         g.close()
+
+
+def test_wide_and_slim_problems_run_side_by_side(cuda):
+    # Problems of more and of at most 64 rows, each kind with fewer units than SMs:
+    # together they take little longer than the slower kind, not the sum of both.
+    torch = cuda
+    wide, slim = [(128, 8192, 2048)] * 4, [(64, 8192, 2048)] * 4
+
+    def us(shapes):
+        A = [torch.randn(m * k, device="cuda") for m, k, n in shapes]
+        B = [torch.randn(k * n, device="cuda") for m, k, n in shapes]
+        C = [torch.empty(m * n, device="cuda") for m, k, n in shapes]
+        torch.cuda.synchronize()
+        g = mm.Grouped([(a, b, c, *s) for a, b, c, s in zip(A, B, C, shapes)], mm.make_plan(2, 128, 128, 1))
+        times = []
+        for _ in range(7):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(5):
+                assert g.launch() == 0
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1) * 200)
+        g.close()
+        return sorted(times)[3]
+
+    assert us(wide + slim) <= 0.8 * (us(wide) + us(slim))
