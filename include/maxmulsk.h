@@ -261,9 +261,9 @@ maxmulsk_status maxmulsk_grouped_launch(maxmulsk_grouped g, void* stream);
  * be NULL), number of work units. */
 maxmulsk_status maxmulsk_grouped_info(maxmulsk_grouped g, maxmulsk_plan* group_plan, int32_t* split_k,
                                       size_t* units);
-/* The plan each problem runs (count entries): FP32 problems the group's tile
- * (own tiles: the problem's, 64 x 64 standing for the 16 x 256 tile that no plan
- * names), their K split and variant; fused problems (precision, 128, 128, K
+/* The plan each problem runs (count entries): FP32 problems the group's tile (a
+ * group on own tiles names 64 x 64; an FP32 C is the same on every tile), their K
+ * split and variant; fused problems (precision, 128, 128, K
  * split, MAXMULSK_TC_FUSED_SPLIT) -- for an A repacked to a padded pitch the
  * result is that of MAXMULSK_TC_SPLIT_INPUTS on the same tiles; problems run as
  * their own launches, their plan. Each problem's C equals a single launch of its

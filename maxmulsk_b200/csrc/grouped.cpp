@@ -175,8 +175,10 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
     std::vector<SimtTile> tiles(idx.size(), SimtTile{plan.tile_m, plan.tile_n, 1.0, 2});
     if (mixed)
         for (size_t j = 0; j < idx.size(); j++) tiles[j] = own_tile(problems[idx[j]]);
-    std::vector<int> sk = plan_splits(problems, idx, tiles, 2 * sms, plan.split_k, share);   // 2 CTAs per SM
-    if (mixed) {
+    std::vector<int> sk(idx.size(), 1);
+    if (!mixed) {
+        sk = plan_splits(problems, idx, tiles, 2 * sms, plan.split_k, share);                 // 2 CTAs per SM
+    } else {
         // Each tile shape is a launch of its own and has to balance by itself.
         for (const SimtTile& t : kSimtTiles) {
             std::vector<size_t> at, sub;
@@ -191,9 +193,7 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
         g->split_k[idx[j]] = sk[j];
         maxmulsk_plan& q = g->plans[idx[j]];
         q = plan;
-        q.split_k = sk[j];
-        // A plan names 128 x 128, 128 x 64 or 64 x 64; C is the same on any tile.
-        if (tiles[j].bm >= 64) { q.tile_m = tiles[j].bm; q.tile_n = tiles[j].bn; }
+        q.split_k = sk[j];                                   // on the group's tile: C is the same on any
     }
 
     std::vector<GroupProblem> hp(idx.size());

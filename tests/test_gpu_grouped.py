@@ -299,3 +299,29 @@ def test_wide_and_slim_problems_run_side_by_side(cuda):
         return sorted(times)[3]
 
     assert us(wide + slim) <= 0.8 * (us(wide) + us(slim))
+
+
+def test_group_on_own_tiles_reports_one_tile_and_equals_the_oracle(cuda, oracle_mod):
+    # Mostly problems of few rows beside larger ones, where own tiles (several
+    # launches over one table of units) win by far: the plans name the group's tile all
+    # the same, and each C is the oracle's for its K split, in two replays.
+    odd = [(1, 300, 257), (16, 1025, 259), (17, 64, 300), (129, 333, 65), (64, 2050, 64), (300, 700, 140)]
+    shapes = odd + [(512, 1024, 512)] * 8 + [(100, 700, 96)] * 16 + [(8, 2048, 2048)] * 40
+    g, cbuf, host, offs = _group(cuda, oracle_mod, shapes, 400)
+    try:
+        plan, splits, _ = g.info()
+        assert {(p.tile_m, p.tile_n) for p in g.plans()} == {(plan.tile_m, plan.tile_n)}
+        assert [p.split_k for p in g.plans()] == list(splits)
+        for _ in range(2):
+            for (M, K, N), off in zip(shapes, offs):
+                cbuf[off: off + M * N].fill_(float("nan"))
+            cuda.cuda.synchronize()
+            assert g.launch() == 0 and mm.stream_status() == 0
+            c = cbuf.cpu().numpy()
+            for i in list(range(8)) + [14, 15, 30, 31, 69]:
+                (M, K, N), (A, B), off = shapes[i], host[i], offs[i]
+                want = oracle_mod.sgemm_panels(A, B, M, K, N, kc=mm.slice_len(K, splits[i]), fma=True)
+                assert np.array_equal(c[off: off + M * N].view(np.uint32), want.ravel().view(np.uint32)), (M, K, N)
+                assert np.all(c[off - 64: off] == SENT)
+    finally:
+        g.close()
