@@ -1,7 +1,7 @@
 // Kernel launches that overlap the end of the kernel before them.
 //
-// Every kernel of a call starts with grid_wait() and is launched with the
-// programmatic-serialization attribute: its blocks may become resident while
+// The kernels launched through launch_overlapped start with grid_wait() and have
+// the programmatic-serialization attribute: their blocks may become resident while
 // the kernel before it in the stream drains -- from the moment that all blocks
 // of that one have called grid_release(), or left -- and wait there until it
 // has completed and its writes are visible. Launch latency, block start-up,

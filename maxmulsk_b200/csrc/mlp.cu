@@ -348,7 +348,7 @@ bool g_env_tried = false;
 std::atomic<uint64_t> g_model_gen{1};         // counts the models there have been
 
 // z[o] = bias[o] + sum_i x[i] W[i][o], i upward, one fused multiply-add a step
-// (the order and rounding of linear_fwd): a row of W at a time, so that the
+// (the order and rounding of mlp_forward_kernel): a row of W at a time, so that the
 // outputs' chains fill vector registers instead of a library call per term.
 #define MMSK_ROWS_FMA(NAME, ATTR)                                                                 \
     ATTR void NAME(const float* x, const float* w, const float* bias, int in, int out, float* z) { \

@@ -171,7 +171,7 @@ struct CpCfg {
     static constexpr int B_FLOATS = BK * BN;
     static constexpr int STAGE_FLOATS = A_FLOATS + B_FLOATS;
     static constexpr int SMEM = STAGES * STAGE_FLOATS * 4;
-    static_assert(THREADS >= BK && BK % 2 == 0 && STAGES >= 3 && THREADS <= 4 * BN, "tile configuration");
+    static_assert(THREADS >= BK && BK % 4 == 0 && STAGES >= 3 && THREADS <= 4 * BN, "tile configuration");
 };
 
 // The plans' tiles. 128 x 128: 8 x 16 outputs a thread (255 registers, two

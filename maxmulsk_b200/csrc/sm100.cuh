@@ -141,7 +141,7 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar, uint32_t leader) {
         :: "r"(smem_u32(bar)), "r"(leader) : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem], FP32 accumulate; TF32 or BF16 inputs, one CTA
-// (CTAS 1) or a pair (2). Descriptors by halves: only the address half differs
+// or a pair (_pair). Descriptors by halves: only the address half differs
 // between the MMAs of a stage.
 #define MMSK_MMA(NAME, FORM)                                                                                     \
     __device__ __forceinline__ void NAME(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, \
@@ -196,14 +196,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
 __device__ __forceinline__ void tmem_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// 32 lanes x 8 columns of 32-bit TMEM from registers: thread i of the warp
-// writes lane (base lane + i), columns [col, col + 8).
-__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-        :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-        : "memory");
-}
 // 32 lanes x 16 columns of 32-bit TMEM from registers: thread i of the warp
 // writes lane (base lane + i), columns [col, col + 16).
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -249,10 +241,6 @@ __device__ __forceinline__ void cluster_sync() {
 // Arrive on an mbarrier given by its cluster address (possibly the peer's).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;"
-                 :: "r"(cluster_addr), "r"(bytes) : "memory");
 }
 // TMA load into this CTA's shared memory whose completion is counted on the
 // barrier at `bar_cluster_addr` (the leader CTA's barrier of the pair).

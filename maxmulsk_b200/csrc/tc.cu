@@ -370,13 +370,9 @@ __device__ __forceinline__ void epilogue_role(const Src& src, int* err, long lon
 #pragma unroll
             for (int c = 0; c < COLS; c += Cf::LDW) {
                 uint32_t r[Cf::LDW];
-                if constexpr (Cf::LDW == 16) {
-                    tmem_ld_32x32b_x16(taddr + (uint32_t)c, r);
-                } else {
 #pragma unroll
-                    for (int h = 0; h < Cf::LDW; h += 32)
-                        tmem_ld_32x32b_x32(taddr + (uint32_t)(c + h), *reinterpret_cast<uint32_t(*)[32]>(&r[h]));
-                }
+                for (int h = 0; h < Cf::LDW; h += 32)
+                    tmem_ld_32x32b_x32(taddr + (uint32_t)(c + h), *reinterpret_cast<uint32_t(*)[32]>(&r[h]));
                 tmem_wait_ld();
                 if (kb0 == 0) {
 #pragma unroll
@@ -903,8 +899,6 @@ struct CfgFused {
     static constexpr int EPI = 4;                    // epilogue warps 2 .. 5, one per TMEM lane quarter
     static constexpr int NCONV = 8;                  // converter warps 6 .. 13: two sets of four
     static constexpr int THREADS = 64 + 32 * (EPI + NCONV);
-    // C leaves from the TMEM sums 32 columns at a time through registers.
-    static constexpr bool TMA_STORE = false;
     static constexpr int SMEM = RING + 1024;
     static_assert(SMEM <= kSmemCap, "shared memory");
     static_assert(NCONV * 16 == BM && NCONV == 2 * NBOX, "one converter lane per A row and per B box row");
@@ -915,8 +909,6 @@ struct CfgFused {
 struct GroupSrc {
     const TcGroupArgs& g;
     __device__ __forceinline__ int64_t units() const { return g.nunits; }
-    // C of a grouped problem is written from registers.
-    __device__ __forceinline__ const CUtensorMap* store_map(const UnitView&) const { return nullptr; }
     // The r-th unit of this CTA: the units are sorted heaviest first and dealt
     // in a snake order (forward in even rounds, backward in odd rounds), which
     // evens out the sums of unequal units across CTAs.
@@ -1077,8 +1069,8 @@ __device__ __forceinline__ void epilogue_role_tsum(const Src& src, int* err, lon
 }
 
 template <int MODE, class Src>
-__device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, const void* tmB1, const void* tmC1,
-                                            int* err, long long timeout) {
+__device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, const void* tmB1, int* err,
+                                            long long timeout) {
     using Cf = CfgFused<MODE>;
     constexpr int BN = Cf::BN;
     extern __shared__ uint8_t smem_raw[];
@@ -1111,7 +1103,6 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
     if (warp == 0 && lane == 0 && tmA1) {
         prefetch_tmap(tmA1);
         prefetch_tmap(tmB1);
-        if (tmC1) prefetch_tmap(tmC1);
     }
     if (warp == 1) { tmem_alloc(&tmem_base_s, Cf::TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
@@ -1301,14 +1292,10 @@ __device__ __forceinline__ void fused_roles(const Src& src, const void* tmA1, co
 
 template <int MODE, bool GROUPED>
 __global__ void __launch_bounds__(CfgFused<MODE>::THREADS, 1)
-tc_fused_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const __grid_constant__ CUtensorMap tmC, const TcParams p, const TcGroupArgs g) {
-    if constexpr (GROUPED) {
-        fused_roles<MODE>(GroupSrc{g}, nullptr, nullptr, nullptr, g.err, g.timeout);
-    } else {
-        const CUtensorMap* c = p.store_c ? &tmC : nullptr;
-        fused_roles<MODE>(SingleSrc{p, c}, &tmA, &tmB, c, p.err, p.timeout);
-    }
+tc_fused_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p,
+                const TcGroupArgs g) {
+    if constexpr (GROUPED) fused_roles<MODE>(GroupSrc{g}, nullptr, nullptr, g.err, g.timeout);
+    else fused_roles<MODE>(SingleSrc{p}, &tmA, &tmB, p.err, p.timeout);
 }
 
 // ============================================================================
@@ -2105,9 +2092,6 @@ cudaError_t launch_fused(const TcArgs& a, cudaStream_t s) {
         PhaseScope ps(kPhaseReduce, s);
         return launch_reduce<BN>(prm, s);
     }
-    CUtensorMap tmC;
-    prm.store_c = (encode_c_map(a.C, a.M, a.N, &tmC) && Cf::TMA_STORE) ? 1 : 0;
-
     static std::atomic<uint64_t> smem_set{0};
     cudaError_t e = set_smem_once(tc_fused_kernel<MODE, false>, Cf::SMEM, smem_set);
     if (e != cudaSuccess) return e;
@@ -2115,7 +2099,7 @@ cudaError_t launch_fused(const TcArgs& a, cudaStream_t s) {
     {
         PhaseScope ps(kPhaseGemm, s);
         e = launch_overlapped(tc_fused_kernel<MODE, false>, dim3((unsigned)sc.grid), Cf::THREADS, Cf::SMEM, s, 1, tmA, tmB,
-                              tmC, prm, none);
+                              prm, none);
     }
     if (e != cudaSuccess || !prm.reduce_after) return e;
     PhaseScope ps(kPhaseReduce, s);
@@ -2283,8 +2267,7 @@ cudaError_t grouped_launch_mode(const TcGroupArgs& g, bool slim, int grid, cudaS
     static std::atomic<uint64_t> smem_set{0};
     cudaError_t e = set_smem_once(tc_fused_kernel<MODE, true>, Cf::SMEM, smem_set);
     if (e != cudaSuccess) return e;
-    return launch_overlapped(tc_fused_kernel<MODE, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1, none, none, none, p,
-                             g);
+    return launch_overlapped(tc_fused_kernel<MODE, true>, dim3((unsigned)grid), Cf::THREADS, Cf::SMEM, s, 1, none, none, p, g);
 }
 }  // namespace
 
