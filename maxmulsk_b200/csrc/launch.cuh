@@ -16,10 +16,10 @@
 // its SM with room for more, the successor's early blocks crowd the SMs that
 // have most of it (FP32 calls back to back at 1024^3: 64 x 64 tiles 57 -> 84 us
 // with a release at the start, 128 x 64 tiles 54 -> 73 with one before the
-// stores). Measured (us a call, without -> with): FP32 256^3 in a graph 4.5 -> 4.1,
-// 777 x 1531 x 901 75.8 -> 71.3, BF16x6 64 x 8192 x 512 16.4 -> 13.9, 128 x 32768 x
-// 512 38.4 -> 34.6, BF16x9 1500 x 2049 x 1999 125.7 -> 118.9, a picker training step 39
-// -> 30.
+// stores). Measured (us a call from Python, this attribute off -> on, in turn on one
+// B200): FP32 256^3 13.4 -> 12.7 (in a graph 4.42 -> 4.00), 777 x 1531 x 901 75.8 ->
+// 71.0, BF16x6 64 x 8192 x 512 16.4 -> 13.5, 128 x 32768 x 512 37.5 -> 35.1, BF16x9 1500 x
+// 2049 x 1999 124.9 -> 120.3, a picker training step 38.9 -> 29.7.
 #pragma once
 
 #include <cstddef>

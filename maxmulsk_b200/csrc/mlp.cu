@@ -128,10 +128,10 @@ mlp_forward_kernel(const float* __restrict__ params, const float* __restrict__ X
 // blocks form a cluster; at the end each adds an eighth of the weights over the
 // cluster's shared memories, in block order, into parts[cluster][NPARAM], and
 // mlp_grad_sum adds the clusters in order (with one cluster, parts is grads).
-// Bound by latency, so the rows are spread thin. At 4000 rows 22.8 us (ncu, cold
+// Bound by latency, so the rows are spread thin. At 4000 rows 22.8-24.2 us (ncu, cold
 // caches) on 256 blocks; 89 blocks of 45 rows without clusters 44 us, one thread
 // per weight walking all rows, in six launches, 840 us. A whole training step
-// 893 -> 39 us.
+// 893 -> 39 us, 30 with its launches overlapped (launch.cuh).
 constexpr int kBwdRows = 8, kBwdCluster = 8;
 __global__ void __launch_bounds__(256)
 mlp_backward_kernel(const float* __restrict__ params, const float* __restrict__ X, const float* __restrict__ Z1,
@@ -524,7 +524,7 @@ bool predict_plan(size_t M, size_t K, size_t N, int precision, maxmulsk_plan* ou
 // times, and a pick (forward pass, 24 or 48 candidates checked and sized) costs
 // 29-34 us on the host with scalar multiply-adds, several times a small
 // product on the GPU; 4.3-5.7 us with host_linear, 1 us or less found here. A
-// 256^3 matmul from Python 34 -> 16 us a call. Per thread, so no
+// 256^3 matmul from Python 34 -> 16 us a call (13 with what came after). Per thread, so no
 // lock; a direct-mapped table of fixed size; an entry holds for one model and
 // one device, whose work slots decide the workspaces.
 struct PickEntry {

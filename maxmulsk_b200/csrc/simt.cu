@@ -174,8 +174,8 @@ struct CpCfg {
     static_assert(THREADS >= BK && BK % 4 == 0 && STAGES >= 3 && THREADS <= 4 * BN, "tile configuration");
 };
 
-// The plans' tiles. 128 x 128: 8 x 16 outputs a thread (255 registers, two
-// CTAs an SM). 128 x 64: 8 x 8 a thread. 64 x 64: 4 x 8 a thread and four CTAs
+// The plans' tiles. 128 x 128: 8 x 16 outputs a thread (244 registers; 255 and 24
+// bytes spilled in the SCALAR variant; two CTAs an SM). 128 x 64: 8 x 8 a thread. 64 x 64: 4 x 8 a thread and four CTAs
 // an SM, which a small C needs to fill the GPU. Measured, per configuration
 // (4096^3 unsplit, 128 x 128: BK 16 x 4 stages 2358 us, 16 x 3 2377, 8 x 6
 // 2496; 2048^3 split 2, 128 x 64: 32 x 3, two CTAs 344, 16 x 4, three CTAs
@@ -462,7 +462,7 @@ sgemm_simt_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUni
 // clearing and counting arrivals costs more than the second launch (128 x 64
 // tiles, two slices: 2048^3 344 -> 331 us, 1024^3 62 -> 53, 300^3 29 -> 13). Bound by the reads of the
 // partials, splits * M * N floats, from L2 while they fit (126 MB). Measured
-// (ncu): 1024^2 x 8 slices 7.8 us (4.8 TB/s), 777 x 901 x 8 6.3 us, 512^2 x 16
+// (ncu): 1024^2 x 8 slices 7.8-9.2 us by run (4.1-4.8 TB/s), 777 x 901 x 8 6.3 us, 512^2 x 16
 // 5.4 us, 256^2 x 8 3.1 us; a grid-stride loop with a fixed batch of 64
 // predicated evict-first loads took 50, 36, 16.4 and 5.7 us.
 template <int BATCH, typename T>

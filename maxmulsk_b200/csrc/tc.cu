@@ -25,8 +25,8 @@
 //               planes: K-major BN x BK with 64-byte swizzle (TF32), or
 //               BK x BN in 128-byte column panels with 128-byte swizzle (BF16),
 //               into a ring of STAGES shared-memory stages.
-//   warp 1      TMEM owner; one thread issues the MMAs (128 x BN x KSTEP) of a
-//               chunk into one of NACC TMEM accumulators (all 512 columns: 4
+//   warp 1      TMEM owner; runs the issue loop whole, one lane issuing the MMAs
+//               (128 x BN x KSTEP) of a chunk into one of NACC TMEM accumulators (all 512 columns: 4
 //               for tiles up to 128 columns wide, 2 for 256) and commits each
 //               stage back to the producer and each chunk to the epilogue.
 //   warps 2..   epilogue (4 or 8 warps): TMEM -> registers (tcgen05.ld
@@ -1698,8 +1698,8 @@ tc_slim_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // wrote one partial tile per (128-row half, slice); here each output is summed
 // over the slices in slice order -- the order of the in-kernel fixup, so C is
 // the same bit for bit. Bound by the reads of the partials (nsplit floats per
-// output, from L2 while they fit). Measured (ncu): 1500 x 1999 x 4 slices 10.8 us
-// (5.4 TB/s), 1024^2 x 4 5.8 us, 128 x 512 x 37 5.0 us; one output per thread
+// output, from L2 while they fit). Measured (ncu): 1500 x 1999 x 4 slices 10.8-12.7 us
+// by run (4.7-5.5 TB/s), 1024^2 x 4 5.8 us, 128 x 512 x 37 5.0 us; one output per thread
 // down a column, which stored C 4 bytes at a time, took 32.1, 12.7 and 5.7 us.
 //
 // Partial tiles are column-major (element (r, c) at c * 128 + r), C is
