@@ -20,10 +20,12 @@
 // matrix is never touched.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "internal.hpp"
@@ -203,24 +205,16 @@ __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
 __device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-// c + a * b per lane: one fused multiply-add, or (SCALAR variant) a multiply,
-// then an add, each rounded. The latter stays on scalar instructions: the
-// compiler contracts a packed multiply and add into the fused form (seen in
-// results), which it never does to __fmul_rn and __fadd_rn.
-template <bool FUSED>
-__device__ __forceinline__ f32x2 mac2(f32x2 a, f32x2 b, f32x2 c) {
-    if constexpr (FUSED) {
-        f32x2 r;
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-        return r;
-    } else {
-        float a0, a1, b0, b1, c0, c1;
-        unpack2(a, a0, a1);
-        unpack2(b, b0, b1);
-        unpack2(c, c0, c1);
-        return pack2(__fadd_rn(c0, __fmul_rn(a0, b0)), __fadd_rn(c1, __fmul_rn(a1, b1)));
-    }
+// c + a * b: one fused multiply-add per lane, or (SCALAR variant) a multiply,
+// then an add, each rounded. The latter is on single floats: the compiler
+// contracts a packed multiply and add into the fused form (seen in results),
+// which it never does to __fmul_rn and __fadd_rn.
+__device__ __forceinline__ f32x2 mac(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
+__device__ __forceinline__ float mac(float a, float b, float c) { return __fadd_rn(c, __fmul_rn(a, b)); }
 
 // W floats from global to shared memory; with `bytes`, that many are read and
 // the rest of the 4 W written as zeros.
@@ -330,15 +324,19 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
         }
     };
 
-    f32x2 acc[RT][LT / 2];
+    // Packed pairs of outputs, or single ones in the SCALAR variant.
+    using Elem = std::conditional_t<FUSED, f32x2, float>;
+    using Quad = std::conditional_t<FUSED, ulonglong2, float4>;
+    constexpr int NE = FUSED ? LT / 2 : LT, PER = NE / GN;
+    Elem acc[RT][NE];
 #pragma unroll
     for (int i = 0; i < RT; i++)
 #pragma unroll
-        for (int j = 0; j < LT / 2; j++) acc[i][j] = 0ull;
+        for (int j = 0; j < NE; j++) acc[i][j] = 0;
 
     // Operand fragments of two k's: rows lm + 8 i of A, column quads of B.
     float2 fa[2][RT];
-    f32x2 fb[2][LT / 2];
+    Elem fb[2][NE];
     const int a_off = (wm * Cf::WM + lm) * AST, b_off = Cf::A_FLOATS + wn * Cf::WN + ln * 4;
     auto load_a = [&](int set, const float* st, int k) {
 #pragma unroll
@@ -347,9 +345,13 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
     auto load_b = [&](int set, const float* st, int k) {
 #pragma unroll
         for (int j = 0; j < GN; j++) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(st + b_off + k * BN + j * 4 * Cf::LN);
-            fb[set][2 * j] = v.x;
-            fb[set][2 * j + 1] = v.y;
+            const Quad v = *reinterpret_cast<const Quad*>(st + b_off + k * BN + j * 4 * Cf::LN);
+            fb[set][PER * j] = v.x;
+            fb[set][PER * j + 1] = v.y;
+            if constexpr (!FUSED) {
+                fb[set][PER * j + 2] = v.z;
+                fb[set][PER * j + 3] = v.w;
+            }
         }
     };
 
@@ -366,40 +368,50 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
     // reads the next stage's first ones, after the barrier that says that stage
     // has landed and that every warp has read the stage before it, whose buffer
     // the next copies take. (Past the last stage it reads a stale buffer, unused.)
+    //
+    // A stage is unrolled whole, or in the SCALAR variant, with four times the
+    // instructions, four k's at a time: eight or sixteen are more code than the
+    // instruction cache holds (sixty 128 x 128 plans, against an earlier kernel: four
+    // k's 0.74 of its time on long K, eight 1.15, sixteen 1.43).
+    constexpr int U = FUSED ? BK : 4;
     int buf = 0;
     for (int64_t t = 0; t < ntiles; t++) {
         const float* cur = smem + buf * Cf::STAGE_FLOATS;
         const int nbuf = buf + 1 == STAGES ? 0 : buf + 1;
         const float* nxt = smem + nbuf * Cf::STAGE_FLOATS;
+#pragma unroll 1
+        for (int k0 = 0; k0 < BK; k0 += U) {
 #pragma unroll
-        for (int k = 0; k < BK; k++) {
-            if (k + 1 < BK) {
-                load_b((k + 1) & 1, cur, k + 1);
-                if ((k & 1) == 1) load_a(((k + 1) >> 1) & 1, cur, k + 1);
-            } else {
-                cp_async_wait<STAGES - 3>();
-                __syncthreads();
-                const int64_t tn = t + STAGES - 1;
-                if (tn < ntiles) load_stage(buf == 0 ? STAGES - 1 : buf - 1, kbeg + tn * BK);
-                cp_async_commit();
-                load_b(0, nxt, 0);
-                load_a(0, nxt, 0);
-            }
-            f32x2 aa[RT];
-#pragma unroll
-            for (int i = 0; i < RT; i++) {
-                const float2 v = fa[(k >> 1) & 1][i];
-                aa[i] = (k & 1) ? pack2(v.y, v.y) : pack2(v.x, v.x);
-            }
-            // Column by column, rows down and up in turn: neighbouring
-            // instructions share an operand.
-#pragma unroll
-            for (int j = 0; j < LT / 2; j++)
-#pragma unroll
-                for (int q = 0; q < RT; q++) {
-                    const int i = (j & 1) ? RT - 1 - q : q;
-                    acc[i][j] = mac2<FUSED>(aa[i], fb[k & 1][j], acc[i][j]);
+            for (int k = 0; k < U; k++) {
+                if (k + 1 < U || k0 + U < BK) {
+                    load_b((k + 1) & 1, cur, k0 + k + 1);
+                    if ((k & 1) == 1) load_a(((k + 1) >> 1) & 1, cur, k0 + k + 1);
+                } else {
+                    cp_async_wait<STAGES - 3>();
+                    __syncthreads();
+                    const int64_t tn = t + STAGES - 1;
+                    if (tn < ntiles) load_stage(buf == 0 ? STAGES - 1 : buf - 1, kbeg + tn * BK);
+                    cp_async_commit();
+                    load_b(0, nxt, 0);
+                    load_a(0, nxt, 0);
                 }
+                Elem aa[RT];
+#pragma unroll
+                for (int i = 0; i < RT; i++) {
+                    const float2 v = fa[(k >> 1) & 1][i];
+                    if constexpr (FUSED) aa[i] = (k & 1) ? pack2(v.y, v.y) : pack2(v.x, v.x);
+                    else aa[i] = (k & 1) ? v.y : v.x;
+                }
+                // Column by column, rows down and up in turn: neighbouring
+                // instructions share an operand.
+#pragma unroll
+                for (int j = 0; j < NE; j++)
+#pragma unroll
+                    for (int q = 0; q < RT; q++) {
+                        const int i = (j & 1) ? RT - 1 - q : q;
+                        acc[i][j] = mac(aa[i], fb[k & 1][j], acc[i][j]);
+                    }
+            }
         }
         buf = nbuf;
     }
@@ -410,7 +422,10 @@ __device__ __forceinline__ void simt_cp_tile(const SimtArgs& p, int64_t m0, int6
 #pragma unroll
     for (int i = 0; i < RT; i++)
 #pragma unroll
-        for (int j = 0; j < LT / 2; j++) unpack2(acc[i][j], out[i][2 * j], out[i][2 * j + 1]);
+        for (int j = 0; j < NE; j++) {
+            if constexpr (FUSED) unpack2(acc[i][j], out[i][2 * j], out[i][2 * j + 1]);
+            else out[i][j] = acc[i][j];
+        }
     auto out_row = [&](int i) { return m0 + wm * Cf::WM + lm + Cf::LM * i; };
     auto out_col = [&](int g) { return n0 + wn * Cf::WN + ln * 4 + 4 * Cf::LN * g; };
     simt_epilogue<RT, GN>(p, out, out_row, out_col, p.wc == 4, z, tile, last_flag);
@@ -426,16 +441,185 @@ sgemm_simt_cp_kernel(SimtArgs p) {
                             blockIdx.y * gridDim.x + blockIdx.x, smem, last_flag);
 }
 
+// ---------------------------------------------------------------------------
+// The register-staged tile, for what the ring above is the slower at: the SCALAR
+// variant on 64 columns.
+//
+// 256 threads, BM / 16 x BN / 16 outputs each; stages of 16 k's go through
+// registers into two shared buffers, A transposed to k-major so that a fragment
+// is read in 128-bit loads: As[k][m ^ (k & 8)], rows of BM + 4 floats, which keeps
+// the transposing stores of a warp on distinct banks. Same chains, same bits.
+//
+// SCALAR: bound by the latency of multiply, then add, where a single wave leaves
+// a warp or two a scheduler; this tile has two, and its unrolled stage fits the
+// instruction cache. 1 x 10786 x 54 on 128 x 64 tiles 2466 us on the ring unrolled
+// whole, 1199 in bodies of four k's, 958 here; over 120 plans 0.56-1.01 of the time
+// of an earlier kernel by tile and K (geometric means), at most 1.03 of it.
+// ---------------------------------------------------------------------------
+constexpr int kRegThreads = 256, RBK = 16;
+
+template <int BM, int BN>
+struct RegSmem {
+    float As[2][RBK][BM + 4];
+    float Bs[2][RBK][BN];
+};
+
+template <bool FUSED>
+__device__ __forceinline__ float reg_mac(float a, float b, float c) {
+    if constexpr (FUSED) return __fmaf_rn(a, b, c);
+    else return mac(a, b, c);
+}
+
+// VEC: 128-bit loads of A and B.
+template <int BM, int BN, bool FUSED>
+__device__ __forceinline__ void simt_reg_tile(const SimtArgs& p, int64_t m0, int64_t n0, int z, unsigned tile,
+                                              RegSmem<BM, BN>& sm, int& last_flag, bool VEC) {
+    constexpr int TM = BM / 16, TN = BN / 16;       // per-thread outputs
+    constexpr int GM = TM / 4, GN = TN / 4;         // 4-wide groups per thread
+    constexpr int A_F4 = BM * RBK / 4 / kRegThreads;   // float4 loads per thread
+    constexpr int B_F4 = BN * RBK / 4 / kRegThreads;
+    auto& As = sm.As;
+    auto& Bs = sm.Bs;
+
+    const int tid = threadIdx.x;
+    const int tx = tid & 15, ty = tid >> 4;
+    const int64_t kbeg = (int64_t)z * p.kchunk;
+    const int64_t kend = min(p.K, kbeg + p.kchunk);
+    const int64_t M = p.M, N = p.N, K = p.K;
+    const float* __restrict__ A = p.A;
+    const float* __restrict__ B = p.B;
+
+    float4 ra[A_F4], rb[B_F4];
+
+    auto load_tile = [&](int64_t k0) {
+#pragma unroll
+        for (int j = 0; j < A_F4; j++) {
+            const int f = tid + j * kRegThreads;
+            const int row = f / (RBK / 4);
+            const int kq = (f % (RBK / 4)) * 4;
+            const int64_t gm = m0 + row, gk = k0 + kq;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (gm < M) {
+                const float* src = A + gm * K + gk;
+                if (VEC) {
+                    if (gk < kend) v = __ldg(reinterpret_cast<const float4*>(src));
+                } else {
+                    if (gk + 0 < kend) v.x = __ldg(src + 0);
+                    if (gk + 1 < kend) v.y = __ldg(src + 1);
+                    if (gk + 2 < kend) v.z = __ldg(src + 2);
+                    if (gk + 3 < kend) v.w = __ldg(src + 3);
+                }
+            }
+            ra[j] = v;
+        }
+#pragma unroll
+        for (int j = 0; j < B_F4; j++) {
+            const int f = tid + j * kRegThreads;
+            const int kr = f / (BN / 4);
+            const int nq = (f % (BN / 4)) * 4;
+            const int64_t gk = k0 + kr, gn = n0 + nq;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (gk < kend) {
+                const float* src = B + gk * N + gn;
+                if (VEC) {
+                    if (gn < N) v = __ldg(reinterpret_cast<const float4*>(src));
+                } else {
+                    if (gn + 0 < N) v.x = __ldg(src + 0);
+                    if (gn + 1 < N) v.y = __ldg(src + 1);
+                    if (gn + 2 < N) v.z = __ldg(src + 2);
+                    if (gn + 3 < N) v.w = __ldg(src + 3);
+                }
+            }
+            rb[j] = v;
+        }
+    };
+    auto store_tile = [&](int buf) {
+#pragma unroll
+        for (int j = 0; j < A_F4; j++) {
+            const int f = tid + j * kRegThreads;
+            const int row = f / (RBK / 4);
+            const int kq = (f % (RBK / 4)) * 4;
+            const int srow = row ^ (kq & 8);
+            As[buf][kq + 0][srow] = ra[j].x;
+            As[buf][kq + 1][srow] = ra[j].y;
+            As[buf][kq + 2][srow] = ra[j].z;
+            As[buf][kq + 3][srow] = ra[j].w;
+        }
+#pragma unroll
+        for (int j = 0; j < B_F4; j++) {
+            const int f = tid + j * kRegThreads;
+            const int kr = f / (BN / 4);
+            const int nq = (f % (BN / 4)) * 4;
+            *reinterpret_cast<float4*>(&Bs[buf][kr][nq]) = rb[j];
+        }
+    };
+
+    float acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
+
+    const int64_t ntiles = (kend - kbeg + RBK - 1) / RBK;
+    if (ntiles > 0) {
+        load_tile(kbeg);
+        store_tile(0);
+        __syncthreads();
+        for (int64_t t = 0; t < ntiles; t++) {
+            const int buf = (int)(t & 1);
+            if (t + 1 < ntiles) load_tile(kbeg + (t + 1) * RBK);
+            // Fragments of step k + 1 are read from shared memory while the
+            // products of step k run (two register sets, fully unrolled).
+            float a[2][TM], b[2][TN];
+            auto load_frag = [&](int set, int k) {
+#pragma unroll
+                for (int g = 0; g < GM; g++) {
+                    float4 v = *reinterpret_cast<const float4*>(&As[buf][k][(g * 64 + ty * 4) ^ (k & 8)]);
+                    a[set][g * 4 + 0] = v.x; a[set][g * 4 + 1] = v.y; a[set][g * 4 + 2] = v.z; a[set][g * 4 + 3] = v.w;
+                }
+#pragma unroll
+                for (int g = 0; g < GN; g++) {
+                    float4 v = *reinterpret_cast<const float4*>(&Bs[buf][k][g * 64 + tx * 4]);
+                    b[set][g * 4 + 0] = v.x; b[set][g * 4 + 1] = v.y; b[set][g * 4 + 2] = v.z; b[set][g * 4 + 3] = v.w;
+                }
+            };
+            load_frag(0, 0);
+#pragma unroll
+            for (int k = 0; k < RBK; k++) {
+                if (k + 1 < RBK) load_frag((k + 1) & 1, k + 1);
+#pragma unroll
+                for (int i = 0; i < TM; i++)
+#pragma unroll
+                    for (int j = 0; j < TN; j++) acc[i][j] = reg_mac<FUSED>(a[k & 1][i], b[k & 1][j], acc[i][j]);
+            }
+            if (t + 1 < ntiles) store_tile(buf ^ 1);
+            __syncthreads();
+        }
+    }
+
+    // Steps past kend multiplied zeros, as above.
+    auto out_row = [&](int i) { return m0 + (i / 4) * 64 + ty * 4 + (i % 4); };
+    auto out_col = [&](int g) { return n0 + g * 64 + tx * 4; };
+    simt_epilogue<TM, GN>(p, acc, out_row, out_col, p.wc == 4, z, tile, last_flag);
+}
+
+template <int BM, int BN, bool FUSED, bool VEC>
+__global__ void __launch_bounds__(kRegThreads, 2)
+sgemm_simt_reg_kernel(SimtArgs p) {
+    __shared__ __align__(16) RegSmem<BM, BN> sm;
+    __shared__ int last_flag;
+    grid_wait();
+    simt_reg_tile<BM, BN, FUSED>(p, (int64_t)blockIdx.y * BM, (int64_t)blockIdx.x * BN, blockIdx.z,
+                                 blockIdx.y * gridDim.x + blockIdx.x, sm, last_flag, VEC);
+}
+
 // Grouped launch: one persistent kernel over a list of (problem, tile, K
 // slice) units taken from an atomic counter, heaviest units first. Each unit
 // is exactly the tile a per-GEMM launch of that problem computes, so results
 // are identical to running the problems one by one.
-template <class Cf, bool FUSED>
-__global__ void __launch_bounds__(Cf::THREADS, Cf::CTAS)
-sgemm_simt_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUnit* __restrict__ units, int nunits,
-                          unsigned* next) {
-    extern __shared__ __align__(16) float smem[];
-    __shared__ int last_flag;
+template <class RunUnit>
+__device__ __forceinline__ void grouped_units(const GroupProblem* __restrict__ probs, const GroupUnit* __restrict__ units,
+                                              int nunits, unsigned* next, RunUnit run) {
     __shared__ int s_unit;
     grid_wait();
     // Thread 0 fetches the next unit's number while the current one runs.
@@ -447,10 +631,34 @@ sgemm_simt_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUni
         if (u >= nunits) break;
         if (threadIdx.x == 0) fetched = atomicAdd(next, 1u);
         const GroupUnit w = units[u];
-        const SimtArgs a = probs[w.problem].a;
-        const unsigned tile = (unsigned)w.tm * (unsigned)probs[w.problem].tiles_n + (unsigned)w.tn;
-        simt_cp_tile<Cf, FUSED>(a, (int64_t)w.tm * Cf::BM, (int64_t)w.tn * Cf::BN, w.z, tile, smem, last_flag);
+        const GroupProblem& P = probs[w.problem];
+        const unsigned tile = (unsigned)w.tm * (unsigned)P.tiles_n + (unsigned)w.tn;
+        run(P.a, w, tile);
     }
+}
+
+template <class Cf, bool FUSED>
+__global__ void __launch_bounds__(Cf::THREADS, Cf::CTAS)
+sgemm_simt_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUnit* __restrict__ units, int nunits,
+                          unsigned* next) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int last_flag;
+    grouped_units(probs, units, nunits, next, [&](const SimtArgs& args, const GroupUnit& w, unsigned tile) {
+        const SimtArgs a = args;
+        simt_cp_tile<Cf, FUSED>(a, (int64_t)w.tm * Cf::BM, (int64_t)w.tn * Cf::BN, w.z, tile, smem, last_flag);
+    });
+}
+
+template <int BM, int BN, bool FUSED>
+__global__ void __launch_bounds__(kRegThreads, 2)
+sgemm_simt_reg_grouped_kernel(const GroupProblem* __restrict__ probs, const GroupUnit* __restrict__ units, int nunits,
+                              unsigned* next) {
+    __shared__ __align__(16) RegSmem<BM, BN> sm;
+    __shared__ int last_flag;
+    grouped_units(probs, units, nunits, next, [&](const SimtArgs& a, const GroupUnit& w, unsigned tile) {
+        simt_reg_tile<BM, BN, FUSED>(a, (int64_t)w.tm * BM, (int64_t)w.tn * BN, w.z, tile, sm, last_flag,
+                                     a.wa == 4 && a.wb == 4);
+    });
 }
 
 // Split-K reduction of the single launches (grouped launches sum in the last
@@ -516,9 +724,16 @@ cudaError_t launch_cp(const SimtArgs& a, dim3 grid, cudaStream_t s) {
     return launch_overlapped(sgemm_simt_cp_kernel<Cf, FUSED>, grid, Cf::THREADS, Cf::SMEM, s, 1, a);
 }
 
+template <int BM, int BN, bool FUSED>
+cudaError_t launch_reg(const SimtArgs& a, dim3 grid, cudaStream_t s) {
+    auto kernel = a.wa == 4 && a.wb == 4 ? sgemm_simt_reg_kernel<BM, BN, FUSED, true> : sgemm_simt_reg_kernel<BM, BN, FUSED, false>;
+    return launch_overlapped(kernel, grid, kRegThreads, 0, s, 1, a);
+}
+
 template <int BM, int BN>
 cudaError_t launch_tile(const SimtArgs& args, int variant, cudaStream_t s) {
     using Cf = CpTile<BM, BN>;
+    const bool scalar = variant == MAXMULSK_FP32_SCALAR;
     SimtArgs a = args;
     a.reduce_after = a.splits > 1 ? 1 : 0;
     simt_set_widths(a);
@@ -526,7 +741,12 @@ cudaError_t launch_tile(const SimtArgs& args, int variant, cudaStream_t s) {
     cudaError_t e;
     {
         PhaseScope ps(kPhaseGemm, s);
-        e = variant != MAXMULSK_FP32_SCALAR ? launch_cp<Cf, true>(a, grid, s) : launch_cp<Cf, false>(a, grid, s);
+        if constexpr (BN == 64) {
+            if (scalar) e = launch_reg<BM, BN, false>(a, grid, s);
+            else e = launch_cp<Cf, true>(a, grid, s);
+        } else {
+            e = scalar ? launch_cp<Cf, false>(a, grid, s) : launch_cp<Cf, true>(a, grid, s);
+        }
     }
     if (e != cudaSuccess || !a.reduce_after) return e;
     PhaseScope ps(kPhaseReduce, s);
@@ -586,12 +806,22 @@ cudaError_t launch_grouped(const GroupProblem* probs, const GroupUnit* units, in
     return launch_overlapped(sgemm_simt_grouped_kernel<Cf, FUSED>, dim3(nunits < slots ? nunits : slots), Cf::THREADS,
                              Cf::SMEM, s, 1, probs, units, nunits, next);
 }
+template <int BM, int BN, bool FUSED>
+cudaError_t launch_reg_grouped(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next, int sms,
+                               cudaStream_t s) {
+    return launch_overlapped(sgemm_simt_reg_grouped_kernel<BM, BN, FUSED>, dim3(std::min(nunits, 2 * sms)), kRegThreads, 0, s, 1,
+                             probs, units, nunits, next);
+}
 template <int BM, int BN>
 cudaError_t launch_grouped_tile(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,
                                 int variant, int sms, cudaStream_t s) {
     using Cf = CpTile<BM, BN>;
-    return variant != MAXMULSK_FP32_SCALAR ? launch_grouped<Cf, true>(probs, units, nunits, next, sms, s)
-                                           : launch_grouped<Cf, false>(probs, units, nunits, next, sms, s);
+    const bool scalar = variant == MAXMULSK_FP32_SCALAR;
+    if constexpr (BN == 64)
+        if (scalar) return launch_reg_grouped<BM, BN, false>(probs, units, nunits, next, sms, s);
+    if constexpr (BN != 64)
+        if (scalar) return launch_grouped<Cf, false>(probs, units, nunits, next, sms, s);
+    return launch_grouped<Cf, true>(probs, units, nunits, next, sms, s);
 }
 }  // namespace
 

@@ -325,3 +325,23 @@ def test_group_on_own_tiles_reports_one_tile_and_equals_the_oracle(cuda, oracle_
                 assert np.all(c[off - 64: off] == SENT)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("tile", [(128, 128), (128, 64), (64, 64)])
+def test_groups_of_short_k_and_of_the_scalar_variant_equal_the_oracle(cuda, oracle_mod, tile, variant):
+    # Groups whose longest slice is 16 k's and longer ones: both kernels of a tile.
+    for shapes in ([(129, 16, 65), (64, 3, 260), (1, 1, 4), (200, 11, 132)], [(129, 17, 65), (64, 300, 260), (1, 64, 4), (70, 3, 68)]):
+        for split in (1, 3):
+            g, cbuf, host, offs = _group(cuda, oracle_mod, shapes, 40, mm.make_plan(0, *tile, split, variant))
+            try:
+                for _ in range(2):
+                    cbuf.fill_(float("nan"))
+                    cuda.cuda.synchronize()
+                    assert g.launch() == 0 and mm.stream_status() == 0
+                    c = cbuf.cpu().numpy()
+                    for (M, K, N), (A, B), off in zip(shapes, host, offs):
+                        want = oracle_mod.sgemm_panels(A, B, M, K, N, kc=mm.slice_len(K, split), fma=variant == 0)
+                        assert np.array_equal(c[off: off + M * N].view(np.uint32), want.ravel().view(np.uint32)), (M, K, N)
+            finally:
+                g.close()

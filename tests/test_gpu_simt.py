@@ -260,3 +260,54 @@ def test_copy_widths_bit_exact(cuda, oracle_mod, tile, variant, K, N, off):
     assert st == 0 and bands, mm.last_error_message()
     ref = oracle_mod.sgemm_panels(A, B, M, K, N, fma=variant == mm.FP32_FMA)
     assert np.array_equal(bits(C), bits(ref))
+
+
+# The tile that stages through registers: the SCALAR variant on 64 columns and K
+# slices of a few stages, around its stage of 16 k's and the lines of its rules.
+@pytest.mark.parametrize("tile", [(128, 64), (64, 64), (128, 128)])
+@pytest.mark.parametrize("variant", [0, 1])
+def test_short_k_and_scalar_tiles_equal_the_oracle(cuda, oracle_mod, tile, variant):
+    for M, N, off in [(130, 65, 0), (64, 132, 0), (1, 4, 0), (129, 260, 1), (63, 68, 4)]:
+        for K in (1, 3, 4, 15, 16, 17, 28, 31, 32, 33, 63, 64, 65, 100):
+            for split in (1, 2):
+                A, B = oracle_mod.fill_uniform(M * K + off, 5), oracle_mod.fill_wide(K * N + off, 6)
+                p = mm.make_plan(0, *tile, split, variant)
+                dA, dB = to_dev(cuda, A)[off:], to_dev(cuda, B)[off:]
+                C = cuda.full((M * N + 64,), 3.75, device="cuda")
+                nb = mm.workspace_bytes(M, K, N, p)
+                ws = cuda.full((nb + 256,), 255, dtype=cuda.uint8, device="cuda")
+                wp = ws.data_ptr() + (-ws.data_ptr()) % 256
+                assert mm.sgemm_plan_dev(dA, dB, C, M, K, N, p, wp, nb) == 0, mm.last_error_message()
+                want = oracle_mod.sgemm_panels(A[off:], B[off:], M, K, N, kc=mm.slice_len(K, split), fma=variant == 0)
+                got = C.cpu().numpy()
+                assert np.array_equal(bits(got[: M * N].reshape(M, N)), bits(want)), (M, K, N, split, off)
+                assert np.all(got[M * N:] == 3.75)
+
+
+def _graph_us(torch, M, K, N, plan, n=20):
+    A, B, C = torch.randn(M * K, device="cuda"), torch.randn(K * N, device="cuda"), torch.empty(M * N, device="cuda")
+    assert mm.sgemm_plan_dev(A, B, C, M, K, N, plan) == 0, mm.last_error_message()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        for _ in range(n):
+            mm.sgemm_plan_dev(A, B, C, M, K, N, plan)
+    times = []
+    for _ in range(7):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        g.replay()
+        e1.record()
+        torch.cuda.synchronize()
+        times.append(e0.elapsed_time(e1) * 1000 / n)
+    return sorted(times)[3]
+
+
+@pytest.mark.parametrize("tile", [(128, 64), (64, 64)])
+def test_scalar_variant_takes_its_arithmetic_longer(cuda, tile):
+    # Two rounded operations a product instead of one: twice the pipe's time and
+    # twice the chain's latency, a quarter allowed on top. It took 3.2 times as long
+    # on 128 x 64 tiles when its unrolled code did not fit the instruction cache.
+    for M, K, N in [(1, 10786, 54), (5, 12891, 27)]:
+        fma, scalar = (_graph_us(cuda, M, K, N, mm.make_plan(0, *tile, 1, v), 4) for v in (0, 1))
+        assert scalar <= 2.5 * fma, (M, K, N, scalar, fma)
