@@ -56,6 +56,7 @@ struct maxmulsk_grouped_s {
     mmsk::GroupUnit* d_units = nullptr;
     struct SimtPart {                      // units of one tile shape: one launch
         int bm, bn, first, count;
+        int64_t longest;                   // k's of its longest unit
     };
     std::vector<SimtPart> simt_parts;
     unsigned* d_next = nullptr;            // a unit counter per part
@@ -253,8 +254,8 @@ maxmulsk_status build_simt(maxmulsk_grouped_s* g, const maxmulsk_problem* proble
     for (size_t i = 0; i < hu.size(); i++) {
         const SimtTile& t = tiles[hu[i].problem];
         if (g->simt_parts.empty() || g->simt_parts.back().bm != t.bm || g->simt_parts.back().bn != t.bn)
-            g->simt_parts.push_back({t.bm, t.bn, (int)i, 0});
-        g->simt_parts.back().count++;
+            g->simt_parts.push_back({t.bm, t.bn, (int)i, 0, std::min(hp[hu[i].problem].a.K, hp[hu[i].problem].a.kchunk)});
+        g->simt_parts.back().count++;                          // heaviest first: the part's first unit is its longest
     }
     g->sms = sms;
     cudaError_t e;
@@ -544,7 +545,7 @@ maxmulsk_status capture_group(maxmulsk_grouped_s* g, const maxmulsk_problem* pro
         for (size_t i = 0; i < g->simt_parts.size(); i++) {
             const auto& t = g->simt_parts[i];
             cudaError_t el = simt_grouped_launch(g->d_probs, g->d_units + t.first, t.count, g->d_next + i, t.bm, t.bn,
-                                                 g->simt_plan.variant, g->sms, g->cap);
+                                                 g->simt_plan.variant, g->sms, t.longest, g->cap);
             if (el != cudaSuccess) e = el;
         }
         for (const auto& sg : g->singles) {

@@ -69,8 +69,9 @@ struct GroupProblem {
 struct GroupUnit {
     int32_t problem, tm, tn, z;
 };
+// `longest`: k's of the longest unit.
 cudaError_t simt_grouped_launch(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,
-                                int tile_m, int tile_n, int variant, int sms, cudaStream_t s);
+                                int tile_m, int tile_n, int variant, int sms, int64_t longest, cudaStream_t s);
 // Runs an FP32 plan whose split-K scratch (counters, then partials) is at
 // `scratch` (>= simt_workspace_bytes; may be null without a K split): lays it
 // out and launches (the counters are unused, their place kept). Both the

@@ -443,7 +443,7 @@ sgemm_simt_cp_kernel(SimtArgs p) {
 
 // ---------------------------------------------------------------------------
 // The register-staged tile, for what the ring above is the slower at: the SCALAR
-// variant on 64 columns.
+// variant on 64 columns, and short K slices.
 //
 // 256 threads, BM / 16 x BN / 16 outputs each; stages of 16 k's go through
 // registers into two shared buffers, A transposed to k-major so that a fragment
@@ -455,8 +455,15 @@ sgemm_simt_cp_kernel(SimtArgs p) {
 // instruction cache. 1 x 10786 x 54 on 128 x 64 tiles 2466 us on the ring unrolled
 // whole, 1199 in bodies of four k's, 958 here; over 120 plans 0.56-1.01 of the time
 // of an earlier kernel by tile and K (geometric means), at most 1.03 of it.
+// Short K: the ring's stage of 32 k's is loaded and multiplied whole, so K of 8 or
+// 11 costs what 32 does: 1275 x 11 x 2921 on 128 x 64 tiles 14.4 -> 10.6 us, 3254 x 8 x 998
+// on 64 x 64 12.1 -> 8.1. kShortK is where that stops paying for every tile; single
+// launches go on to 31 k's on 64 x 64 tiles and 64 on 128 x 64, whose ring fills late
+// (times over the ring's, geometric means: 17-32 k's 0.94 on 128 x 64, 1.01 on 64 x 64;
+// 33-64 k's 0.97 and 1.04).
 // ---------------------------------------------------------------------------
 constexpr int kRegThreads = 256, RBK = 16;
+constexpr int64_t kShortK = 16;
 
 template <int BM, int BN>
 struct RegSmem {
@@ -586,6 +593,8 @@ __device__ __forceinline__ void simt_reg_tile(const SimtArgs& p, int64_t m0, int
             load_frag(0, 0);
 #pragma unroll
             for (int k = 0; k < RBK; k++) {
+                // A short K stops after its last four k's.
+                if (FUSED && k > 0 && k % 4 == 0 && kbeg + t * RBK + k >= kend) break;
                 if (k + 1 < RBK) load_frag((k + 1) & 1, k + 1);
 #pragma unroll
                 for (int i = 0; i < TM; i++)
@@ -743,6 +752,7 @@ cudaError_t launch_tile(const SimtArgs& args, int variant, cudaStream_t s) {
         PhaseScope ps(kPhaseGemm, s);
         if constexpr (BN == 64) {
             if (scalar) e = launch_reg<BM, BN, false>(a, grid, s);
+            else if (std::min(a.K, a.kchunk) <= (BM == 128 ? 64 : 31)) e = launch_reg<BM, BN, true>(a, grid, s);
             else e = launch_cp<Cf, true>(a, grid, s);
         } else {
             e = scalar ? launch_cp<Cf, false>(a, grid, s) : launch_cp<Cf, true>(a, grid, s);
@@ -814,11 +824,13 @@ cudaError_t launch_reg_grouped(const GroupProblem* probs, const GroupUnit* units
 }
 template <int BM, int BN>
 cudaError_t launch_grouped_tile(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,
-                                int variant, int sms, cudaStream_t s) {
+                                int variant, int sms, int64_t longest, cudaStream_t s) {
     using Cf = CpTile<BM, BN>;
     const bool scalar = variant == MAXMULSK_FP32_SCALAR;
-    if constexpr (BN == 64)
-        if (scalar) return launch_reg_grouped<BM, BN, false>(probs, units, nunits, next, sms, s);
+    if constexpr (BM >= 64) {
+        if (scalar && (BN == 64 || longest <= kShortK)) return launch_reg_grouped<BM, BN, false>(probs, units, nunits, next, sms, s);
+        if (!scalar && longest <= kShortK) return launch_reg_grouped<BM, BN, true>(probs, units, nunits, next, sms, s);
+    }
     if constexpr (BN != 64)
         if (scalar) return launch_grouped<Cf, false>(probs, units, nunits, next, sms, s);
     return launch_grouped<Cf, true>(probs, units, nunits, next, sms, s);
@@ -826,11 +838,11 @@ cudaError_t launch_grouped_tile(const GroupProblem* probs, const GroupUnit* unit
 }  // namespace
 
 cudaError_t simt_grouped_launch(const GroupProblem* probs, const GroupUnit* units, int nunits, unsigned* next,
-                                int tile_m, int tile_n, int variant, int sms, cudaStream_t s) {
-    if (tile_m == 128 && tile_n == 128) return launch_grouped_tile<128, 128>(probs, units, nunits, next, variant, sms, s);
-    if (tile_m == 128 && tile_n == 64) return launch_grouped_tile<128, 64>(probs, units, nunits, next, variant, sms, s);
-    if (tile_m == 64 && tile_n == 64) return launch_grouped_tile<64, 64>(probs, units, nunits, next, variant, sms, s);
-    if (tile_m == 16 && tile_n == 256) return launch_grouped_tile<16, 256>(probs, units, nunits, next, variant, sms, s);
+                                int tile_m, int tile_n, int variant, int sms, int64_t longest, cudaStream_t s) {
+    if (tile_m == 128 && tile_n == 128) return launch_grouped_tile<128, 128>(probs, units, nunits, next, variant, sms, longest, s);
+    if (tile_m == 128 && tile_n == 64) return launch_grouped_tile<128, 64>(probs, units, nunits, next, variant, sms, longest, s);
+    if (tile_m == 64 && tile_n == 64) return launch_grouped_tile<64, 64>(probs, units, nunits, next, variant, sms, longest, s);
+    if (tile_m == 16 && tile_n == 256) return launch_grouped_tile<16, 256>(probs, units, nunits, next, variant, sms, longest, s);
     return cudaErrorInvalidValue;
 }
 

@@ -311,3 +311,12 @@ def test_scalar_variant_takes_its_arithmetic_longer(cuda, tile):
     for M, K, N in [(1, 10786, 54), (5, 12891, 27)]:
         fma, scalar = (_graph_us(cuda, M, K, N, mm.make_plan(0, *tile, 1, v), 4) for v in (0, 1))
         assert scalar <= 2.5 * fma, (M, K, N, scalar, fma)
+
+
+@pytest.mark.parametrize("tile", [(128, 64), (64, 64)])
+def test_short_k_does_not_pay_for_a_whole_stage(cuda, tile):
+    # 4096 x K x 4096: at K = 32 the products take 14 us of the FP32 pipe at best, at
+    # K = 8 a quarter, beside 10 us of stores. Multiplied as a stage of 32 k's, K = 8 took
+    # as long as K = 32.
+    us = {K: _graph_us(cuda, 4096, K, 4096, mm.make_plan(0, *tile, 1, 0)) for K in (8, 32)}
+    assert us[8] <= 0.85 * us[32], us
