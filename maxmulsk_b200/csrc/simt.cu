@@ -176,7 +176,7 @@ struct CpCfg {
     static_assert(THREADS >= BK && BK % 4 == 0 && STAGES >= 3 && THREADS <= 4 * BN, "tile configuration");
 };
 
-// The plans' tiles. 128 x 128: 8 x 16 outputs a thread (244 registers; 255 and 24
+// The plans' tiles. 128 x 128: 8 x 16 outputs a thread (244 registers; 255 and 8
 // bytes spilled in the SCALAR variant; two CTAs an SM). 128 x 64: 8 x 8 a thread. 64 x 64: 4 x 8 a thread and four CTAs
 // an SM, which a small C needs to fill the GPU. Measured, per configuration
 // (4096^3 unsplit, 128 x 128: BK 16 x 4 stages 2358 us, 16 x 3 2377, 8 x 6
